@@ -30,6 +30,7 @@ UNITS = [
     ("amg_setup.cu", []),
     ("cycle.cu", []),
     ("adjoint.cu", []),
+    ("coo.cu", []),
     ("noalloc.cu", []),
     ("capi.cpp", []),
     ("foam.cpp", []),

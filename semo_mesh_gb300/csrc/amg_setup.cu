@@ -1193,5 +1193,6 @@ template void build_hierarchy<float>(semo_ctx*, Amg<float>&, const int*, const i
 template void build_hierarchy<double>(semo_ctx*, Amg<double>&, const int*, const int*, const double*, int, int64_t);
 
 int device_scan(cudaStream_t s, int* d, int n, int* hpin) { return scan_exclusive(s, d, n, hpin); }
+void device_scan_async(cudaStream_t s, int* d, int n) { scan_async(s, d, n, nullptr); }
 
 }  // namespace semo

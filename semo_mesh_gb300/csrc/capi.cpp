@@ -1154,29 +1154,12 @@ semo_status semo_solve_coo(semo_ctx* c, int n, int64_t nnz, const int32_t* rows,
         need(nnz < INT32_MAX, SEMO_ERR_ARGUMENT, "nnz too large");
         SEMO_CUDA(cudaSetDevice(c->device));
         // COO -> CSR exactly as solveAMGCL.cpp:206-251 (in-row order = COO order)
-        std::vector<int> ptr(n + 1, 0), col(nnz);
-        std::vector<double> val(nnz);
-        for (int64_t k = 0; k < nnz; ++k) {
-            need(rows[k] >= 0 && rows[k] < n && cols[k] >= 0 && cols[k] < n, SEMO_ERR_ARGUMENT, "COO index out of range");
-            need(std::isfinite(vals[k]), SEMO_ERR_NAN, "non-finite matrix value");
-            ptr[rows[k]]++;
-        }
-        for (int i = 0, s = 0; i < n; ++i) { int t = ptr[i]; ptr[i] = s; s += t; }
-        ptr[n] = (int)nnz;
-        for (int64_t k = 0; k < nnz; ++k) { int d = ptr[rows[k]]++; col[d] = cols[k]; val[d] = vals[k]; }
-        for (int i = 0, last = 0; i <= n; ++i) { int t = ptr[i]; ptr[i] = last; last = t; }
-        for (int i = 0; i < n; ++i) need(std::isfinite(b[i]) && std::isfinite(x[i]), SEMO_ERR_NAN, "non-finite rhs/guess");
         cudaStream_t s = c->stream;
-        semo::DBuf<int> dp, dc;
-        semo::DBuf<double> dv, db, dx;
-        dp.upload(ptr.data(), n + 1, s);
-        dc.upload(col.data(), nnz, s);
-        dv.upload(val.data(), nnz, s);
-        db.upload(b, n, s);
-        dx.upload(x, n, s);
+        semo::CooSystem S;
+        semo::coo_system(c, n, nnz, rows, cols, vals, 1, b, x, false, S);
         semo_solve_info inf{};
-        semo::solve_system(c, dp.p, dc.p, dv.p, n, nnz, db.p, dx.p, &inf, false);
-        SEMO_CUDA(cudaMemcpyAsync(x, dx.p, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
+        semo::solve_system(c, S.ptr.p, S.col.p, S.val.p, n, nnz, S.b.p, S.x.p, &inf, false);
+        SEMO_CUDA(cudaMemcpyAsync(x, S.x.p, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
         SEMO_CUDA(cudaStreamSynchronize(s));
         if (info) *info = inf;
         if (!(inf.rel_residual <= c->prm.tol)) conv = std::isfinite(inf.rel_residual) ? SEMO_ERR_NOT_CONVERGED : SEMO_ERR_NAN;
@@ -1194,43 +1177,12 @@ semo_status semo_solve_coo_multi(semo_ctx* c, int nrhs, int n, int64_t nnz, cons
         need(nnz < INT32_MAX, SEMO_ERR_ARGUMENT, "nnz too large");
         SEMO_CUDA(cudaSetDevice(c->device));
         // COO -> CSR as solveAMGCL.cpp:1129-1172 (stable: in-row order = COO order)
-        std::vector<int> ptr(n + 1, 0), col(nnz), dig(n, -1);
-        std::vector<double> val(nnz);
-        for (int64_t k = 0; k < nnz; ++k) {
-            need(rows[k] >= 0 && rows[k] < n && cols[k] >= 0 && cols[k] < n, SEMO_ERR_ARGUMENT, "COO index out of range");
-            need(std::isfinite(vals[k]), SEMO_ERR_NAN, "non-finite matrix value");
-            ptr[rows[k]]++;
-        }
-        for (int i = 0, t = 0; i < n; ++i) { int u = ptr[i]; ptr[i] = t; t += u; }
-        ptr[n] = (int)nnz;
-        for (int64_t k = 0; k < nnz; ++k) {
-            const int d = ptr[rows[k]]++;
-            col[d] = cols[k];
-            val[d] = vals[k];
-            if (cols[k] == rows[k] && dig[rows[k]] < 0) dig[rows[k]] = d;   // each row's first diagonal entry
-        }
-        for (int i = 0, last = 0; i <= n; ++i) { int t = ptr[i]; ptr[i] = last; last = t; }
-        for (int i = 0; i < n; ++i) {
-            need(dig[i] >= 0, SEMO_ERR_ARGUMENT, "row " + std::to_string(i) + " has no diagonal entry");
-            need(val[dig[i]] != 0.0, SEMO_ERR_ARGUMENT, "row " + std::to_string(i) + " has a zero diagonal");
-        }
-        bool guess = false;
-        for (int64_t i = 0; i < (int64_t)nrhs * n; ++i) {
-            need(std::isfinite(b[i]) && std::isfinite(x[i]), SEMO_ERR_NAN, "non-finite rhs/guess");
-            guess |= x[i] != 0.0;
-        }
         cudaStream_t s = c->stream;
-        semo::DBuf<int> dp, dc, dd;
-        semo::DBuf<double> dv, db, dx;
-        dp.upload(ptr.data(), n + 1, s);
-        dc.upload(col.data(), nnz, s);
-        dd.upload(dig.data(), n, s);
-        dv.upload(val.data(), nnz, s);
-        db.upload(b, (size_t)nrhs * n, s);
-        dx.upload(x, (size_t)nrhs * n, s);
+        semo::CooSystem S;
+        const bool guess = semo::coo_system(c, n, nnz, rows, cols, vals, nrhs, b, x, true, S);
         semo_solve_info inf[3] = {};
-        conv = semo::solve_csr_multi(c, n, dp.p, dc.p, dd.p, dv.p, nrhs, db.p, dx.p, guess, inf);
-        SEMO_CUDA(cudaMemcpyAsync(x, dx.p, sizeof(double) * nrhs * n, cudaMemcpyDeviceToHost, s));
+        conv = semo::solve_csr_multi(c, n, S.ptr.p, S.col.p, S.dig.p, S.val.p, nrhs, S.b.p, S.x.p, guess, inf);
+        SEMO_CUDA(cudaMemcpyAsync(x, S.x.p, sizeof(double) * nrhs * n, cudaMemcpyDeviceToHost, s));
         SEMO_CUDA(cudaStreamSynchronize(s));
         if (info) for (int j = 0; j < nrhs; ++j) info[j] = inf[j];
     });

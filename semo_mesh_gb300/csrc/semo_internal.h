@@ -388,6 +388,8 @@ void build_hierarchy(semo_ctx* c, Amg<V>& h, const int* ptr, const int* col, con
 // exclusive scan of d[0..n) on the stream; returns the total, read through
 // the pinned int *hpin (one host sync)
 int device_scan(cudaStream_t s, int* d, int n, int* hpin);
+// the same without the total and without the sync
+void device_scan_async(cudaStream_t s, int* d, int n);
 
 // pressure matrix values only (A_val: off-diagonals and diagonal, the values
 // assemble_pressure writes) on stream s, after assemble_face_values
@@ -423,6 +425,17 @@ semo_status solve_vof(semo_ctx* c, semo_solve_info* info);
 // when guess); info[nrhs]; returns the worst status as solve_momentum does
 semo_status solve_csr_multi(semo_ctx* c, int n, const int* ptr, const int* col, const int* dig, const double* val,
                             int nrhs, const double* b, double* x, bool guess, semo_solve_info* info);
+
+// coo.cu: a caller's COO system on the device -- CSR with each row in COO
+// order, dig (when wanted) each row's first diagonal place, b and x (nrhs
+// planes of n).  Returns whether the guess x has a value other than 0; throws
+// on a bad index, a non-finite value or (with dig) a missing or zero diagonal.
+struct CooSystem {
+    DBuf<int> ptr, col, dig;
+    DBuf<double> val, b, x;
+};
+bool coo_system(semo_ctx* c, int n, int64_t nnz, const int32_t* rows, const int32_t* cols, const double* vals,
+                int nrhs, const double* b, const double* x, bool want_dig, CooSystem& S);
 
 // momentum.cu (face_values_done: assemble_face_values(c, true) already ran)
 void assemble_momentum(semo_ctx* c, bool face_values_done = false);
