@@ -373,7 +373,7 @@ semo_status semo_vjp_fields(semo_ctx* ctx, const double* dJ_dx, double* lambda, 
    and VF are unchanged since the last full pass),"surface_tension";
    pressure "pface","pbface","pcell","amg_setup" (with "setup_aggregate",
    "setup_prolong","setup_galerkin","setup_level","setup_coarse",
-   "setup_cycle"),"pcg","vcycle","gauss_green","update"; momentum "mface",
+   "setup_cycle"; the levels built in one kernel count as "setup_galerkin"),"pcg","vcycle","gauss_green","update"; momentum "mface",
    "mbface","mcell","msolve","mupdate"; volume fraction "mstacs","vface",
    "vsolve","vupdate"; coupled "cgrad","cface","ccell","csolve","cupdate".  semo_stage_time returns the summed device time and
    number of timed calls since the last semo_reset_stats. */

@@ -27,6 +27,7 @@
 #include <cmath>
 #include <vector>
 
+#include "amg_rows.cuh"
 #include "semo_internal.h"
 
 namespace semo {
@@ -36,11 +37,7 @@ constexpr int kRedBlocks = 608;
 constexpr int kRedThreads = 256;
 inline int blocks(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
-__device__ __forceinline__ uint32_t hash_u32(uint32_t x) {
-    // integer avalanche mixer (public-domain "lowbias32" constants)
-    x ^= x >> 16; x *= 0x7feb352dU; x ^= x >> 15; x *= 0x846ca68bU; x ^= x >> 16;
-    return x;
-}
+using namespace semo::amg;
 
 // --------------------------------------------------------------------- scans
 constexpr int kScanT = 256, kScanItems = 8, kScanTile = kScanT * kScanItems;
@@ -193,11 +190,6 @@ __global__ void k_strength(int n, const int* __restrict__ ptr, const int* __rest
     }
     has = grp_sum<VS>(has);
     if (i < n && lane == 0) state[i] = has ? 1 : -1;   // -1: no strong connection, never aggregated
-}
-
-__device__ __forceinline__ unsigned long long mis_key(int st, int i) {
-    const unsigned long long s = (st < 0) ? 0ull : (unsigned long long)st;
-    return (s << 62) | ((unsigned long long)hash_u32((uint32_t)i) << 30) | (unsigned long long)i;
 }
 
 // need[i] marks the rows whose m1 an undecided row reads in the next round
@@ -553,57 +545,20 @@ __global__ void __launch_bounds__(128) k_spgemm_small(int n, const int* __restri
     }
 }
 
-// Row-wise SpGEMM C = A * B, one warp per row, open-addressing hash table in
-// shared memory.  Pass 0 counts distinct columns (flagging rows that fill
-// more than 3/4 of the table); pass 1 fills.  Products are consumed in a fixed
-// order (A entries in row order, B entries in chunks of 32) and summed as
-// 64-bit fixed-point integers (integer addition is associative, so the sums
-// do not depend on the order the shared-memory atomics land in): with
-// S = sum_k |a_ik| sum_j |b_kj| >= the row's sum of |products|, each product
-// is scaled by 2^s, S 2^s < 2^62, and rounded to an integer -- an error of at
-// most 2^-63 S per product, below what FP64 accumulation of the same
-// products incurs (2^-53 S per addition).  Occupied slots are compacted and
-// ranked by column, so output rows are sorted.
+// Row-wise SpGEMM C = A * B, one warp per row (hash_row in amg_rows.cuh): rows
+// of up to 3/4 of a table of HT slots, written to their slots (cptr) with
+// their lengths in cnt.  A row that fills the table is deferred to the next
+// launch, made with a larger one, or reported in overflow.
 constexpr int kGemmWarps = 4;
 
-// babs[k] = sum_j |b_kj| (FP64)
+// bmag[k] = sum_j |b_kj|, rounded up
 template <class V>
-__global__ void k_row_abs(int n, const int* __restrict__ ptr, const V* __restrict__ val, double* __restrict__ babs) {
+__global__ void k_row_size(int n, const int* __restrict__ ptr, const V* __restrict__ val, Mag* __restrict__ bmag) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    double s = 0.0;
-    for (int k = ptr[i]; k < ptr[i + 1]; ++k) s += fabs((double)val[k]);
-    babs[i] = s;
-}
-
-// round(a b 2^sc) to the nearest integer (ties to even) for finite floats,
-// on the integer pipes: the 24-bit significands multiply exactly into 48
-// bits, so this equals __double2ll_rn(((double)a * b) * 2^sc) (the FP64
-// product of two floats is exact too) without touching the FP64 unit.
-// Requires |a b| 2^sc < 2^62.
-__device__ __forceinline__ long long fixed_product(float a, float b, int sc) {
-    const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
-    int ea = (int)((ua >> 23) & 0xff), eb = (int)((ub >> 23) & 0xff);
-    const uint32_t ma = (ua & 0x7fffffu) | (ea ? 0x800000u : 0u);
-    const uint32_t mb = (ub & 0x7fffffu) | (eb ? 0x800000u : 0u);
-    ea = ea ? ea : 1;
-    eb = eb ? eb : 1;
-    const unsigned long long m = (unsigned long long)ma * (unsigned long long)mb;   // exact
-    const int e = (ea - 150) + (eb - 150) + sc;                                     // |a b| 2^sc = m 2^e
-    unsigned long long q;
-    if (m == 0ull) {
-        q = 0ull;
-    } else if (e >= 0) {
-        q = (e < 64) ? (m << e) : 0ull;   // e <= 61 whenever the scale bound holds
-    } else if (e <= -64) {
-        q = 0ull;   // below half a unit (m < 2^48)
-    } else {
-        const int sh = -e;
-        q = m >> sh;
-        const unsigned long long rem = m & ((1ull << sh) - 1ull), half = 1ull << (sh - 1);
-        if (rem > half || (rem == half && (q & 1ull))) ++q;
-    }
-    return ((ua ^ ub) >> 31) ? -(long long)q : (long long)q;
+    Mag s{0.0f, kMagNone};
+    for (int k = ptr[i]; k < ptr[i + 1]; ++k) mag_add(s, mag_of(val[k]));
+    bmag[i] = s;
 }
 
 template <class V, int HT>
@@ -611,155 +566,30 @@ __global__ void __launch_bounds__(32 * kGemmWarps) k_spgemm(int n, const int* __
                                                             const int* __restrict__ acol, const V* __restrict__ aval,
                                                             const int* __restrict__ bptr, const int* __restrict__ bcol,
                                                             const V* __restrict__ bval,
-                                                            const double* __restrict__ babs, int pass,
-                                                            int* __restrict__ cnt, const int* __restrict__ cptr,
-                                                            int* __restrict__ ccol, V* __restrict__ cval,
-                                                            int* __restrict__ overflow,
-                                                            const int* __restrict__ small, int defer,
-                                                            int* __restrict__ list, int* __restrict__ nlist) {
+                                                            const Mag* __restrict__ bmag, int* __restrict__ cnt,
+                                                            const int* __restrict__ cptr, int* __restrict__ ccol,
+                                                            V* __restrict__ cval, int* __restrict__ overflow,
+                                                            int defer, int* __restrict__ list,
+                                                            int* __restrict__ nlist) {
     extern __shared__ unsigned char smem[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // per warp: keys[HT] int, ckeys[HT] int, vals[HT] and cvals[HT] 64-bit fixed point
-    int* keys = reinterpret_cast<int*>(smem) + wid * 2 * HT;
-    int* ckeys = keys + HT;
-    unsigned long long* vals =
-        reinterpret_cast<unsigned long long*>(smem + sizeof(int) * 2 * HT * kGemmWarps) + wid * 2 * HT;
-    unsigned long long* cvals = vals + HT;
+    RowTable tb;
+    tb.keys = reinterpret_cast<int*>(smem) + wid * 2 * HT;
+    tb.ckeys = tb.keys + HT;
+    tb.vals = reinterpret_cast<unsigned long long*>(smem + sizeof(int) * 2 * HT * kGemmWarps) + wid * 2 * HT;
+    tb.cvals = tb.vals + HT;
     // rows: all of them, or (list given, defer 0) the ones a previous launch deferred
     const int nrows = (list && !defer) ? *nlist : n;
     for (int idx = blockIdx.x * kGemmWarps + wid; idx < nrows; idx += gridDim.x * kGemmWarps) {
         const int row = (list && !defer) ? list[idx] : idx;
-        if (small && small[row] >= 0) {   // the row was done by the thread-per-row kernel
-            if (pass == 0 && lane == 0) cnt[row] = small[row];
-            continue;
-        }
-        __syncwarp();
-        // table size for this row (power of two, 32..HT): from the product
-        // count in the counting pass, from the known column count when filling
-        int need;
-        if (pass == 0) {
-            int prod = 0;
-            for (int ka = aptr[row] + lane; ka < aptr[row + 1]; ka += 32) prod += bptr[acol[ka] + 1] - bptr[acol[ka]];
-            for (int o = 16; o > 0; o >>= 1) prod += __shfl_xor_sync(0xffffffffu, prod, o);
-            need = 2 * prod;
-        } else {
-            need = (4 * (cptr[row + 1] - cptr[row])) / 3 + 2;
-        }
-        int ht = 32;
-        while (ht < need && ht < HT) ht <<= 1;
-        const int hmask = ht - 1;
-        for (int t = lane; t < ht; t += 32) { keys[t] = -1; vals[t] = 0ull; }
-        // the row's fixed-point scale 2^sc (a fixed reduction tree: deterministic)
-        double up_scale = 1.0, down_scale = 1.0;
-        int sc = 0;
-        if (pass != 0) {
-            double bound = 0.0;
-            for (int ka = aptr[row] + lane; ka < aptr[row + 1]; ka += 32)
-                bound += fabs((double)aval[ka]) * babs[acol[ka]];
-            for (int o = 16; o > 0; o >>= 1) bound += __shfl_xor_sync(0xffffffffu, bound, o);
-            // bound < 2^e with e from the biased exponent (subnormals: e = -1022)
-            const int be = (int)((__double_as_longlong(bound) >> 52) & 0x7ff);
-            const int e = be ? be - 1022 : -1022;
-            sc = max(-960, min(1000, 62 - e));
-            up_scale = __longlong_as_double((long long)(1023 + sc) << 52);     // 2^sc
-            down_scale = __longlong_as_double((long long)(1023 - sc) << 52);   // 2^-sc
-        }
-        __syncwarp();
-        int distinct = 0;
-        bool full = false;
-        // Products are taken in a fixed flattened order: up to 32 A entries at
-        // a time, their B rows laid end to end, 32 products per step.
-        const int ab = aptr[row], ae = aptr[row + 1];
-        for (int k0 = ab; k0 < ae && !full; k0 += 32) {
-            const int k = k0 + lane;
-            const bool ka = k < ae;
-            const int a = ka ? acol[k] : 0;
-            const V avk = ka ? aval[k] : V(0);
-            const int bb = ka ? bptr[a] : 0;
-            const int blen = ka ? bptr[a + 1] - bb : 0;
-            int incl = blen;   // inclusive scan of the B row lengths over the lanes
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += t;
-            }
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            const int excl = incl - blen;
-            for (int t0 = 0; t0 < total; t0 += 32) {
-                const int t = t0 + lane;
-                const bool act = t < total;
-                // owner lane: the last lane whose B-row run starts at or before t
-                int j = 0;
-#pragma unroll
-                for (int step = 16; step >= 1; step >>= 1) {
-                    const int e = __shfl_sync(0xffffffffu, excl, j + step);
-                    if (e <= t) j += step;
-                }
-                const int q = __shfl_sync(0xffffffffu, bb, j) + (t - __shfl_sync(0xffffffffu, excl, j));
-                const V av = __shfl_sync(0xffffffffu, avk, j);
-                const int c = act ? bcol[q] : -1;
-                int slot = -1;
-                bool fresh = false;
-                if (act) {
-                    uint32_t h = hash_u32((uint32_t)c) & hmask;
-                    for (int probe = 0; probe < ht; ++probe) {
-                        const int prev = atomicCAS(keys + h, -1, c);
-                        if (prev == -1) { slot = (int)h; fresh = true; break; }
-                        if (prev == c) { slot = (int)h; break; }
-                        h = (h + 1) & hmask;
-                    }
-                }
-                distinct += __popc(__ballot_sync(0xffffffffu, fresh));
-                const bool lost = __any_sync(0xffffffffu, act && slot < 0);
-                if (pass != 0 && !lost && act) {
-                    long long fx;
-                    if constexpr (sizeof(V) == 4) fx = fixed_product(av, bval[q], sc);
-                    else fx = __double2ll_rn((av * bval[q]) * up_scale);
-                    atomicAdd(vals + slot, (unsigned long long)fx);   // two's complement: signed sum mod 2^64
-                }
-                __syncwarp();
-                if (lost || distinct > (ht * 3) / 4) { full = true; break; }
-            }
-        }
-        if (full && pass == 2 && defer) {
-            // single pass: a row that fills this launch's table is left for
-            // the next launch, made with a larger one (it has written nothing)
-            if (lane == 0) list[atomicAdd(nlist, 1)] = row;   // list order does not affect any result
-            __syncwarp();
-            continue;
-        }
-        if (full) {
-            if (lane == 0) atomicExch(overflow, 1);
-            if (pass != 1 && lane == 0) cnt[row] = 0;
-            __syncwarp();
-            continue;
-        }
-        if (pass == 0) {
-            if (lane == 0) cnt[row] = distinct;
-        } else {
-            // compact occupied slots (slot order), then rank by column
-            int base_c = 0;
-            for (int t0 = 0; t0 < ht; t0 += 32) {
-                const int t = t0 + lane;
-                const bool occ = keys[t] >= 0;
-                const unsigned bal = __ballot_sync(0xffffffffu, occ);
-                if (occ) {
-                    const int pos = base_c + __popc(bal & ((1u << lane) - 1u));
-                    ckeys[pos] = keys[t];
-                    cvals[pos] = vals[t];
-                }
-                base_c += __popc(bal);
-            }
-            if (pass == 2 && lane == 0) cnt[row] = base_c;
-            __syncwarp();
-            const int out = cptr[row];
-            for (int e = lane; e < base_c; e += 32) {
-                const int ce = ckeys[e];
-                int rank = 0;
-                for (int u = 0; u < base_c; ++u) rank += (ckeys[u] < ce);
-                ccol[out + rank] = ce;
-                cval[out + rank] = (V)((double)(long long)cvals[e] * down_scale);
-            }
+        if (cnt[row] >= 0) continue;   // done by the thread-per-row kernel
+        const int out = cptr[row];
+        const int m = hash_row<V>(lane, table_size(cptr[row + 1] - out, HT), tb, aptr[row], aptr[row + 1], acol, aval,
+                                  RowSpan{bptr, nullptr}, bcol, bval, bmag, ccol + out, cval + out);
+        if (lane == 0) {
+            if (m >= 0) cnt[row] = m;
+            else if (defer) list[atomicAdd(nlist, 1)] = row;   // list order does not affect any result
+            else { atomicExch(overflow, 1); cnt[row] = 0; }
         }
         __syncwarp();
     }
@@ -837,12 +667,10 @@ int pick_vs(const DCsr<V>& A) {
 }
 
 template <class V>
-void spgemm_pass(cudaStream_t s, int ht, int pass, const DCsr<V>& A, const DCsr<V>& B, const double* babs,
-                 DCsr<V>& C, int* cnt,
-                 int* overflow, const int* small, const int* cptr, int* ccol, V* cval, int defer, int* list,
-                 int* nlist) {
+void spgemm_rows(cudaStream_t s, int ht, const DCsr<V>& A, const DCsr<V>& B, const Mag* bmag, int* cnt,
+                 int* overflow, const int* cptr, int* ccol, V* cval, int defer, int* list, int* nlist) {
     const int n = A.n;
-    const size_t shm = (size_t)kGemmWarps * ht * 2 * (sizeof(int) + sizeof(double));
+    const size_t shm = (size_t)kGemmWarps * ht * kTableSlotBytes;
     // grid-stride over the rows, 32 blocks a multiprocessor (the sums are exact
     // integers, so the grid does not change the result)
     int dev = 0;
@@ -852,9 +680,8 @@ void spgemm_pass(cudaStream_t s, int ht, int pass, const DCsr<V>& A, const DCsr<
     case H:                                                                                                      \
         if (shm > 48 * 1024)                                                                                     \
             SEMO_CUDA(cudaFuncSetAttribute(k_spgemm<V, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm)); \
-        k_spgemm<V, H><<<grid, 32 * kGemmWarps, shm, s>>>(n, A.ptr, A.col, A.val, B.ptr, B.col, B.val, babs, pass, \
-                                                           cnt,                                                  \
-                                                           cptr, ccol, cval, overflow, small, defer, list, nlist); \
+        k_spgemm<V, H><<<grid, 32 * kGemmWarps, shm, s>>>(n, A.ptr, A.col, A.val, B.ptr, B.col, B.val, bmag, cnt, \
+                                                           cptr, ccol, cval, overflow, defer, list, nlist);       \
         break;
     switch (ht) {
         SEMO_GEMM_CASE(64)
@@ -914,14 +741,14 @@ void spgemm(cudaStream_t s, semo_ctx* c, const DCsr<V>& A, const DCsr<V>& B, DCs
             nlist.alloc(1, s);
             nlist.zero();
         }
-        DBuf<double> babs;   // per B row sum of |b|: the fixed-point scales
-        babs.alloc(std::max(B.n, 1), s);
-        k_row_abs<V><<<blocks(B.n, 256), 256, 0, s>>>(B.n, B.ptr, B.val, babs);
+        DBuf<Mag> bmag;   // per B row sum of |b|: the fixed-point scales
+        bmag.alloc(std::max(B.n, 1), s);
+        k_row_size<V><<<blocks(B.n, 256), 256, 0, s>>>(B.n, B.ptr, B.val, bmag);
         SEMO_CHECK_LAUNCH();
-        spgemm_pass(s, first, 2, A, B, babs.p, C, cnt.p, flags.p, cnt.p, up.p, tcol.p, tval.p, ht > first ? 1 : 0,
-                    list.p, nlist.p);
+        spgemm_rows(s, first, A, B, bmag.p, cnt.p, flags.p, up.p, tcol.p, tval.p, ht > first ? 1 : 0, list.p,
+                    nlist.p);
         if (ht > first)
-            spgemm_pass(s, ht, 2, A, B, babs.p, C, cnt.p, flags.p, cnt.p, up.p, tcol.p, tval.p, 0, list.p, nlist.p);
+            spgemm_rows(s, ht, A, B, bmag.p, cnt.p, flags.p, up.p, tcol.p, tval.p, 0, list.p, nlist.p);
     }
     SEMO_CUDA(cudaMemcpyAsync(C.ptr.p, cnt.p, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
     SEMO_CUDA(cudaMemsetAsync(C.ptr.p + n, 0, sizeof(int), s));
@@ -1022,8 +849,24 @@ void amg_setup(semo_ctx* c, Amg<V>& h, const int* ptr, const int* col, const dou
     }
     float eps = (float)c->prm.eps_strong;
     const double omega = 2.0 / 3.0;
+    int* const hf = c->hpin_int + 8;   // sflag[0..5)
+    auto read_back = [&] {             // the bounds and flags of the levels built here
+        SEMO_CUDA(cudaMemcpyAsync(c->hpin_setup, lam_dev.p, sizeof(double) * 64, cudaMemcpyDeviceToHost, s));
+        SEMO_CUDA(cudaMemcpyAsync(hf, c->sflag.p, 5 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    };
+    SmallResult small = SmallResult::no_room;
+    bool try_small = true;
+    int above = 0;   // levels built here
     for (int l = 0;; ++l) {
         AmgLevel<V>& L = h.lev[l];
+        if (try_small && small_setup_fits(L.A.n, L.A.nnz, s != c->stream)) {
+            StageScope sc(c, ST_SETUP_GALERKIN);
+            read_back();
+            small = small_setup(c, h, eps, omega, hf);
+            if (small != SmallResult::no_room) break;
+            try_small = false;   // the levels below are taken here too
+        }
+        above = l + 1;
         DBuf<V> dia;
         {
             StageScope sc(c, ST_SETUP_LEVEL);
@@ -1157,25 +1000,24 @@ void amg_setup(semo_ctx* c, Amg<V>& h, const int* ptr, const int* col, const dou
         spgemm(s, c, Lf.R, AP, Lc.A);
         Lc.A.m = Lc.A.n;
     }
-    StageScope scs(c, ST_SETUP_COARSE);
-    // coarsest level: explicit FP64 inverse (Gauss-Jordan, partial pivoting)
-    AmgLevel<V>& Lc = h.lev.back();
-    const int m = Lc.A.n;
-    if (m > 4096) throw Error(SEMO_ERR_CUDA, "AMG coarsening stalled above 4096 rows");
-    h.coarse_n = m;
-    DBuf<double> dense;
-    dense.alloc((size_t)m * m, s);
-    h.cinv.alloc((size_t)m * m, s);
-    k_dense<V><<<1, 1024, 0, s>>>(m, Lc.A.ptr, Lc.A.col, Lc.A.val, dense);
-    SEMO_CHECK_LAUNCH();
-    k_gauss_jordan<<<1, 1024, 0, s>>>(m, dense, h.cinv, c->sflag);
-    SEMO_CHECK_LAUNCH();
-    int* const hf = c->hpin_int + 8;   // sflag[0..5)
-    const int nlev = (int)h.lev.size();
-    SEMO_CUDA(cudaMemcpyAsync(c->hpin_setup, lam_dev.p, sizeof(double) * nlev, cudaMemcpyDeviceToHost, s));
-    SEMO_CUDA(cudaMemcpyAsync(hf, c->sflag.p, 5 * sizeof(int), cudaMemcpyDeviceToHost, s));
-    SEMO_CUDA(cudaStreamSynchronize(s));
-    for (int l = 0; l < nlev; ++l) h.lev[l].lam_max = c->hpin_setup[l];
+    if (small != SmallResult::done) {
+        StageScope scs(c, ST_SETUP_COARSE);
+        // coarsest level: explicit FP64 inverse (Gauss-Jordan, partial pivoting)
+        AmgLevel<V>& Lc = h.lev.back();
+        const int m = Lc.A.n;
+        if (m > 4096) throw Error(SEMO_ERR_CUDA, "AMG coarsening stalled above 4096 rows");
+        h.coarse_n = m;
+        DBuf<double> dense;
+        dense.alloc((size_t)m * m, s);
+        h.cinv.alloc((size_t)m * m, s);
+        k_dense<V><<<1, 1024, 0, s>>>(m, Lc.A.ptr, Lc.A.col, Lc.A.val, dense);
+        SEMO_CHECK_LAUNCH();
+        k_gauss_jordan<<<1, 1024, 0, s>>>(m, dense, h.cinv, c->sflag);
+        SEMO_CHECK_LAUNCH();
+        read_back();
+        SEMO_CUDA(cudaStreamSynchronize(s));
+    }
+    for (int l = 0; l < above; ++l) h.lev[l].lam_max = c->hpin_setup[l];
     if (hf[2]) throw Error(SEMO_ERR_ARGUMENT, "matrix has a zero diagonal entry");
     if (hf[3]) throw Error(SEMO_ERR_NAN, "non-finite matrix entry");
     if (hf[4]) throw Error(SEMO_ERR_BREAKDOWN, "coarsest AMG matrix is singular");

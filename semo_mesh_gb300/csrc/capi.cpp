@@ -156,6 +156,7 @@ semo_status semo_ctx_destroy(semo_ctx* c) {
     if (c->hpin) cudaFreeHost(c->hpin);
     if (c->hpin_int) cudaFreeHost(c->hpin_int);
     if (c->hpin_setup) cudaFreeHost(c->hpin_setup);
+    if (c->hpin_small) cudaFreeHost(c->hpin_small);
     if (c->hpin_scan) cudaFreeHost(c->hpin_scan);
     cudaStream_t s = c->stream, aux = c->aux_stream;
     delete c;  // DBuf destructors enqueue frees on the (still valid) streams

@@ -56,12 +56,13 @@ struct DBuf {
     T* p = nullptr;
     size_t n = 0;
     cudaStream_t s = 0;
+    bool owned = true;   // false: a view of memory another buffer owns
     DBuf() = default;
     DBuf(const DBuf&) = delete;
     DBuf& operator=(const DBuf&) = delete;
     DBuf(DBuf&& o) noexcept { *this = std::move(o); }
     DBuf& operator=(DBuf&& o) noexcept {
-        if (this != &o) { release(); p = o.p; n = o.n; s = o.s; o.p = nullptr; o.n = 0; }
+        if (this != &o) { release(); p = o.p; n = o.n; s = o.s; owned = o.owned; o.p = nullptr; o.n = 0; o.owned = true; }
         return *this;
     }
     ~DBuf() { release(); }
@@ -77,9 +78,12 @@ struct DBuf {
         alloc(count, st);
         if (count) SEMO_CUDA(cudaMemcpyAsync(p, h, sizeof(T) * count, cudaMemcpyHostToDevice, st));
     }
+    void view(T* q, size_t count) { release(); p = q; n = count; owned = false; }
     void release() {
-        if (p) { cudaFreeAsync(p, s); p = nullptr; }
+        if (p && owned) cudaFreeAsync(p, s);
+        p = nullptr;
         n = 0;
+        owned = true;
     }
     operator T*() const { return p; }
 };
@@ -109,8 +113,9 @@ struct Amg {
     int coarse_n = 0;
     DBuf<double> cinv;     // explicit FP64 inverse of the coarsest matrix (row-major)
     int64_t total_nnz = 0;
+    DBuf<unsigned char> arena;   // the small levels' arrays (amg_small.cu)
     bool ready = false;
-    void clear() { lev.clear(); cinv.release(); coarse_n = 0; total_nnz = 0; ready = false; }
+    void clear() { lev.clear(); cinv.release(); arena.release(); coarse_n = 0; total_nnz = 0; ready = false; }
 };
 
 struct Timer {
@@ -255,6 +260,7 @@ struct semo_ctx {
     int* hpin_scan = nullptr;                     // context's stream: scan totals and flags (kHostInts)
     int* hpin_int = nullptr;                      // setup: counters and scan totals (kHostInts)
     double* hpin_setup = nullptr;                 // setup: per-level scalars (kHostScalars)
+    void* hpin_small = nullptr;                   // setup: records of the small levels (amg_small.cu)
     cudaEvent_t sync_ev[2] = {nullptr, nullptr};  // completion of those counter copies
     std::shared_ptr<void> apply;                  // V-cycle/Krylov apply state (cycle.cu)
     std::shared_ptr<void> setup_worker;           // host thread of the overlapped pressure setup (capi.cpp)
@@ -384,6 +390,15 @@ double coupled_update(semo_ctx* c);
 template <class V>
 void build_hierarchy(semo_ctx* c, Amg<V>& h, const int* ptr, const int* col, const double* val, int n,
                      int64_t nnz);
+// amg_small.cu: every level from h.lev.back() (its A set) down to the coarsest
+// in one kernel.  done: the hierarchy is complete; needs_inverse: all but the
+// coarsest level's inverse; no_room: nothing was built (the level-by-level
+// kernels take it).  Waits for the stream; sflag is then read: the error flags
+// of the levels above, whose copy the caller queued
+enum class SmallResult { done, needs_inverse, no_room };
+bool small_setup_fits(int n, int64_t nnz, bool beside);   // beside: kernels of another stream run meanwhile
+template <class V>
+SmallResult small_setup(semo_ctx* c, Amg<V>& h, float eps, double omega, const int* sflag);
 // exclusive scan of d[0..n) in place on the context's stream; returns the total
 // exclusive scan of d[0..n) on the stream; returns the total, read through
 // the pinned int *hpin (one host sync)
