@@ -65,6 +65,7 @@ constexpr int kSoloRows = 64, kSoloNnz = 1024;
 
 struct SmallRec {
     int n, nnz, nagg, nnzP;
+    int runA, runP, runR;     // entries of the longest cluster run of rows
     long long dinv, Pptr, Pcol, Pval, Rptr, Rcol, Rval, Aptr, Acol, Aval;   // arena offsets (bytes)
     unsigned long long lam;   // bits of the Gershgorin bound
 };
@@ -349,6 +350,12 @@ __device__ void block_product(const SmallArgs<V>& a, int level, int c0, int c1, 
     __syncthreads();
 }
 
+// *most = entries of the longest cluster run of n rows
+__device__ __forceinline__ void longest_run(int n, const int* ptr, int* most) {
+    const int k = blockIdx.x * kT + threadIdx.x, ch = cluster_run(n);
+    if (k < kClusterBlocks) atomicMax(most, ptr[min(n, (k + 1) * ch)] - ptr[min(n, k * ch)]);
+}
+
 template <class V>
 __global__ void __launch_bounds__(kT, 1) k_small_setup(SmallArgs<V> a) {
     extern __shared__ unsigned long long sm64[];
@@ -398,6 +405,7 @@ __global__ void __launch_bounds__(kT, 1) k_small_setup(SmallArgs<V> a) {
         V* const dia = reinterpret_cast<V*>(a.arena + temp((long long)n * sizeof(V)));
         SMALL_ROOM();
         if (first) { rec.n = n; rec.nnz = nnz; rec.dinv = o_dinv; }
+        longest_run(n, ptr, &rec.runA);
         const int vs = lanes_for(n, nnz, GT), rpw = 32 / vs, sub = lane % vs;
         // diagonal, its reciprocal, the Gershgorin bound of D^-1 A
         double ratio = 0.0;
@@ -697,6 +705,7 @@ __global__ void __launch_bounds__(kT, 1) k_small_setup(SmallArgs<V> a) {
             }
         }
         SMALL_SYNC();
+        longest_run(n, pptr, &rec.runP);
         // R's row counts; A P of the block's rows
         const int qh = (nagg + G - 1) / G, q0 = min(nagg, cta * qh), q1 = min(nagg, q0 + qh);
         {
@@ -722,6 +731,7 @@ __global__ void __launch_bounds__(kT, 1) k_small_setup(SmallArgs<V> a) {
             }
         }
         SMALL_SYNC();
+        longest_run(nagg, rptr, &rec.runR);
         for (int i = gt; i < n; i += GT)
             for (int k = pptr[i]; k < pptr[i + 1]; ++k) {
                 const int d = atomicAdd(fill + pcol[k], 1);
@@ -962,6 +972,9 @@ SmallResult small_setup(semo_ctx* c, Amg<V>& h, float eps, double omega, const i
             vals(L.A.val, q.Aval, q.nnz);
         }
         AmgLevel<V>& L = h.lev.back();
+        L.A.run = q.runA;
+        L.P.run = q.runP;
+        L.R.run = q.runR;
         vals(L.dinv, q.dinv, q.n);
         std::memcpy(&L.lam_max, &q.lam, sizeof(double));
         h.total_nnz += q.nnz;

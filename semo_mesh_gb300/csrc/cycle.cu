@@ -32,7 +32,7 @@ namespace {
 
 // Grid of the kernels that end in a reduction (dot products fused into the
 // SpMVs and vector updates), grid-stride: a fixed 608-way partition of the
-// rows, one partial sum per block, summed in a fixed order.  608 is 4 blocks
+// rows at most (a block per 256 rows below that), one partial sum per block, summed in a fixed order.  608 is 4 blocks
 // of 256 per multiprocessor on GB300's 152 (measured faster here than 16 a
 // multiprocessor); it is not taken from the device so that the partition,
 // and with it every sum's bits, is the same on any GPU.
@@ -44,19 +44,29 @@ __device__ __forceinline__ double warp_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     return v;
 }
+// sum over a block of kRedThreads (sh: kRedThreads doubles), in thread 0.  The
+// values go through shared memory to one warp: a shuffle tree in every warp is
+// 40 FP64 warp instructions of 16 clocks a multiprocessor each where this is 12.
 __device__ __forceinline__ double block_sum(double v, double* sh) {
-    v = warp_sum(v);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) sh[wid] = v;
+    __syncthreads();   // sh may still be read
+    sh[threadIdx.x] = v;
     __syncthreads();
-    v = 0.0;
     if (threadIdx.x < 32) {
-        v = (lane < (int)(blockDim.x >> 5)) ? sh[lane] : 0.0;
+        v = sh[threadIdx.x];
+#pragma unroll
+        for (int k = 1; k < kRedThreads / 32; ++k) v += sh[threadIdx.x + 32 * k];
         v = warp_sum(v);
     }
-    __syncthreads();
     return v;
 }
+// sum of a kernel's nb partial sums, by one warp (every lane gets it)
+__device__ __forceinline__ double parts_sum(const double* part, int nb) {
+    double s = 0.0;
+    for (int i = threadIdx.x & 31; i < nb; i += 32) s += part[i];
+    return __shfl_sync(0xffffffffu, warp_sum(s), 0);
+}
+// blocks of a reducing kernel over n rows
+inline int red_blocks(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>(kRedBlocks, (n + kRedThreads - 1) / kRedThreads)); }
 
 // ------------------------------------------------------------ matrix views
 // CSR with VS lanes per row.
@@ -324,7 +334,7 @@ __global__ void __launch_bounds__(kRedThreads) k_post1_dots(M A, const V* __rest
                                                             const double* __restrict__ q,
                                                             double* __restrict__ part) {
     pdl_enter();
-    __shared__ double sh[32];
+    __shared__ double sh[kRedThreads];
     double zr = 0.0, zq = 0.0;
     const int per_block = blockDim.x / M::kVS, lane = threadIdx.x % M::kVS;
     for (int row0 = blockIdx.x * per_block; row0 < A.n; row0 += gridDim.x * per_block) {
@@ -333,8 +343,9 @@ __global__ void __launch_bounds__(kRedThreads) k_post1_dots(M A, const V* __rest
         if (row < A.n && lane == 0) {
             const V zi = y[row] + c1 * d[row] + c2 * (dinv[row] * (b[row] - s));
             z[row] = zi;
-            zr += (double)zi * r[row];
-            zq += (double)zi * q[row];
+            const double zd = (double)(zi);
+            zr += zd * r[row];
+            zq += zd * q[row];
         }
     }
     zr = block_sum(zr, sh);
@@ -379,68 +390,77 @@ __global__ void k_coarse_solve(int n, const double* __restrict__ inv, const V* _
 }
 
 // ---------------------------------------------------------- CG kernels
-// device scalars: 0 rz, 1 zq, 2 pq, 3 rr, 4 alpha_prev, 5 beta, 6 alpha,
-// 7 rz_prev, 8/9 scratch, 10 iteration count
-__device__ __forceinline__ double sum_parts(const double* part, double* sh) {
+// device scalars: 0 rz, 2 pq, 4 alpha of the last iteration, 7 its rz, 10
+// iterations begun, 11 b.b, 12 r0.r0, 13 iterations done, 14 status, 16 the
+// true residual's r.r
+// sum of nb partial sums by a block of kRedThreads, in thread 0
+__device__ __forceinline__ double sum_parts(const double* part, int nb, double* sh) {
     double s = 0.0;
-    for (int i = threadIdx.x; i < kRedBlocks; i += blockDim.x) s += part[i];
+    for (int i = threadIdx.x; i < nb; i += blockDim.x) s += part[i];
     return block_sum(s, sh);
 }
-__global__ void k_fin_beta(const double* __restrict__ part, double* __restrict__ scal) {
-    pdl_enter();
-    __shared__ double sh[32];
-    const double rz = sum_parts(part, sh);
-    const double zq = sum_parts(part + kRedBlocks, sh);
-    if (threadIdx.x == 0) {
-        scal[0] = rz;
-        scal[1] = zq;
-        // Polak-Ribiere: beta = z.(r_k - r_{k-1}) / (z_{k-1}.r_{k-1}) = -alpha_{k-1} z.q_{k-1} / rz_prev
-        scal[5] = (scal[10] == 0.0) ? 0.0 : (-scal[4] * zq / scal[7]);
-        scal[7] = rz;
-        scal[10] += 1.0;
-    }
-}
-// w = A z;  q = w + beta q;  p = z + beta p;  part = p.q   (FP64 SELL operator)
+// The scalars of an iteration are formed by the kernels that use them, each
+// block adding the producer's partial sums itself (one warp): a kernel of their
+// own for beta, alpha and r.r cost ~2.75 us each.  Block 0 keeps what later
+// kernels need; no block reads a scalar that this kernel writes.
+// beta from z.r and z.q (part);  w = A z;  q = w + beta q;  p = z + beta p;
+// ppq = p.q   (FP64 SELL operator)
 template <class M, class Z>
 __global__ void __launch_bounds__(kRedThreads) k_outer_mv(M A, const Z* __restrict__ z,
                                                           double* __restrict__ p, double* __restrict__ q,
-                                                          const double* __restrict__ scal,
-                                                          double* __restrict__ part) {
+                                                          double* __restrict__ scal,
+                                                          const double* __restrict__ part, int nb,
+                                                          double* __restrict__ ppq) {
     pdl_enter();
-    __shared__ double sh[32];
-    const double beta = scal[5];
+    __shared__ double sh[kRedThreads], sbeta;
+    if (threadIdx.x < 32) {
+        const double rz = parts_sum(part, nb);
+        // Polak-Ribiere: beta = z.(r_k - r_{k-1}) / (z_{k-1}.r_{k-1}) = -alpha_{k-1} z.q_{k-1} / rz_prev
+        const double bt = scal[10] == 0.0 ? 0.0 : -scal[4] * parts_sum(part + kRedBlocks, nb) / scal[7];
+        if (threadIdx.x == 0) {
+            sbeta = bt;
+            if (blockIdx.x == 0) scal[0] = rz;
+        }
+    }
+    __syncthreads();
+    const double beta = sbeta;
     double pq = 0.0;
     const int stride = gridDim.x * blockDim.x;
     for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n; row += stride) {
         const double w = A.dot(row, 0, Vec<double, Z>{z});
         const double qi = w + beta * q[row];
-        const double pi = (double)z[row] + beta * p[row];
+        const double pi = (double)(z[row]) + beta * p[row];
         q[row] = qi;
         p[row] = pi;
         pq += pi * qi;
     }
     pq = block_sum(pq, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = pq;
+    if (threadIdx.x == 0) ppq[blockIdx.x] = pq;
 }
-__global__ void k_fin_alpha(const double* __restrict__ part, double* __restrict__ scal) {
-    pdl_enter();
-    __shared__ double sh[32];
-    const double pq = sum_parts(part, sh);
-    if (threadIdx.x == 0) {
-        scal[2] = pq;
-        scal[6] = scal[7] / pq;
-        scal[4] = scal[6];
-    }
-}
-// x += alpha p;  r -= alpha q;  rv = r in the V-cycle's type;  part = r.r
+// alpha from p.q (ppq);  x += alpha p;  r -= alpha q;  rv = r in the V-cycle's
+// type;  part = r.r
 template <class V>
 __global__ void __launch_bounds__(kRedThreads) k_xr(int n, double* __restrict__ x, double* __restrict__ r,
                                                     V* __restrict__ rv, const double* __restrict__ p,
-                                                    const double* __restrict__ q, const double* __restrict__ scal,
+                                                    const double* __restrict__ q, double* __restrict__ scal,
+                                                    const double* __restrict__ ppq, int nb,
                                                     double* __restrict__ part) {
     pdl_enter();
-    __shared__ double sh[32];
-    const double alpha = scal[6];
+    __shared__ double sh[kRedThreads], salpha;
+    if (threadIdx.x < 32) {
+        const double pq = parts_sum(ppq, nb), rz = scal[0];
+        if (threadIdx.x == 0) {
+            salpha = rz / pq;
+            if (blockIdx.x == 0) {
+                scal[2] = pq;
+                scal[4] = rz / pq;
+                scal[7] = rz;
+                scal[10] += 1.0;
+            }
+        }
+    }
+    __syncthreads();
+    const double alpha = salpha;
     double s = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         x[i] += alpha * p[i];
@@ -452,20 +472,20 @@ __global__ void __launch_bounds__(kRedThreads) k_xr(int n, double* __restrict__ 
     s = block_sum(s, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
-__global__ void k_fin_rr(const double* __restrict__ part, double* __restrict__ scal) {
-    pdl_enter();
-    __shared__ double sh[32];
-    const double rr = sum_parts(part, sh);
-    if (threadIdx.x == 0) scal[3] = rr;
+// out[0] = sum of nb partial sums
+__global__ void k_fin_sum(const double* __restrict__ part, int nb, double* __restrict__ out) {
+    __shared__ double sh[kRedThreads];
+    const double s = sum_parts(part, nb, sh);
+    if (threadIdx.x == 0) out[0] = s;
 }
 // generic dots for the non-fused path: part = a.b, part+R = a.c
 template <class A>
 __global__ void __launch_bounds__(kRedThreads) k_dot2(int n, const A* __restrict__ a, const double* __restrict__ b,
                                                       const double* __restrict__ c, double* __restrict__ part) {
-    __shared__ double sh[32];
+    __shared__ double sh[kRedThreads];
     double s = 0.0, t = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double ai = (double)a[i];
+        const double ai = (double)(a[i]);
         s += ai * b[i];
         t += ai * c[i];
     }
@@ -475,7 +495,7 @@ __global__ void __launch_bounds__(kRedThreads) k_dot2(int n, const A* __restrict
 }
 __global__ void __launch_bounds__(kRedThreads) k_dot(int n, const double* __restrict__ a, const double* __restrict__ b,
                                                      double* __restrict__ part) {
-    __shared__ double sh[32];
+    __shared__ double sh[kRedThreads];
     double s = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += a[i] * b[i];
     s = block_sum(s, sh);
@@ -743,7 +763,10 @@ struct LevelMats {
 template <class V>
 struct Cycle {
     std::vector<LevelMats<V>> lev;
+    int local_from = -1;   // first level of k_local_cycle
 };
+
+#include "cycle_cluster.cuh"
 
 // run f on the SELL view of a level operator if it has one, else on CSR
 template <class V, class F>
@@ -921,6 +944,12 @@ template <class V>
 void vcycle_from(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, int l) {
     cudaStream_t s = c->stream;
     AmgLevel<V>& L = h.lev[l];
+    if (l == cy.local_from) {   // this level and those below in one kernel
+        ClArgs<V> a;
+        if (!cl_args<V>(h, l, false, a, nullptr)) throw Error(SEMO_ERR_STATE, "V-cycle: the small levels do not fit");
+        launch_cluster(k_local_cycle<V>, s, 1, a.smem, true, a);
+        return;
+    }
     if (l == (int)h.lev.size() - 1) {
         launch_pdl(k_coarse_solve<V>, 1, 256, s, h.coarse_n, h.cinv.p, L.b.p, L.x.p);
         return;
@@ -983,31 +1012,31 @@ void cg_iteration(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const OuterOp& outer, do
     double* q = c->kq.p;
     const int degree = c->prm.cheb_degree;
     const bool single = h.lev.size() == 1;
+    const int nb = red_blocks(n);
     if (single) {
         k_coarse_solve<V><<<1, 256, 0, s>>>(h.coarse_n, h.cinv, L.b, L.x);
         SEMO_CHECK_LAUNCH();
-        k_dot2<V><<<kRedBlocks, kRedThreads, 0, s>>>(n, L.x.p, r, q, R.part);
+        k_dot2<V><<<nb, kRedThreads, 0, s>>>(n, L.x.p, r, q, R.part);
         SEMO_CHECK_LAUNCH();
     } else if (degree == 2 && !cy.lev[0].gs) {
         const ChebCoef cc = cheb2(L.lam_max);
         vcycle_from(c, h, cy, 0);   // everything but the last smoothing step of the finest level
         // z lands in L.x; z.r and z.q folded in
         with_A(cy.lev[0], L.A, [&](auto A) {
-            launch_pdl(k_post1_dots<decltype(A), V>, kRedBlocks, kRedThreads, s, A, L.dinv.p, L.b.p, (V)cc.c1,
-                       (V)cc.c2, L.r.p, L.t.p, L.x.p, r, q, R.part);
+            launch_pdl(k_post1_dots<decltype(A), V>, nb, kRedThreads, s, A, L.dinv.p, L.b.p, (V)cc.c1, (V)cc.c2,
+                       L.r.p, L.t.p, L.x.p, r, q, R.part);
         });
     } else {
         vcycle_from(c, h, cy, 0);
-        k_dot2<V><<<kRedBlocks, kRedThreads, 0, s>>>(n, L.x.p, r, q, R.part);
+        k_dot2<V><<<nb, kRedThreads, 0, s>>>(n, L.x.p, r, q, R.part);
         SEMO_CHECK_LAUNCH();
     }
-    launch_pdl(k_fin_beta, 1, 256, s, R.part, R.scal);
     outer.with([&](auto A) {
-        launch_pdl(k_outer_mv<decltype(A), V>, kRedBlocks, kRedThreads, s, A, L.x.p, p, q, R.scal, R.part);
+        launch_pdl(k_outer_mv<decltype(A), V>, nb, kRedThreads, s, A, L.x.p, p, q, R.scal, R.part, nb,
+                   R.part + 2 * kRedBlocks);
     });
-    launch_pdl(k_fin_alpha, 1, 256, s, R.part, R.scal);
-    launch_pdl(k_xr<V>, kRedBlocks, kRedThreads, s, n, x, r, L.b.p, p, q, R.scal, R.part);
-    launch_pdl(k_fin_rr, 1, 256, s, R.part, R.scal);
+    launch_pdl(k_xr<V>, nb, kRedThreads, s, n, x, r, L.b.p, p, q, R.scal, R.part + 2 * kRedBlocks, nb,
+               R.part + 3 * kRedBlocks);
 }
 
 struct GraphGuard {
@@ -1038,17 +1067,40 @@ __global__ void k_cg_begin(cudaGraphConditionalHandle h, const double* __restric
 // loop goes on (scal[13] iterations, scal[14] status: 1 NaN/Inf, 2 p.q <= 0).
 // The loop is a conditional WHILE node, so no iteration waits for the host;
 // max_iter bounds it.
-__global__ void k_cg_check(cudaGraphConditionalHandle h, double* __restrict__ scal, double tol, int max_iter) {
+// One warp; prr: the iteration's partial sums of r.r.
+__global__ void k_cg_check(cudaGraphConditionalHandle h, double* __restrict__ scal, const double* __restrict__ prr,
+                           int nb, double tol, int max_iter) {
     pdl_enter();
+    const double rr = parts_sum(prr, nb);
+    if (threadIdx.x != 0) return;
     const double stop_rr = cg_stop_rr(scal, tol);
     const double it = scal[13] + 1.0;
     scal[13] = it;
-    const double pq = scal[2], rr = scal[3];
+    const double pq = scal[2];
     unsigned go = 1;
     if (!isfinite(rr) || !isfinite(pq)) { scal[14] = 1.0; go = 0; }
     else if (!(pq > 0.0)) { scal[14] = 2.0; go = 0; }
     else if (!(rr > stop_rr) || it >= (double)max_iter) go = 0;
     cudaGraphSetConditional(h, go);
+}
+
+// what a solve reports: h2 the scalars read back, nodes the loop's kernels
+void pcg_outcome(const double* h2, size_t nodes, semo_solve_info* info) {
+    const double bn = std::sqrt(h2[11]), rn0 = std::sqrt(h2[12]);
+    if (!std::isfinite(bn) || !std::isfinite(rn0)) throw Error(SEMO_ERR_NAN, "non-finite right-hand side");
+    const int it = (int)h2[13];
+    if (nodes) __atomic_add_fetch(&g_kernel_launches, 1LL + (long long)nodes * it, __ATOMIC_RELAXED);
+    if (h2[14] == 1.0) throw Error(SEMO_ERR_NAN, "NaN/Inf in the Krylov residual");
+    if (h2[14] == 2.0) throw Error(SEMO_ERR_BREAKDOWN, "CG breakdown: p.Ap <= 0 (matrix not SPD?)");
+    info->iterations = it;
+    info->rel_residual = (bn > 0.0) ? std::sqrt(h2[16]) / bn : 0.0;
+}
+
+// systems that k_cluster_cg solves whole: its arguments
+template <class V>
+bool cluster_cg_fits(const semo_ctx* c, const Amg<V>& h, const Cycle<V>& cy, ClArgs<V>& a, ClCg& g) {
+    if (c->prm.cheb_degree != 2 || (!cy.lev.empty() && cy.lev[0].gs)) return false;
+    return h.lev[0].A.n <= kClBlocks * kClThreads && cl_args<V>(h, 0, h.lev.size() > 1, a, &g);
 }
 
 template <class V>
@@ -1059,6 +1111,27 @@ void pcg(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const OuterOp& outer, const int* 
     c->kr.alloc(n, s); c->kp.alloc(n, s); c->kq.alloc(n, s);
     double* h2 = c->hpin;
     double* r = c->kr.p;
+    const int nb = red_blocks(n);
+    size_t body_nodes = 0;
+    ClArgs<V> ca;
+    ClCg g{};
+    g.A.gptr = ptr;
+    g.A.gcol = col;
+    g.A.gval = val;
+    g.b = b;
+    g.x = x;
+    g.scal = R.scal;
+    g.tol = c->prm.tol;
+    g.max_iter = c->prm.max_iter;
+    g.zero_guess = zero_guess;
+    if (cluster_cg_fits(c, h, cy, ca, g)) {   // the whole solve in one kernel
+        SEMO_CUDA(cudaMemsetAsync(R.scal, 0, sizeof(double) * 17, s));
+        launch_cluster(k_cluster_cg<V>, s, kClBlocks, ca.smem, false, ca, g);
+        SEMO_CUDA(cudaMemcpyAsync(h2, R.scal, sizeof(double) * 17, cudaMemcpyDeviceToHost, s));
+        SEMO_CUDA(cudaStreamSynchronize(s));
+        pcg_outcome(h2, 0, info);
+        return;
+    }
     const CsrView<double, 8> A8{ptr, col, val, n};
     if (zero_guess) {
         SEMO_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * n, s));
@@ -1071,14 +1144,14 @@ void pcg(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const OuterOp& outer, const int* 
     SEMO_CHECK_LAUNCH();
     SEMO_CUDA(cudaMemsetAsync(c->kq.p, 0, sizeof(double) * n, s));
     SEMO_CUDA(cudaMemsetAsync(c->kp.p, 0, sizeof(double) * n, s));
-    SEMO_CUDA(cudaMemsetAsync(R.scal, 0, sizeof(double) * 16, s));
-    k_dot<<<kRedBlocks, kRedThreads, 0, s>>>(n, b, b, R.part);
+    SEMO_CUDA(cudaMemsetAsync(R.scal, 0, sizeof(double) * 17, s));
+    k_dot<<<nb, kRedThreads, 0, s>>>(n, b, b, R.part);
     SEMO_CHECK_LAUNCH();
-    k_dot<<<kRedBlocks, kRedThreads, 0, s>>>(n, r, r, R.part + kRedBlocks);
+    k_dot<<<nb, kRedThreads, 0, s>>>(n, r, r, R.part + kRedBlocks);
     SEMO_CHECK_LAUNCH();
-    k_fin_rr<<<1, 256, 0, s>>>(R.part, R.scal + 8);   // ||b||^2 -> scal[11]
+    k_fin_sum<<<1, kRedThreads, 0, s>>>(R.part, nb, R.scal + 11);   // ||b||^2
     SEMO_CHECK_LAUNCH();
-    k_fin_rr<<<1, 256, 0, s>>>(R.part + kRedBlocks, R.scal + 9);   // ||r0||^2 -> scal[12]
+    k_fin_sum<<<1, kRedThreads, 0, s>>>(R.part + kRedBlocks, nb, R.scal + 12);   // ||r0||^2
     SEMO_CHECK_LAUNCH();
     // The loop is one graph: k_cg_begin, then a conditional WHILE node whose
     // body is one CG iteration (~30 kernels) plus k_cg_check, which decides on
@@ -1111,7 +1184,7 @@ void pcg(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const OuterOp& outer, const int* 
     SEMO_CUDA(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     try {
         cg_iteration(c, h, cy, outer, x, R);
-        launch_pdl(k_cg_check, 1, 1, s, handle, R.scal, tol, max_iter);
+        launch_pdl(k_cg_check, 1, 32, s, handle, R.scal, R.part + 3 * kRedBlocks, nb, tol, max_iter);
     } catch (...) {
         cudaGraph_t junk = nullptr;
         cudaStreamEndCapture(s, &junk);
@@ -1119,7 +1192,6 @@ void pcg(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const OuterOp& outer, const int* 
     }
     cudaGraph_t captured = nullptr;
     SEMO_CUDA(cudaStreamEndCapture(s, &captured));
-    size_t body_nodes = 0;
     SEMO_CUDA(cudaGraphGetNodes(body, nullptr, &body_nodes));
     __atomic_store_n(&g_kernel_launches, before, __ATOMIC_RELAXED);
     SEMO_CUDA(cudaGraphInstantiate(&gg.e, gg.g, 0));
@@ -1127,20 +1199,13 @@ void pcg(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const OuterOp& outer, const int* 
     // true FP64 residual of the returned solution -> scal[16]
     k_res64<<<blocks((int64_t)n * 8, 256), 256, 0, s>>>(A8, x, b, r);
     SEMO_CHECK_LAUNCH();
-    k_dot<<<kRedBlocks, kRedThreads, 0, s>>>(n, r, r, R.part);
+    k_dot<<<nb, kRedThreads, 0, s>>>(n, r, r, R.part);
     SEMO_CHECK_LAUNCH();
-    k_fin_rr<<<1, 256, 0, s>>>(R.part, R.scal + 13);
+    k_fin_sum<<<1, kRedThreads, 0, s>>>(R.part, nb, R.scal + 16);
     SEMO_CHECK_LAUNCH();
     SEMO_CUDA(cudaMemcpyAsync(h2, R.scal, sizeof(double) * 17, cudaMemcpyDeviceToHost, s));
     SEMO_CUDA(cudaStreamSynchronize(s));
-    const double bn = std::sqrt(h2[11]), rn0 = std::sqrt(h2[12]);
-    if (!std::isfinite(bn) || !std::isfinite(rn0)) throw Error(SEMO_ERR_NAN, "non-finite right-hand side");
-    const int it = (int)h2[13];
-    __atomic_add_fetch(&g_kernel_launches, 1LL + (long long)body_nodes * it, __ATOMIC_RELAXED);
-    if (h2[14] == 1.0) throw Error(SEMO_ERR_NAN, "NaN/Inf in the Krylov residual");
-    if (h2[14] == 2.0) throw Error(SEMO_ERR_BREAKDOWN, "CG breakdown: p.Ap <= 0 (matrix not SPD?)");
-    info->iterations = it;
-    info->rel_residual = (bn > 0.0) ? std::sqrt(h2[16]) / bn : 0.0;
+    pcg_outcome(h2, body_nodes, info);
 }
 
 template <class V>
@@ -1184,9 +1249,19 @@ void prepare_cycle(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const std::shared_ptr<S
     cudaStream_t s = setup_stream(c);
     const int nl = (int)h.lev.size();
     cy.lev.resize(std::max(nl - 1, 0));
+    cy.local_from = -1;
+    if (c->prm.cheb_degree == 2)
+        for (int l = 1; l + 1 < nl && cy.local_from < 0; ++l) {
+            ClArgs<V> a;
+            if (h.lev[l].A.nnz <= kLocalNnz && cl_args<V>(h, l, false, a, nullptr)) cy.local_from = l;
+        }
     for (int l = 0; l + 1 < nl; ++l) {
         AmgLevel<V>& L = h.lev[l];
         LevelMats<V>& M = cy.lev[l];
+        if (cy.local_from >= 0 && l >= cy.local_from) {   // CSR, all of them
+            M.a = M.p = M.r = M.a16 = M.gs = false;
+            continue;
+        }
         M.a = sell_pays(L.A);
         M.p = sell_pays(L.P);
         M.r = sell_pays(L.R);
@@ -1258,7 +1333,7 @@ __global__ void __launch_bounds__(kRedThreads) k_bi_init(int n, const double* __
                                                          double* __restrict__ r, double* __restrict__ rh,
                                                          double* __restrict__ p, double* __restrict__ v,
                                                          double* __restrict__ part) {
-    __shared__ double sh[32];
+    __shared__ double sh[kRedThreads];
     double bb[NR] = {};
     const size_t N = n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -1273,10 +1348,10 @@ __global__ void __launch_bounds__(kRedThreads) k_bi_init(int n, const double* __
     }
 }
 template <int NR>
-__global__ void k_bi_fin0(const double* __restrict__ part, double* __restrict__ scal, double tol2) {
-    __shared__ double sh[32];
+__global__ void k_bi_fin0(const double* __restrict__ part, int nb, double* __restrict__ scal, double tol2) {
+    __shared__ double sh[kRedThreads];
     for (int j = 0; j < NR; ++j) {
-        const double bb = sum_parts(part + j * kRedBlocks, sh);
+        const double bb = sum_parts(part + j * kRedBlocks, nb, sh);
         if (threadIdx.x == 0) {
             double* S = scal + kMomScal * j;
             for (int k = 0; k < kMomScal; ++k) S[k] = 0.0;
@@ -1306,7 +1381,7 @@ template <int NR>
 __global__ void __launch_bounds__(kRedThreads) k_bi_mv1(SellView<double> A, const double* __restrict__ x,
                                                         double* __restrict__ y, const double* __restrict__ rh,
                                                         const double* __restrict__ scal, double* __restrict__ part) {
-    __shared__ double sh[32];
+    __shared__ double sh[kRedThreads];
     const size_t N = A.n;
     double d[NR] = {};
     for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n; row += gridDim.x * blockDim.x) {
@@ -1324,10 +1399,10 @@ __global__ void __launch_bounds__(kRedThreads) k_bi_mv1(SellView<double> A, cons
     }
 }
 template <int NR>
-__global__ void k_bi_fin1(const double* __restrict__ part, double* __restrict__ scal) {
-    __shared__ double sh[32];
+__global__ void k_bi_fin1(const double* __restrict__ part, int nb, double* __restrict__ scal) {
+    __shared__ double sh[kRedThreads];
     for (int j = 0; j < NR; ++j) {
-        const double rv = sum_parts(part + j * kRedBlocks, sh);
+        const double rv = sum_parts(part + j * kRedBlocks, nb, sh);
         if (threadIdx.x == 0) {
             double* S = scal + kMomScal * j;
             if (S[9] != 0.0) {
@@ -1358,7 +1433,7 @@ template <int NR>
 __global__ void __launch_bounds__(kRedThreads) k_bi_mv2(SellView<double> A, const double* __restrict__ x,
                                                         double* __restrict__ t, const double* __restrict__ s,
                                                         const double* __restrict__ scal, double* __restrict__ part) {
-    __shared__ double sh[32];
+    __shared__ double sh[kRedThreads];
     const size_t N = A.n;
     double ts[NR] = {}, tt[NR] = {};
     for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n; row += gridDim.x * blockDim.x) {
@@ -1378,11 +1453,11 @@ __global__ void __launch_bounds__(kRedThreads) k_bi_mv2(SellView<double> A, cons
     }
 }
 template <int NR>
-__global__ void k_bi_fin2(const double* __restrict__ part, double* __restrict__ scal) {
-    __shared__ double sh[32];
+__global__ void k_bi_fin2(const double* __restrict__ part, int nb, double* __restrict__ scal) {
+    __shared__ double sh[kRedThreads];
     for (int j = 0; j < NR; ++j) {
-        const double ts = sum_parts(part + (2 * j) * kRedBlocks, sh);
-        const double tt = sum_parts(part + (2 * j + 1) * kRedBlocks, sh);
+        const double ts = sum_parts(part + (2 * j) * kRedBlocks, nb, sh);
+        const double tt = sum_parts(part + (2 * j + 1) * kRedBlocks, nb, sh);
         if (threadIdx.x == 0) {
             double* S = scal + kMomScal * j;
             if (S[9] != 0.0) { S[5] = ts; S[6] = tt; S[2] = (tt > 0.0) ? ts / tt : 0.0; }
@@ -1395,7 +1470,7 @@ __global__ void __launch_bounds__(kRedThreads) k_bi_xr(int n, double* __restrict
                                                        const double* __restrict__ shv, double* __restrict__ r,
                                                        const double* __restrict__ t, const double* __restrict__ rh,
                                                        const double* __restrict__ scal, double* __restrict__ part) {
-    __shared__ double sh[32];
+    __shared__ double sh[kRedThreads];
     const size_t N = n;
     double a[NR] = {}, b[NR] = {};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -1415,11 +1490,11 @@ __global__ void __launch_bounds__(kRedThreads) k_bi_xr(int n, double* __restrict
     }
 }
 template <int NR>
-__global__ void k_bi_fin3(const double* __restrict__ part, double* __restrict__ scal, double tol2) {
-    __shared__ double sh[32];
+__global__ void k_bi_fin3(const double* __restrict__ part, int nb, double* __restrict__ scal, double tol2) {
+    __shared__ double sh[kRedThreads];
     for (int j = 0; j < NR; ++j) {
-        const double rho1 = sum_parts(part + (2 * j) * kRedBlocks, sh);
-        const double rr = sum_parts(part + (2 * j + 1) * kRedBlocks, sh);
+        const double rho1 = sum_parts(part + (2 * j) * kRedBlocks, nb, sh);
+        const double rr = sum_parts(part + (2 * j + 1) * kRedBlocks, nb, sh);
         if (threadIdx.x == 0) {
             double* S = scal + kMomScal * j;
             if (S[9] != 0.0) {
@@ -1441,7 +1516,7 @@ __global__ void k_bi_fin3(const double* __restrict__ part, double* __restrict__ 
 template <int NR>
 __global__ void __launch_bounds__(kRedThreads) k_bi_res(SellView<double> A, const double* __restrict__ x,
                                                         const double* __restrict__ b, double* __restrict__ part) {
-    __shared__ double sh[32];
+    __shared__ double sh[kRedThreads];
     const size_t N = A.n;
     double d[NR] = {};
     for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n; row += gridDim.x * blockDim.x) {
@@ -1455,10 +1530,10 @@ __global__ void __launch_bounds__(kRedThreads) k_bi_res(SellView<double> A, cons
     }
 }
 template <int NR>
-__global__ void k_bi_fin_res(const double* __restrict__ part, double* __restrict__ out) {
-    __shared__ double sh[32];
+__global__ void k_bi_fin_res(const double* __restrict__ part, int nb, double* __restrict__ out) {
+    __shared__ double sh[kRedThreads];
     for (int j = 0; j < NR; ++j) {
-        const double rr = sum_parts(part + j * kRedBlocks, sh);
+        const double rr = sum_parts(part + j * kRedBlocks, nb, sh);
         if (threadIdx.x == 0) out[j] = rr;
     }
 }
@@ -1650,6 +1725,7 @@ semo_status bicgstab_jacobi(semo_ctx* c, int stage, const KrylovPattern& pat, co
     cudaStream_t s = c->stream;
     const int n = pat.n;
     const size_t N = n;
+    const int nb = red_blocks(n);
     MomState& st = mom_state(c);
     st.dinv.alloc(N, s);
     st.vec.alloc(7 * 3 * N, s);       // r, rh, p, v, ph, sh, t (room for 3 systems)
@@ -1678,9 +1754,9 @@ semo_status bicgstab_jacobi(semo_ctx* c, int stage, const KrylovPattern& pat, co
     SEMO_CHECK_LAUNCH();
     SEMO_CUDA(cudaEventRecord(c->ev[1], s));
     const SellView<double> A = st.A.view();
-    k_bi_init<NR><<<kRedBlocks, kRedThreads, 0, s>>>(n, b, x, r, rh, p, v, st.part);
+    k_bi_init<NR><<<nb, kRedThreads, 0, s>>>(n, b, x, r, rh, p, v, st.part);
     SEMO_CHECK_LAUNCH();
-    k_bi_fin0<NR><<<1, 256, 0, s>>>(st.part, st.scal, tol2);
+    k_bi_fin0<NR><<<1, 256, 0, s>>>(st.part, nb, st.scal, tol2);
     SEMO_CHECK_LAUNCH();
     // The iterations run as one graph: a conditional WHILE node around one
     // iteration (8 kernels + k_bi_check), launched without a host round trip
@@ -1713,19 +1789,19 @@ semo_status bicgstab_jacobi(semo_ctx* c, int stage, const KrylovPattern& pat, co
         try {
             k_bi_p<NR><<<blocks(n, 256), 256, 0, s>>>(n, st.dinv, r, p, v, ph, st.scal);
             SEMO_CHECK_LAUNCH();
-            k_bi_mv1<NR><<<kRedBlocks, kRedThreads, 0, s>>>(A, ph, v, rh, st.scal, st.part);
+            k_bi_mv1<NR><<<nb, kRedThreads, 0, s>>>(A, ph, v, rh, st.scal, st.part);
             SEMO_CHECK_LAUNCH();
-            k_bi_fin1<NR><<<1, 256, 0, s>>>(st.part, st.scal);
+            k_bi_fin1<NR><<<1, 256, 0, s>>>(st.part, nb, st.scal);
             SEMO_CHECK_LAUNCH();
             k_bi_s<NR><<<blocks(n, 256), 256, 0, s>>>(n, st.dinv, r, v, shv, st.scal);
             SEMO_CHECK_LAUNCH();
-            k_bi_mv2<NR><<<kRedBlocks, kRedThreads, 0, s>>>(A, shv, t, r, st.scal, st.part);
+            k_bi_mv2<NR><<<nb, kRedThreads, 0, s>>>(A, shv, t, r, st.scal, st.part);
             SEMO_CHECK_LAUNCH();
-            k_bi_fin2<NR><<<1, 256, 0, s>>>(st.part, st.scal);
+            k_bi_fin2<NR><<<1, 256, 0, s>>>(st.part, nb, st.scal);
             SEMO_CHECK_LAUNCH();
-            k_bi_xr<NR><<<kRedBlocks, kRedThreads, 0, s>>>(n, x, ph, shv, r, t, rh, st.scal, st.part);
+            k_bi_xr<NR><<<nb, kRedThreads, 0, s>>>(n, x, ph, shv, r, t, rh, st.scal, st.part);
             SEMO_CHECK_LAUNCH();
-            k_bi_fin3<NR><<<1, 256, 0, s>>>(st.part, st.scal, tol2);
+            k_bi_fin3<NR><<<1, 256, 0, s>>>(st.part, nb, st.scal, tol2);
             SEMO_CHECK_LAUNCH();
             k_bi_check<NR><<<1, 1, 0, s>>>(handle, st.scal, c->prm.mom_max_iter);
             SEMO_CHECK_LAUNCH();
@@ -1744,9 +1820,9 @@ semo_status bicgstab_jacobi(semo_ctx* c, int stage, const KrylovPattern& pat, co
     SEMO_CUDA(cudaMemsetAsync(st.scal.p + 3 * kMomScal, 0, sizeof(double) * kMomScal, s));
     SEMO_CUDA(cudaGraphLaunch(G.e, s));
     // true FP64 residuals of the returned solutions
-    k_bi_res<NR><<<kRedBlocks, kRedThreads, 0, s>>>(A, x, b, st.part);
+    k_bi_res<NR><<<nb, kRedThreads, 0, s>>>(A, x, b, st.part);
     SEMO_CHECK_LAUNCH();
-    k_bi_fin_res<NR><<<1, 256, 0, s>>>(st.part, st.scal.p + 3 * kMomScal - 3);
+    k_bi_fin_res<NR><<<1, 256, 0, s>>>(st.part, nb, st.scal.p + 3 * kMomScal - 3);
     SEMO_CHECK_LAUNCH();
     // pinned: the systems' scalars and the iteration count hpin[0, 64), the
     // true residuals hpin[64, 64 + NR)

@@ -93,9 +93,14 @@ template <class V>
 struct DCsr {
     int n = 0, m = 0;      // rows, cols
     int64_t nnz = 0;
+    int run = 0;           // entries of the longest cluster run of rows (0: not known)
     DBuf<int> ptr, col;
     DBuf<V> val;
 };
+// Small levels are cycled by clusters of kClusterBlocks blocks, each with a run
+// of rows that starts on a 16-byte boundary of any vector (cycle_cluster.cuh).
+constexpr int kClusterBlocks = 8;
+__host__ __device__ inline int cluster_run(int n) { return ((n + kClusterBlocks - 1) / kClusterBlocks + 3) & ~3; }
 
 // One level of the smoothed-aggregation hierarchy, value type V.
 template <class V>
