@@ -23,6 +23,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 UNITS = [
     ("geometry.cu", ["--fmad=false"]),
     ("assemble.cu", []),
+    ("stencil.cu", []),
     ("momentum.cu", []),
     ("vof.cu", []),
     ("coupled.cu", []),

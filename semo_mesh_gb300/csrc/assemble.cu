@@ -4,9 +4,7 @@
 //   k_cell_eos        calcIncomCellEOSVF            src/solvers/eos.cpp:10-151
 //   k_bface_values    reconIncomZeroOrder + face EOS src/solvers/reconIncom.cpp:501-1035, :440-496
 //   k_grav_face/cell  calcSourceGravity             src/solvers/source/gravity.cpp:7-75
-//   k_stencil         setCellVarMinMax x4 + calcLeastSquare("cellVertex","1st") x5
-//                                                   src/solvers/cellVarMinMax.cpp:8-23,
-//                                                   src/math/gradient.cpp:761-816, :997-1050, :1136-1159
+//   (stencil.cu)      setCellVarMinMax x4 + calcLeastSquare("cellVertex","1st") x5
 //   k_pface           calcPressureEq face loop      src/solvers/eqPressure.cpp:246-564
 //                     + Rhie-Chow helpers           src/solvers/surfaceNormalVelocity.cpp:125-187
 //   k_pbface          calcPressureEq boundary loop  src/solvers/eqPressure.cpp:570-673
@@ -140,93 +138,6 @@ __global__ void k_grav_cell(int nc, int nf, const int* __restrict__ cfp, const i
         }
     }
     sg[i] = s0; sg[nc + i] = s1; sg[2 * nc + i] = s2; sg[3 * nc + i] = s3;
-}
-
-// One pass over each cell's vertex stencil: LSQ gradients of P,U,V,W,VF and
-// stencil min/max of U,V,W,VF,P (mm planes maxU,minU,maxV,minV,maxW,minW,
-// maxVF,minVF,maxP,minP).  Stencil weights w_k*d_k are precomputed, and so is
-// their per-cell sum S (stencil and boundary faces): the gradient's sum
-// sum_k w_k (phi_k - phi_i) is formed as sum_k w_k phi_k - phi_i S, three FMAs
-// an entry and field instead of a difference and three FMAs (FP64 issue bounds
-// this kernel on GB300).  With kPVF false only the U,V,W parts are computed
-// and the P and VF planes are left as they are (they are still current: see
-// assemble_gravity_stencil).
-template <bool kPVF>
-__global__ void __launch_bounds__(128) k_stencil(int nc, int nf, int ni, int nb, const int* __restrict__ stp,
-                                                 const int* __restrict__ sti, const double* __restrict__ stw,
-                                                 int64_t stn, const int* __restrict__ cfp,
-                                                 const int* __restrict__ cfi, const double* __restrict__ bfw,
-                                                 const double* __restrict__ stws,
-                                                 const double* __restrict__ minv, const double* __restrict__ P,
-                                                 const double* __restrict__ U, const double* __restrict__ V,
-                                                 const double* __restrict__ W, const double* __restrict__ VF,
-                                                 const double* __restrict__ bf, double* __restrict__ grad,
-                                                 double* __restrict__ mm) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nc) return;
-    const double pi = P[i], ui = U[i], vi = V[i], wi = W[i], fi = VF[i];
-    double g[5][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    long long kmaxu = okey(ui), kminu = kmaxu, kmaxv = okey(vi), kminv = kmaxv;
-    long long kmaxw = okey(wi), kminw = kmaxw, kmaxf = okey(fi), kminf = kmaxf;
-    long long kmaxp = okey(pi), kminp = kmaxp;
-    const int kb = stp[i], ke = stp[i + 1];
-    for (int k = kb; k < ke; ++k) {
-        const int j = __ldg(sti + k);
-        const double wx = __ldg(stw + k), wy = __ldg(stw + stn + k), wz = __ldg(stw + 2 * stn + k);
-        const double uj = __ldg(U + j), vj = __ldg(V + j), wj = __ldg(W + j);
-        long long t;
-        if constexpr (kPVF) {
-            const double pj = __ldg(P + j), fj = __ldg(VF + j);
-            g[0][0] = fma(wx, pj, g[0][0]); g[0][1] = fma(wy, pj, g[0][1]); g[0][2] = fma(wz, pj, g[0][2]);
-            g[4][0] = fma(wx, fj, g[4][0]); g[4][1] = fma(wy, fj, g[4][1]); g[4][2] = fma(wz, fj, g[4][2]);
-            t = okey(fj); kmaxf = (kmaxf < t) ? t : kmaxf; kminf = (t < kminf) ? t : kminf;
-            t = okey(pj); kmaxp = (kmaxp < t) ? t : kmaxp; kminp = (t < kminp) ? t : kminp;
-        }
-        g[1][0] = fma(wx, uj, g[1][0]); g[1][1] = fma(wy, uj, g[1][1]); g[1][2] = fma(wz, uj, g[1][2]);
-        g[2][0] = fma(wx, vj, g[2][0]); g[2][1] = fma(wy, vj, g[2][1]); g[2][2] = fma(wz, vj, g[2][2]);
-        g[3][0] = fma(wx, wj, g[3][0]); g[3][1] = fma(wy, wj, g[3][1]); g[3][2] = fma(wz, wj, g[3][2]);
-        t = okey(uj); kmaxu = (kmaxu < t) ? t : kmaxu; kminu = (t < kminu) ? t : kminu;
-        t = okey(vj); kmaxv = (kmaxv < t) ? t : kmaxv; kminv = (t < kminv) ? t : kminv;
-        t = okey(wj); kmaxw = (kmaxw < t) ? t : kmaxw; kminw = (t < kminw) ? t : kminw;
-    }
-    // boundary faces (face index >= ni) come last in the ascending list
-    {
-        int kfirst = cfp[i + 1];
-        while (kfirst > cfp[i] && (cfi[kfirst - 1] & kFaceMask) >= ni) --kfirst;
-        for (int k = kfirst; k < cfp[i + 1]; ++k) {
-            const int b = (cfi[k] & kFaceMask) - ni;
-            const double wx = bfw[b], wy = bfw[nb + b], wz = bfw[2 * nb + b];
-            double d;
-            if constexpr (kPVF) { d = bf[b]; g[0][0] += wx * d; g[0][1] += wy * d; g[0][2] += wz * d; }
-            d = bf[nb + b]; g[1][0] += wx * d; g[1][1] += wy * d; g[1][2] += wz * d;
-            d = bf[2 * nb + b]; g[2][0] += wx * d; g[2][1] += wy * d; g[2][2] += wz * d;
-            d = bf[3 * nb + b]; g[3][0] += wx * d; g[3][1] += wy * d; g[3][2] += wz * d;
-            if constexpr (kPVF) { d = bf[4 * nb + b]; g[4][0] += wx * d; g[4][1] += wy * d; g[4][2] += wz * d; }
-        }
-    }
-    const double sx = stws[i], sy = stws[nc + i], sz = stws[2 * nc + i];
-    const double phi_i[5] = {pi, ui, vi, wi, fi};
-    const double m0 = minv[i], m1 = minv[nc + i], m2 = minv[2 * nc + i];
-    const double m3 = minv[3 * nc + i], m4 = minv[4 * nc + i], m5 = minv[5 * nc + i];
-#pragma unroll
-    for (int q = kPVF ? 0 : 1; q < (kPVF ? 5 : 4); ++q) {
-        const double a0 = fma(-phi_i[q], sx, g[q][0]);
-        const double a1 = fma(-phi_i[q], sy, g[q][1]);
-        const double a2 = fma(-phi_i[q], sz, g[q][2]);
-        double t0 = 0.0; t0 += m0 * a0; t0 += m1 * a1; t0 += m2 * a2;
-        double t1 = 0.0; t1 += m1 * a0; t1 += m3 * a1; t1 += m4 * a2;
-        double t2 = 0.0; t2 += m2 * a0; t2 += m4 * a1; t2 += m5 * a2;
-        grad[(3 * q + 0) * (size_t)nc + i] = t0;
-        grad[(3 * q + 1) * (size_t)nc + i] = t1;
-        grad[(3 * q + 2) * (size_t)nc + i] = t2;
-    }
-    mm[i] = ounkey(kmaxu); mm[nc + i] = ounkey(kminu);
-    mm[2 * (size_t)nc + i] = ounkey(kmaxv); mm[3 * (size_t)nc + i] = ounkey(kminv);
-    mm[4 * (size_t)nc + i] = ounkey(kmaxw); mm[5 * (size_t)nc + i] = ounkey(kminw);
-    if constexpr (kPVF) {
-        mm[6 * (size_t)nc + i] = ounkey(kmaxf); mm[7 * (size_t)nc + i] = ounkey(kminf);
-        mm[8 * (size_t)nc + i] = ounkey(kmaxp); mm[9 * (size_t)nc + i] = ounkey(kminp);
-    }
 }
 
 // SEMO's clamp sequence (if x <= lo: x = lo; if x >= hi: x = hi) on the
@@ -533,28 +444,6 @@ void assemble_gravity(semo_ctx* c) {
         c->sg.zero();
     }
     c->sg_current = true;
-}
-
-void stencil_pass(semo_ctx* c, bool full) {
-    const int nc = c->nc, nf = c->nf, ni = c->ni, nb = c->nb;
-    cudaStream_t s = c->stream;
-    StageScope sc(c, full ? ST_STENCIL : ST_STENCIL_UVW);
-    auto launch = [&](auto kern) {
-        kern<<<blocks(nc, 128), 128, 0, s>>>(nc, nf, ni, nb, c->st_ptr, c->st_idx, c->stw, c->st_nnz, c->cf_ptr,
-                                             c->cf_idx, c->bfw, c->stws, c->minv, c->P, c->U, c->V, c->W, c->VF, c->bface,
-                                             c->grad, c->mm);
-    };
-    if (full) launch(k_stencil<true>);
-    else launch(k_stencil<false>);
-    SEMO_CHECK_LAUNCH();
-}
-
-void lsq_gradients5(semo_ctx* c, const double* f0, const double* f1, const double* f2, const double* f3,
-                    const double* f4, const double* bf, double* grad, double* mm) {
-    k_stencil<true><<<blocks(c->nc, 128), 128, 0, c->stream>>>(c->nc, c->nf, c->ni, c->nb, c->st_ptr, c->st_idx,
-                                                               c->stw, c->st_nnz, c->cf_ptr, c->cf_idx, c->bfw,
-                                                               c->stws, c->minv, f0, f1, f2, f3, f4, bf, grad, mm);
-    SEMO_CHECK_LAUNCH();
 }
 
 void assemble_gravity_stencil(semo_ctx* c) {
