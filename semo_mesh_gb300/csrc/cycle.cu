@@ -107,13 +107,29 @@ struct SellView {
             const int b = sptr[sl], w = (sptr[sl + 1] - b) >> 5;
             int k = b + l;
             int j = 0;
-            for (; j + 1 < w; j += 2, k += 64) {   // two independent loads in flight
-                const int c0 = col[k], c1 = col[k + 32];
-                const V v0 = val[k], v1 = val[k + 32];
-                s += v0 * x(c0);
-                s += v1 * x(c1);
+            if constexpr (sizeof(V) == 4) {   // transfer operators: eight entries in flight
+                for (; j < w; j += 8, k += 256) {
+                    int cj[8];
+                    V vj[8], xj[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (j + q < w) { cj[q] = col[k + 32 * q]; vj[q] = val[k + 32 * q]; }
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (j + q < w) xj[q] = x(cj[q]);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (j + q < w) s += vj[q] * xj[q];
+                }
+            } else {
+                for (; j + 1 < w; j += 2, k += 64) {   // two independent loads in flight
+                    const int c0 = col[k], c1 = col[k + 32];
+                    const V v0 = val[k], v1 = val[k + 32];
+                    s += v0 * x(c0);
+                    s += v1 * x(c1);
+                }
+                if (j < w) s += val[k] * x(col[k]);
             }
-            if (j < w) s += val[k] * x(col[k]);
         }
         return s;
     }
@@ -132,7 +148,7 @@ struct SellView {
 // point at the row (mode 0) or at the group's base (1, 2) with value 0.
 template <class V>
 struct Sell16View {
-    static constexpr int kVS = 1;
+    static constexpr int kVS = 1, kEven = 0;
     const int* __restrict__ sptr;
     const int* __restrict__ smode;
     const int* __restrict__ gbase;
@@ -168,16 +184,16 @@ struct Sell16View {
                 for (int q = 0; q < 8; ++q)
                     if (q < w) s += vj[q] * xj[q];
             } else if (mode == 0) {
-                if (sizeof(V) == 4)   // longer FP32 rows (coarse levels): four entries in flight
-                    for (; j + 3 < w; j += 4, k += 128) {
-                        const int c0 = row + (short)dcol[k], c1 = row + (short)dcol[k + 32];
-                        const int c2 = row + (short)dcol[k + 64], c3 = row + (short)dcol[k + 96];
-                        const V v0 = val[k], v1 = val[k + 32], v2 = val[k + 64], v3 = val[k + 96];
-                        const V x0 = x(c0), x1 = x(c1), x2 = x(c2), x3 = x(c3);
-                        s += v0 * x0;
-                        s += v1 * x1;
-                        s += v2 * x2;
-                        s += v3 * x3;
+                if (sizeof(V) == 4)   // longer FP32 rows (coarse levels): eight entries in flight
+                    for (; j + 7 < w; j += 8, k += 256) {
+                        int cj[8];
+                        V vj[8], xj[8];
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) { cj[q] = row + (short)dcol[k + 32 * q]; vj[q] = val[k + 32 * q]; }
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) xj[q] = x(cj[q]);
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) s += vj[q] * xj[q];
                     }
                 for (; j + 1 < w; j += 2, k += 64) {   // two independent loads in flight
                     const int c0 = row + (short)dcol[k], c1 = row + (short)dcol[k + 32];
@@ -210,18 +226,120 @@ struct Sell16View {
     }
 };
 
+// SELL-32 with 16-bit columns whose slices are all W entries wide and all of mode
+// 0 (the finest level of a mesh of one cell type: 7 for hexahedra, 5 for
+// tetrahedra).  A slice's place follows from its number, so the entries are
+// fetched at once, without the trip for the slice pointer and encoding, and the
+// width is known to the compiler: y = b - A x in FP32 at 128^3 cells 30.8 -> 22.6
+// us (111 MB: 4.9 TB/s), at 96^3 10.3 -> 6.4 (the width as a run-time value: 26.7
+// and 10.3).
+template <class V, int W>
+struct Sell16UView {
+    static constexpr int kVS = 1, kEven = W;
+    const unsigned short* __restrict__ dcol;
+    const V* __restrict__ val;
+    int n;
+    template <class F>
+    __device__ __forceinline__ V dot(int row, int, const F& x) const {
+        V s = V(0);
+        if (row < n) {
+            const int k = (row >> 5) * (32 * W) + (row & 31);
+            int cj[W];
+            V vj[W];
+            typename F::Raw xj[W];
+#pragma unroll
+            for (int q = 0; q < W; ++q) { cj[q] = row + (short)dcol[k + 32 * q]; vj[q] = val[k + 32 * q]; }
+#pragma unroll
+            for (int q = 0; q < W; ++q) xj[q] = x.load(cj[q]);
+#pragma unroll
+            for (int q = 0; q < W; ++q) s += vj[q] * x.value(xj[q]);
+        }
+        return s;
+    }
+};
+
+// An FP32 number as a double, by integer instructions: the conversion
+// instruction takes longer in the FP64 unit than a multiply-add (k_outer_mv at
+// 128^3: 83 us, 48 with the integers, 37 without any FP64 arithmetic).  Every value, subnormal, infinite and
+// not-a-number ones too.
+__host__ __device__ __forceinline__ uint64_t wide_bits(uint32_t b) {
+    const uint32_t sign = b & 0x80000000u, m = b & 0x7fffffu, e = (b >> 23) & 0xffu;
+    // exponents: 127 -> 1023, 255 -> 2047
+    uint32_t hi = sign | (((b & 0x7fffffffu) >> 3) + (e == 255 ? 0x70000000u : 0x38000000u));
+    uint32_t lo = b << 29;
+    if (e == 0) {   // zero or subnormal: m 2^-149
+        hi = sign;
+        lo = 0;
+#pragma unroll 1
+        for (uint32_t k = m, x = 896; k != 0; k <<= 1, --x)
+            if (k & 0x400000u) {   // the leading bit becomes the implicit one
+                hi = sign | (x << 20) | ((k & 0x3fffffu) >> 2);
+                lo = k << 30;
+                break;
+            }
+    }
+    return ((uint64_t)hi << 32) | lo;
+}
+// (float)d by integer instructions, rounded to nearest even, for the same reason
+__host__ __device__ __forceinline__ uint32_t narrow_bits(uint64_t u) {
+    const uint32_t sign = (uint32_t)(u >> 32) & 0x80000000u, e = (uint32_t)(u >> 52) & 0x7ffu;
+    if (e - 897u <= 253u) {   // in the range of normal FP32 numbers
+        const uint32_t t = (uint32_t)((u & 0x7fffffffffffffffull) >> 29) - (896u << 23);
+        const uint32_t rest = (uint32_t)u & 0x1fffffffu;
+        return sign | (t + (rest > 0x10000000u - (t & 1u) ? 1u : 0u));
+    }
+    if (e == 0x7ff && (u & 0xfffffffffffffull)) return sign | 0x7fc00000u;
+    if (e > 1150u) return sign | 0x7f800000u;
+    if (e < 872u) return sign;   // below half the smallest subnormal
+    const uint64_t m = (u & 0xfffffffffffffull) | 0x10000000000000ull;
+    const int sh = 29 + (int)(897u - e);   // 30 .. 54
+    const uint64_t t = m >> sh, rest = m & ((1ull << sh) - 1), half = 1ull << (sh - 1);
+    return sign | (uint32_t)(t + (rest > half || (rest == half && (t & 1)) ? 1 : 0));
+}
+template <class V>
+__device__ __forceinline__ V narrow(double d) {
+    if constexpr (sizeof(V) == 4) return __uint_as_float(narrow_bits((uint64_t)__double_as_longlong(d)));
+    else return d;
+}
+template <class V, class X>
+__device__ __forceinline__ V widen(X x) {
+    if constexpr (sizeof(V) > sizeof(X)) return __longlong_as_double((long long)wide_bits(__float_as_uint(x)));
+    else return x;
+}
+
 template <class V, class X>
 struct Vec {
+    using Raw = X;
     const X* __restrict__ p;
-    __device__ __forceinline__ V operator()(int j) const { return (V)__ldg(p + j); }
+    __device__ __forceinline__ X load(int j) const { return __ldg(p + j); }
+    __device__ __forceinline__ V value(X x) const { return widen<V>(x); }
+    __device__ __forceinline__ V operator()(int j) const { return value(load(j)); }
 };
-// the first Chebyshev iterate from zero, D^-1 b / theta, formed on the fly
+// The first Chebyshev iterate from zero, d0 = D^-1 b / theta, of a vector b that
+// the V-cycle starts a level with.  Below the finest level the kernel that
+// writes b writes d0 beside it (into the level's t, free until k_post0): formed
+// in k_pre2 it is two gathers and two products an entry instead of one gather
+// (second level at 128^3, 188k rows of 33 entries: 19.4 us formed there, 15.9
+// now).  On the finest level k_xr would have to write it, 25 MB more at 128^3
+// for +6 us there against -1 us in k_pre2, so k_pre2 forms it.
 template <class V>
 struct FirstIterate {
+    const V* dinv;   // null: not wanted
+    V inv_theta;
+    V* d0;
+    __device__ __forceinline__ void put(int i, V bi) const {
+        if (dinv) d0[i] = dinv[i] * bi * inv_theta;
+    }
+};
+template <class V>
+struct FirstGather {   // d0 formed on the fly
+    using Raw = V;
     const V* __restrict__ dinv;
     const V* __restrict__ b;
     V inv_theta;
-    __device__ __forceinline__ V operator()(int j) const { return __ldg(dinv + j) * __ldg(b + j) * inv_theta; }
+    __device__ __forceinline__ V load(int j) const { return __ldg(dinv + j) * __ldg(b + j) * inv_theta; }
+    __device__ __forceinline__ V value(V x) const { return x; }
+    __device__ __forceinline__ V operator()(int j) const { return load(j); }
 };
 
 // ------------------------------------------- programmatic dependent launch
@@ -257,18 +375,16 @@ void launch_pdl(void (*k)(P...), int grid, int block, cudaStream_t s, A&&... arg
 
 // ------------------------------------------------------- V-cycle kernels
 // pre-smoothing, degree 2 from x = 0:  x = d0 + c1 d0 + c2 D^-1 (b - A d0),  d0 = D^-1 b / theta
-template <class M, class V>
+template <class M, class V, class X>
 __global__ void __launch_bounds__(256) k_pre2(M A, const V* __restrict__ dinv, const V* __restrict__ b,
-                                              V inv_theta, V c1, V c2, V* __restrict__ x) {
+                                              X d0, V c1, V c2, V* __restrict__ x) {
     pdl_enter();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int row = g / M::kVS, lane = g % M::kVS;
-    const V s = A.dot(row, lane, FirstIterate<V>{dinv, b, inv_theta});
-    if (row < A.n && lane == 0) {
-        const V di = dinv[row], bi = b[row];
-        const V d0 = di * bi * inv_theta;
-        x[row] = d0 + c1 * d0 + c2 * (di * (bi - s));
-    }
+    const bool mine = row < A.n && lane == 0;   // the row's own values are loaded before the product's wait
+    const V d = mine ? d0(row) : V(0), di = mine ? dinv[row] : V(0), bi = mine ? b[row] : V(0);
+    const V s = A.dot(row, lane, d0);
+    if (mine) x[row] = d + c1 * d + c2 * (di * (bi - s));
 }
 // r = b - A x
 template <class M, class V>
@@ -277,17 +393,22 @@ __global__ void __launch_bounds__(256) k_res(M A, const V* __restrict__ x, const
     pdl_enter();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int row = g / M::kVS, lane = g % M::kVS;
+    const bool mine = row < A.n && lane == 0;
+    const V bi = mine ? b[row] : V(0);
     const V s = A.dot(row, lane, Vec<V, V>{x});
-    if (row < A.n && lane == 0) r[row] = b[row] - s;
+    if (mine) r[row] = bi - s;
 }
-// y = A x (restriction with R, or any plain product)
+// y = A x (restriction with R, and then the coarse level's d0; or any plain product)
 template <class M, class V>
-__global__ void __launch_bounds__(256) k_mv(M A, const V* __restrict__ x, V* __restrict__ y) {
+__global__ void __launch_bounds__(256) k_mv(M A, const V* __restrict__ x, V* __restrict__ y, FirstIterate<V> f) {
     pdl_enter();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int row = g / M::kVS, lane = g % M::kVS;
     const V s = A.dot(row, lane, Vec<V, V>{x});
-    if (row < A.n && lane == 0) y[row] = s;
+    if (row < A.n && lane == 0) {
+        y[row] = s;
+        f.put(row, s);
+    }
 }
 // x += P xc
 template <class M, class V>
@@ -295,8 +416,10 @@ __global__ void __launch_bounds__(256) k_prolong_add(M P, const V* __restrict__ 
     pdl_enter();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int row = g / M::kVS, lane = g % M::kVS;
+    const bool mine = row < P.n && lane == 0;
+    const V xi = mine ? x[row] : V(0);
     const V s = P.dot(row, lane, Vec<V, V>{xc});
-    if (row < P.n && lane == 0) x[row] += s;
+    if (mine) x[row] = xi + s;
 }
 // post-smoothing step 0 from x:  d = D^-1 (b - A x) / theta ;  y = x + d
 template <class M, class V>
@@ -306,11 +429,13 @@ __global__ void __launch_bounds__(256) k_post0(M A, const V* __restrict__ dinv, 
     pdl_enter();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int row = g / M::kVS, lane = g % M::kVS;
+    const bool mine = row < A.n && lane == 0;
+    const V di = mine ? dinv[row] : V(0), bi = mine ? b[row] : V(0), xi = mine ? x[row] : V(0);
     const V s = A.dot(row, lane, Vec<V, V>{x});
-    if (row < A.n && lane == 0) {
-        const V dv = dinv[row] * (b[row] - s) * inv_theta;
+    if (mine) {
+        const V dv = di * (bi - s) * inv_theta;
         d[row] = dv;
-        y[row] = x[row] + dv;
+        y[row] = xi + dv;
     }
 }
 // post-smoothing step 1:  x = y + c1 d + c2 D^-1 (b - A y)
@@ -321,8 +446,11 @@ __global__ void __launch_bounds__(256) k_post1(M A, const V* __restrict__ dinv, 
     pdl_enter();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int row = g / M::kVS, lane = g % M::kVS;
+    const bool mine = row < A.n && lane == 0;
+    const V yi = mine ? y[row] : V(0), dv = mine ? d[row] : V(0), di = mine ? dinv[row] : V(0);
+    const V bi = mine ? b[row] : V(0);
     const V s = A.dot(row, lane, Vec<V, V>{y});
-    if (row < A.n && lane == 0) x[row] = y[row] + c1 * d[row] + c2 * (dinv[row] * (b[row] - s));
+    if (mine) x[row] = yi + c1 * dv + c2 * (di * (bi - s));
 }
 // finest-level post-smoothing step 1 (SELL), also folding in the CG dots
 // z.r and z.q (q = A p of the previous iteration); grid-stride, fixed grid
@@ -339,13 +467,17 @@ __global__ void __launch_bounds__(kRedThreads) k_post1_dots(M A, const V* __rest
     const int per_block = blockDim.x / M::kVS, lane = threadIdx.x % M::kVS;
     for (int row0 = blockIdx.x * per_block; row0 < A.n; row0 += gridDim.x * per_block) {
         const int row = row0 + threadIdx.x / M::kVS;   // every lane runs the dot's shuffles
+        const bool mine = row < A.n && lane == 0;
+        const V yi = mine ? y[row] : V(0), dv = mine ? d[row] : V(0), di = mine ? dinv[row] : V(0);
+        const V bi = mine ? b[row] : V(0);
+        const double ri = mine ? r[row] : 0.0, qi = mine ? q[row] : 0.0;
         const V s = A.dot(row, lane, Vec<V, V>{y});
-        if (row < A.n && lane == 0) {
-            const V zi = y[row] + c1 * d[row] + c2 * (dinv[row] * (b[row] - s));
+        if (mine) {
+            const V zi = yi + c1 * dv + c2 * (di * (bi - s));
             z[row] = zi;
-            const double zd = (double)(zi);
-            zr += zd * r[row];
-            zq += zd * q[row];
+            const double zd = widen<double>(zi);
+            zr += zd * ri;
+            zq += zd * qi;
         }
     }
     zr = block_sum(zr, sh);
@@ -406,7 +538,7 @@ __device__ __forceinline__ double sum_parts(const double* part, int nb, double* 
 // beta from z.r and z.q (part);  w = A z;  q = w + beta q;  p = z + beta p;
 // ppq = p.q   (FP64 SELL operator)
 template <class M, class Z>
-__global__ void __launch_bounds__(kRedThreads) k_outer_mv(M A, const Z* __restrict__ z,
+__global__ void __launch_bounds__(kRedThreads, 4) k_outer_mv(M A, const Z* __restrict__ z,
                                                           double* __restrict__ p, double* __restrict__ q,
                                                           double* __restrict__ scal,
                                                           const double* __restrict__ part, int nb,
@@ -427,9 +559,11 @@ __global__ void __launch_bounds__(kRedThreads) k_outer_mv(M A, const Z* __restri
     double pq = 0.0;
     const int stride = gridDim.x * blockDim.x;
     for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n; row += stride) {
+        const double q0 = q[row], p0 = p[row];
+        const Z zi = z[row];
         const double w = A.dot(row, 0, Vec<double, Z>{z});
-        const double qi = w + beta * q[row];
-        const double pi = (double)(z[row]) + beta * p[row];
+        const double qi = w + beta * q0;
+        const double pi = widen<double>(zi) + beta * p0;
         q[row] = qi;
         p[row] = pi;
         pq += pi * qi;
@@ -466,7 +600,7 @@ __global__ void __launch_bounds__(kRedThreads) k_xr(int n, double* __restrict__ 
         x[i] += alpha * p[i];
         const double ri = r[i] - alpha * q[i];
         r[i] = ri;
-        rv[i] = (V)ri;
+        rv[i] = narrow<V>(ri);
         s += ri * ri;
     }
     s = block_sum(s, sh);
@@ -513,6 +647,28 @@ __global__ void __launch_bounds__(256) k_res64(CsrView<double, 8> A, const doubl
     const int row = g / 8, lane = g % 8;
     const double s = A.dot(row, lane, Vec<double, double>{x});
     if (row < A.n && lane == 0) r[row] = b[row] - s;
+}
+
+// the same on equally wide slices, a thread a row: the products and the order
+// of their sum are those of the 8 lanes above, whose sums take 8 x 4 FP64
+// instructions a row where this takes 2 W: 164 -> 60 us at 128^3 (W = 7, bound
+// by the FP64 unit)
+template <int W>
+__global__ void __launch_bounds__(256) k_res64_even(Sell16UView<double, W> A, const double* __restrict__ x,
+                                                    const double* __restrict__ b, double* __restrict__ r) {
+    const int row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row >= A.n) return;
+    const int k = (row >> 5) * (32 * W) + (row & 31);
+    double t[8] = {};
+    const double bi = b[row];
+#pragma unroll
+    for (int q = 0; q < W; ++q) t[q] = __dmul_rn(A.val[k + 32 * q], __ldg(x + row + (short)A.dcol[k + 32 * q]));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < o; ++q)
+            if (q + o < W) t[q] = __dadd_rn(t[q], t[q + o]);
+    r[row] = bi - t[0];
 }
 
 // --------------------------------------------------------------- SELL build
@@ -590,10 +746,11 @@ void build_sell(cudaStream_t s, const int* ptr, const int* col, const V* val, in
 
 // One warp per slice (blocks of whole warps): the slice's encoding, the base
 // column (smallest column) of every (slice, j) group and the slice's 32-bit
-// column count in wsz (0 unless its encoding is 2).
+// column count in wsz (0 unless its encoding is 2).  most (or null): the widest
+// slice, and whether any has another encoding than 0.
 __global__ void k_sell16_groups(int n, const int* __restrict__ ptr, const int* __restrict__ col,
                                 const int* __restrict__ sptr, int* __restrict__ smode, int* __restrict__ gbase,
-                                int* __restrict__ wsz) {
+                                int* __restrict__ wsz, int* most) {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     const int sl = row >> 5;
     if (sl >= ((n + 31) >> 5)) return;   // whole warps: the test is uniform in a warp
@@ -613,7 +770,15 @@ __global__ void k_sell16_groups(int n, const int* __restrict__ ptr, const int* _
     if ((threadIdx.x & 31) == 0) {
         smode[sl] = mode;
         wsz[sl] = (mode == 2) ? 32 * w : 0;
+        if (most) {
+            if (most[0] < w) atomicMax(most, w);
+            if (mode != 0) most[1] = 1;
+        }
     }
+}
+__global__ void k_sell16_even(int nslices, int width, int* __restrict__ sptr) {
+    const int sl = blockIdx.x * blockDim.x + threadIdx.x;
+    if (sl <= nslices) sptr[sl] = 32 * width * sl;
 }
 
 __global__ void k_sell16_cols(int n, const int* __restrict__ ptr, const int* __restrict__ col,
@@ -654,6 +819,7 @@ __global__ void k_sell16_vals(int n, const int* __restrict__ ptr, const V* __res
 struct Sell16Struct {
     int n = 0, nslices = 0;
     int slots = 0;   // padded entries (sptr[nslices])
+    int width = 0;   // every slice's, when they are made equal (all of mode 0)
     DBuf<int> sptr, smode, gbase, wptr, wcol;
     DBuf<unsigned short> dcol;
 };
@@ -665,18 +831,33 @@ struct Sell16 {
         return Sell16View<V>{st->sptr.p, st->smode.p, st->gbase.p, st->wptr.p, st->dcol.p, st->wcol.p, val.p,
                              st->n};
     }
+    // run f on the view that suits the structure
+    template <class F>
+    void with(F&& f) const {
+        switch (st->width) {
+            case 5: f(Sell16UView<V, 5>{st->dcol.p, val.p, st->n}); break;
+            case 6: f(Sell16UView<V, 6>{st->dcol.p, val.p, st->n}); break;
+            case 7: f(Sell16UView<V, 7>{st->dcol.p, val.p, st->n}); break;
+            default: f(view());
+        }
+    }
 };
 
 // SELL-32 structure with 16-bit columns of a square CSR pattern (slices that
-// fit no 16-bit encoding keep 32-bit columns)
+// fit no 16-bit encoding keep 32-bit columns).  hmost (two pinned ints, or
+// null): make the slices equally wide where Sell16UView has that width, every
+// slice has encoding 0 and it adds at most an eighth of padding -- more costs
+// what the known place gains.
 std::shared_ptr<Sell16Struct> build_sell16_struct(cudaStream_t s, const int* ptr, const int* col, int n,
-                                                  int* hpin) {
+                                                  int* hpin, int* hmost) {
     auto S = std::make_shared<Sell16Struct>();
     S->n = n;
     S->nslices = (n + 31) / 32;
     S->sptr.alloc(S->nslices + 1, s);
     S->wptr.alloc(S->nslices + 1, s);
-    S->smode.alloc(S->nslices, s);
+    S->smode.alloc(S->nslices + 2, s);   // and the widest slice, any encoding but 0
+    int* const most = hmost ? S->smode.p + S->nslices : nullptr;
+    if (most) SEMO_CUDA(cudaMemsetAsync(most, 0, 2 * sizeof(int), s));
     SEMO_CUDA(cudaMemsetAsync(S->sptr.p + S->nslices, 0, sizeof(int), s));
     SEMO_CUDA(cudaMemsetAsync(S->wptr.p + S->nslices, 0, sizeof(int), s));
     const int rows_pad = S->nslices * 32;
@@ -685,9 +866,19 @@ std::shared_ptr<Sell16Struct> build_sell16_struct(cudaStream_t s, const int* ptr
     S->slots = device_scan(s, S->sptr.p, S->nslices + 1, hpin);
     S->gbase.alloc(std::max(S->slots / 32, 1), s);
     k_sell16_groups<<<blocks(rows_pad, 256), 256, 0, s>>>(n, ptr, col, S->sptr.p, S->smode.p, S->gbase.p,
-                                                          S->wptr.p);
+                                                          S->wptr.p, most);
     SEMO_CHECK_LAUNCH();
-    const int wide = device_scan(s, S->wptr.p, S->nslices + 1, hpin);
+    if (most) SEMO_CUDA(cudaMemcpyAsync(hmost, most, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+    const int wide = device_scan(s, S->wptr.p, S->nslices + 1, hpin);   // its sync lands hmost too
+    if (most && hmost[1] == 0 && hmost[0] >= 5 && hmost[0] <= 7) {
+        const int64_t even = 32 * (int64_t)hmost[0] * S->nslices;
+        if (even <= (int64_t)S->slots + S->slots / 8) {
+            S->width = hmost[0];
+            S->slots = (int)even;
+            k_sell16_even<<<blocks(S->nslices + 1, 256), 256, 0, s>>>(S->nslices, S->width, S->sptr.p);
+            SEMO_CHECK_LAUNCH();
+        }
+    }
     S->dcol.alloc(std::max(S->slots, 1), s);
     S->wcol.alloc(std::max(wide, 1), s);
     k_sell16_cols<<<blocks(rows_pad, 256), 256, 0, s>>>(n, ptr, col, S->sptr.p, S->smode.p, S->gbase.p, S->wptr.p,
@@ -706,21 +897,17 @@ void fill_sell16(cudaStream_t s, const int* ptr, const V* val, const std::shared
     SEMO_CHECK_LAUNCH();
 }
 template <class V, class W>
-bool build_sell16(cudaStream_t s, const int* ptr, const int* col, const V* val, int n, Sell16<W>& S, int* hpin) {
-    fill_sell16<V, W>(s, ptr, val, build_sell16_struct(s, ptr, col, n, hpin), S);
+bool build_sell16(cudaStream_t s, const int* ptr, const int* col, const V* val, int n, Sell16<W>& S, int* hpin,
+                  int* hmost) {
+    fill_sell16<V, W>(s, ptr, val, build_sell16_struct(s, ptr, col, n, hpin, hmost), S);
     return true;
 }
 
-// The FP64 outer operator: 16-bit column offsets when they fit, else SELL-32
+// The FP64 outer operator
 struct OuterOp {
-    Sell<double> s32;
     Sell16<double> s16;
-    bool use16 = false;
     template <class F>
-    void with(F&& f) const {
-        if (use16) f(s16.view());
-        else f(s32.view());
-    }
+    void with(F&& f) const { s16.with(f); }
 };
 
 struct ChebCoef {
@@ -777,7 +964,7 @@ void with_op(const Sell<V>& S, bool use_sell, const DCsr<V>& M, F&& f) {
 // the level's A: 16-bit-offset SELL, SELL, or CSR
 template <class V, class F>
 void with_A(const LevelMats<V>& M, const DCsr<V>& A, F&& f) {
-    if (M.a16) f(M.A16.view());
+    if (M.a16) M.A16.with(f);
     else with_op(M.A, M.a, A, f);
 }
 
@@ -939,7 +1126,16 @@ void chebyshev_generic(cudaStream_t s, AmgLevel<V>& L, int degree, bool zero_sta
     }
 }
 
-// V-cycle from level l down, input L.b, output L.x
+// what writes level l's b writes beside it: d0, on the levels that k_pre2 starts
+template <class V>
+FirstIterate<V> first_iterate(semo_ctx* c, Amg<V>& h, const Cycle<V>& cy, int l) {
+    AmgLevel<V>& L = h.lev[l];
+    if (l == (int)h.lev.size() - 1 || l == cy.local_from || cy.lev[l].gs || c->prm.cheb_degree != 2)
+        return FirstIterate<V>{nullptr, V(0), nullptr};
+    return FirstIterate<V>{L.dinv.p, (V)cheb2(L.lam_max).inv_theta, L.t.p};
+}
+
+// V-cycle from level l down, input L.b (and d0 below the finest level), output L.x
 template <class V>
 void vcycle_from(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, int l) {
     cudaStream_t s = c->stream;
@@ -961,15 +1157,21 @@ void vcycle_from(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, int l) {
         gs_sweep(s, L, M, false, true);   // forward sweep from x = 0
     } else if (degree == 2) {
         with_A(M, L.A, [&](auto A) {
-            launch_pdl(k_pre2<decltype(A), V>, grid_for(A), 256, s, A, L.dinv.p, L.b.p, (V)cc.inv_theta, (V)cc.c1,
-                       (V)cc.c2, L.x.p);
+            if (l == 0)
+                launch_pdl(k_pre2<decltype(A), V, FirstGather<V>>, grid_for(A), 256, s, A, L.dinv.p, L.b.p,
+                           FirstGather<V>{L.dinv.p, L.b.p, (V)cc.inv_theta}, (V)cc.c1, (V)cc.c2, L.x.p);
+            else
+                launch_pdl(k_pre2<decltype(A), V, Vec<V, V>>, grid_for(A), 256, s, A, L.dinv.p, L.b.p,
+                           Vec<V, V>{L.t.p}, (V)cc.c1, (V)cc.c2, L.x.p);
         });
     } else {
         chebyshev_generic(s, L, degree, true);
     }
     with_A(M, L.A, [&](auto A) { launch_pdl(k_res<decltype(A), V>, grid_for(A), 256, s, A, L.x.p, L.b.p, L.r.p); });
     AmgLevel<V>& C = h.lev[l + 1];
-    with_op(M.R, M.r, L.R, [&](auto R) { launch_pdl(k_mv<decltype(R), V>, grid_for(R), 256, s, R, L.r.p, C.b.p); });
+    with_op(M.R, M.r, L.R, [&](auto R) {
+        launch_pdl(k_mv<decltype(R), V>, grid_for(R), 256, s, R, L.r.p, C.b.p, first_iterate(c, h, cy, l + 1));
+    });
     vcycle_from(c, h, cy, l + 1);
     with_op(M.P, M.p, L.P,
             [&](auto P) { launch_pdl(k_prolong_add<decltype(P), V>, grid_for(P), 256, s, P, C.x.p, L.x.p); });
@@ -1132,13 +1334,20 @@ void pcg(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const OuterOp& outer, const int* 
         pcg_outcome(h2, 0, info);
         return;
     }
-    const CsrView<double, 8> A8{ptr, col, val, n};
+    auto residual = [&] {
+        outer.with([&](auto A) {
+            if constexpr (decltype(A)::kEven > 0)
+                k_res64_even<decltype(A)::kEven><<<blocks(n, 256), 256, 0, s>>>(A, x, b, r);
+            else
+                k_res64<<<blocks((int64_t)n * 8, 256), 256, 0, s>>>(CsrView<double, 8>{ptr, col, val, n}, x, b, r);
+        });
+        SEMO_CHECK_LAUNCH();
+    };
     if (zero_guess) {
         SEMO_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * n, s));
         SEMO_CUDA(cudaMemcpyAsync(r, b, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
     } else {
-        k_res64<<<blocks((int64_t)n * 8, 256), 256, 0, s>>>(A8, x, b, r);
-        SEMO_CHECK_LAUNCH();
+        residual();
     }
     k_conv<double, V><<<blocks(n, 256), 256, 0, s>>>(n, r, h.lev[0].b.p);
     SEMO_CHECK_LAUNCH();
@@ -1197,8 +1406,7 @@ void pcg(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const OuterOp& outer, const int* 
     SEMO_CUDA(cudaGraphInstantiate(&gg.e, gg.g, 0));
     SEMO_CUDA(cudaGraphLaunch(gg.e, s));
     // true FP64 residual of the returned solution -> scal[16]
-    k_res64<<<blocks((int64_t)n * 8, 256), 256, 0, s>>>(A8, x, b, r);
-    SEMO_CHECK_LAUNCH();
+    residual();
     k_dot<<<nb, kRedThreads, 0, s>>>(n, r, r, R.part);
     SEMO_CHECK_LAUNCH();
     k_fin_sum<<<1, kRedThreads, 0, s>>>(R.part, nb, R.scal + 16);
@@ -1270,7 +1478,8 @@ void prepare_cycle(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const std::shared_ptr<S
             fill_sell16<V, V>(s, L.A.ptr, L.A.val, lev0, M.A16);
             M.a16 = true;
         } else {
-            M.a16 = M.a && build_sell16<V, V>(s, L.A.ptr, L.A.col, L.A.val, L.A.n, M.A16, hp);
+            M.a16 = M.a && build_sell16<V, V>(s, L.A.ptr, L.A.col, L.A.val, L.A.n, M.A16, hp,
+                                                  l == 0 ? c->hpin_int + 14 : nullptr);
         }
         if (M.a16) M.a = false;
         if (M.a) build_sell<V, V>(s, L.A.ptr, L.A.col, L.A.val, L.A.n, M.A, hp);
@@ -1638,18 +1847,17 @@ void pressure_setup(semo_ctx* c, const int* ptr, const int* col, const double* v
             std::shared_ptr<Sell16Struct> pat;
             if (ptr == c->A_ptr.p && col == c->A_col.p) {
                 if (!st.pat16 || st.pat16_gen != c->mesh_gen || st.pat16->n != n)
-                    st.pat16 = build_sell16_struct(s, ptr, col, n, c->hpin_int + 4);
+                    st.pat16 = build_sell16_struct(s, ptr, col, n, c->hpin_int + 4, c->hpin_int + 14);
                 st.pat16_gen = c->mesh_gen;
                 pat = st.pat16;
             } else {
-                pat = build_sell16_struct(s, ptr, col, n, c->hpin_int + 4);
+                pat = build_sell16_struct(s, ptr, col, n, c->hpin_int + 4, c->hpin_int + 14);
             }
             if (c->prm.precision == SEMO_PREC_MIXED)
                 prepare_cycle(c, c->amg32, st.cy32, pat);
             else
                 prepare_cycle(c, c->amg64, st.cy64, pat);
             fill_sell16<double, double>(s, ptr, val, pat, st.outer.s16);
-            st.outer.use16 = true;
             st.src_prec = -1;
             if (may_reuse && c->prm.reuse_hierarchy) {
                 st.src_val.alloc(nnz, s);
@@ -1969,9 +2177,9 @@ double time_spmv(semo_ctx* c, int which, int reps) {
             if (which == 0) {
                 AmgLevel<V>& L = h.lev[0];
                 with_A(pressure_cycle<V>(st).lev[0], L.A,
-                       [&](auto A) { k_mv<<<grid_for(A), 256, 0, s>>>(A, L.x.p, L.t.p); });
+                       [&](auto A) { k_mv<<<grid_for(A), 256, 0, s>>>(A, L.x.p, L.r.p, FirstIterate<V>{}); });
             } else {
-                st.outer.with([&](auto A) { k_mv<<<grid_for(A), 256, 0, s>>>(A, c->kp.p, c->kq.p); });
+                st.outer.with([&](auto A) { k_mv<<<grid_for(A), 256, 0, s>>>(A, c->kp.p, c->kq.p, FirstIterate<double>{}); });
             }
             SEMO_CHECK_LAUNCH();
         }
