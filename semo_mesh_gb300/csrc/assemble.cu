@@ -118,36 +118,24 @@ __global__ void k_grav_face(int nf, int ni, int nc, int nb, const int* __restric
 
 __global__ void k_grav_cell(int nc, int nf, const int* __restrict__ cfp, const int* __restrict__ cfi,
                             const double* __restrict__ fn, const double* __restrict__ fa,
-                            const double* __restrict__ vol, const double* __restrict__ gf, double* __restrict__ sg) {
+                            const double* __restrict__ ivol, const double* __restrict__ gf,
+                            double* __restrict__ sg) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nc) return;
-    // one reciprocal per cell instead of four divisions per face (FP64 division
-    // is the bottleneck here on GB300); agrees with SEMO's x*n*A/V to rounding
-    const double iv = 1.0 / vol[i];
+    // the cell's reciprocal volume, stored and applied at the end, instead of four
+    // divisions a face (the FP64 unit bounds this kernel: with k_grav_face 0.26 ->
+    // 0.19 ms at 96^3); agrees with SEMO's x*n*A/V to rounding
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
     for (int k = cfp[i]; k < cfp[i + 1]; ++k) {
         const int e = cfi[k], f = e & kFaceMask;
         const double n0 = fn[f], n1 = fn[nf + f], n2 = fn[2 * nf + f], a = fa[f];
         const double un = gf[2 * nf + f];
-        if (e >> 30) {
-            const double w = gf[nf + f] * a * iv;
-            s0 -= w * n0; s1 -= w * n1; s2 -= w * n2; s3 -= w * un;
-        } else {
-            const double w = gf[f] * a * iv;
-            s0 += w * n0; s1 += w * n1; s2 += w * n2; s3 += w * un;
-        }
+        const bool nei = e >> 30;
+        const double w = signed_by(gf[nei ? nf + f : f] * a, nei);
+        s0 += w * n0; s1 += w * n1; s2 += w * n2; s3 += w * un;
     }
-    sg[i] = s0; sg[nc + i] = s1; sg[2 * nc + i] = s2; sg[3 * nc + i] = s3;
-}
-
-// SEMO's clamp sequence (if x <= lo: x = lo; if x >= hi: x = hi) on the
-// integer pipes
-__device__ __forceinline__ double clamp_seq(double x, double lo, double hi) {
-    long long k = okey(x);
-    const long long kl = okey(lo), kh = okey(hi);
-    if (k <= kl) k = kl;
-    if (k >= kh) k = kh;
-    return ounkey(k);
+    const double iv = ivol[i];
+    sg[i] = s0 * iv; sg[nc + i] = s1 * iv; sg[2 * nc + i] = s2 * iv; sg[3 * nc + i] = s3 * iv;
 }
 
 // Pressure-matrix coefficients, written with explicit roundings so that the
@@ -273,33 +261,35 @@ __global__ void k_gg_face(int nf, int ni, int nc, int nb, const int* __restrict_
     if (f < ni) {
         const int q = nei[f];
         const double wL = wc[f], wR = 1.0 - wL;
-        double v = wL * x[o] + wR * x[q];
+        double l = x[o], r = x[q];   // each side's value, then the weights: 9 FP64 instructions, term by term 15
         for (int k = 0; k < 3; ++k) {
             const double s = skew[(size_t)k * nf + f];
-            v += wL * g[(size_t)k * nc + o] * s;
-            v += wR * g[(size_t)k * nc + q] * s;
+            l += g[(size_t)k * nc + o] * s;
+            r += g[(size_t)k * nc + q] * s;
         }
-        vF[f] = v;
+        vF[f] = wL * l + wR * r;
     } else {
         vF[f] = (bct[3 * bpatch[f - ni]] == SEMO_BC_FIXED_VALUE) ? 0.0 : x[o];
     }
 }
 
+// Bound by the FP64 unit as k_gg_face: one product, three multiply-adds a face
+// (the sign by an integer instruction), the reciprocal volume stored and applied
+// once.  Both sweeps of both kernels: 0.91 -> 0.43 ms at 128^3, 0.40 -> 0.20 at
+// 96^3.
 __global__ void k_gg_cell(int nc, int nf, const int* __restrict__ cfp, const int* __restrict__ cfi,
                           const double* __restrict__ fn, const double* __restrict__ fa,
-                          const double* __restrict__ vol, const double* __restrict__ vF, double* __restrict__ g) {
+                          const double* __restrict__ ivol, const double* __restrict__ vF, double* __restrict__ g) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nc) return;
-    const double iv = 1.0 / vol[i];   // one reciprocal per cell, not three divisions per face
     double g0 = 0.0, g1 = 0.0, g2 = 0.0;
     for (int k = cfp[i]; k < cfp[i + 1]; ++k) {
         const int e = cfi[k], f = e & kFaceMask;
-        const double w = vF[f] * fa[f] * iv;
-        const double c0 = w * fn[f], c1 = w * fn[nf + f], c2 = w * fn[2 * nf + f];
-        if (e >> 30) { g0 -= c0; g1 -= c1; g2 -= c2; }
-        else { g0 += c0; g1 += c1; g2 += c2; }
+        const double w = signed_by(vF[f] * fa[f], e >> 30);
+        g0 += w * fn[f]; g1 += w * fn[nf + f]; g2 += w * fn[2 * nf + f];
     }
-    g[i] = g0; g[nc + i] = g1; g[2 * (size_t)nc + i] = g2;
+    const double iv = ivol[i];
+    g[i] = g0 * iv; g[nc + i] = g1 * iv; g[2 * (size_t)nc + i] = g2 * iv;
 }
 
 // The divisions dt/rho use the EOS's reciprocal density (one FP64 division a
@@ -438,7 +428,7 @@ void assemble_gravity(semo_ctx* c) {
                                                  c->W, c->irho, c->bface, c->phys.gravity[0], c->phys.gravity[1],
                                                  c->phys.gravity[2], c->fscr);
         SEMO_CHECK_LAUNCH();
-        k_grav_cell<<<blocks(nc, T), T, 0, s>>>(nc, nf, c->cf_ptr, c->cf_idx, c->fn, c->fa, c->vol, c->fscr, c->sg);
+        k_grav_cell<<<blocks(nc, T), T, 0, s>>>(nc, nf, c->cf_ptr, c->cf_idx, c->fn, c->fa, c->ivol, c->fscr, c->sg);
         SEMO_CHECK_LAUNCH();
     } else {
         c->sg.zero();
@@ -466,7 +456,7 @@ void assemble_pressure(semo_ctx* c) {
         FaceArgs a;
         a.ni = ni; a.nf = nf; a.nc = nc;
         a.own = c->own; a.nei = c->nei; a.lr = c->A_lr; a.rl = c->A_rl;
-        a.fn = c->fn; a.epn = c->epn; a.skew = c->skew; a.alf = c->alf; a.fk = c->fk;
+        a.fn = c->fn; a.skew = c->skew; a.alf = c->alf; a.fk = c->fk;
         a.P = c->P; a.U = c->U; a.V = c->V; a.W = c->W; a.irho = c->irho; a.grad = c->grad; a.mm = c->mm; a.sg = c->sg;
         a.dt = c->phys.dt; a.g0 = c->phys.gravity[0]; a.g1 = c->phys.gravity[1]; a.g2 = c->phys.gravity[2];
         a.use_gravity = c->phys.use_gravity;
@@ -516,7 +506,7 @@ double pressure_update(semo_ctx* c) {
         k_gg_face<<<blocks(nf, T), T, 0, s>>>(nf, ni, nc, nb, c->own, c->nei, c->bpatch, c->bc_type, c->wc, c->skew,
                                                c->x, c->gx, vF);
         SEMO_CHECK_LAUNCH();
-        k_gg_cell<<<blocks(nc, T), T, 0, s>>>(nc, nf, c->cf_ptr, c->cf_idx, c->fn, c->fa, c->vol, vF, c->gx);
+        k_gg_cell<<<blocks(nc, T), T, 0, s>>>(nc, nf, c->cf_ptr, c->cf_idx, c->fn, c->fa, c->ivol, vF, c->gx);
         SEMO_CHECK_LAUNCH();
     }
     c->red.alloc(4 * kRedBlocks + 32, s);

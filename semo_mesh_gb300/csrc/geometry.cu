@@ -98,7 +98,8 @@ __global__ void k_face_polygon(int nf, const double* __restrict__ pts, const int
 
 __global__ void k_cell_volume(int nc, int nf, const int* __restrict__ cfp, const int* __restrict__ cfi,
                               const double* __restrict__ vsn3, const double* __restrict__ cen,
-                              double* __restrict__ vol, double* __restrict__ cc, int* __restrict__ flag) {
+                              double* __restrict__ vol, double* __restrict__ ivol, double* __restrict__ cc,
+                              int* __restrict__ flag) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nc) return;
     double v = 0.0, x = 0.0, y = 0.0, z = 0.0;
@@ -109,6 +110,7 @@ __global__ void k_cell_volume(int nc, int nf, const int* __restrict__ cfp, const
     }
     const double s = 1.0 / (24.0 * 2.0 * v);
     vol[i] = v;
+    ivol[i] = 1.0 / v;
     cc[i] = x * s; cc[nc + i] = y * s; cc[2 * nc + i] = z * s;
     if (!(v >= 2.2250738585072014e-308)) atomicExch(flag + 0, 1);   // non-positive volume
 }
@@ -216,13 +218,15 @@ __global__ void k_lsq_setup(int nc, int nf, int ni, const int* __restrict__ stp,
 // Per-internal-face constants of the pressure face kernel:
 // kA = alpha*area/magPN (coefficient factor), kP = alpha/magPN (pressure jump).
 __global__ void k_face_consts(int ni, int nf, const double* __restrict__ fa, const double* __restrict__ mpn,
-                              const double* __restrict__ alf, const double* __restrict__ wc, double* __restrict__ fk) {
+                              const double* __restrict__ alf, const double* __restrict__ wc,
+                              const double* __restrict__ epn, double* __restrict__ fk) {
     int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= ni) return;
     fk[f] = alf[f] * fa[f] / mpn[f];
     fk[ni + f] = alf[f] / mpn[f];
-    fk[2 * ni + f] = fa[f];
-    fk[3 * ni + f] = wc[f];
+    fk[2 * (size_t)ni + f] = fa[f];
+    fk[3 * (size_t)ni + f] = wc[f];
+    for (int k = 0; k < 3; ++k) fk[(4 + k) * (size_t)ni + f] = alf[f] * epn[(size_t)k * nf + f];
 }
 
 inline int blocks(int64_t n, int t) { return (int)((n + t - 1) / t); }
@@ -238,11 +242,11 @@ void geometry_build(semo_ctx* c, const double* d_points, const int* d_fptr, cons
     c->fn.alloc(3 * (size_t)nf, s); c->fa.alloc(nf, s); c->fc.alloc(3 * (size_t)nf, s);
     c->wc.alloc(nf, s); c->mpn.alloc(nf, s); c->alf.alloc(nf, s); c->epn.alloc(3 * (size_t)nf, s);
     c->skew.alloc(3 * (size_t)nf, s); c->pf.alloc(3 * (size_t)nf, s); c->nfv.alloc(3 * (size_t)nf, s);
-    c->vol.alloc(nc, s); c->cc.alloc(3 * (size_t)nc, s); c->minv.alloc(6 * (size_t)nc, s);
+    c->vol.alloc(nc, s); c->ivol.alloc(nc, s); c->cc.alloc(3 * (size_t)nc, s); c->minv.alloc(6 * (size_t)nc, s);
     c->stw.alloc(3 * (size_t)std::max<int64_t>(c->st_nnz, 1), s);
     c->bfw.alloc(3 * (size_t)std::max(nb, 1), s);
     c->stws.alloc(3 * (size_t)nc, s);
-    c->fk.alloc(4 * (size_t)std::max(ni, 1), s);
+    c->fk.alloc(7 * (size_t)std::max(ni, 1), s);
     DBuf<double> vsn3, cen;
     vsn3.alloc(nf, s);
     cen.alloc(3 * (size_t)nf, s);
@@ -250,7 +254,8 @@ void geometry_build(semo_ctx* c, const double* d_points, const int* d_fptr, cons
     const int T = 128;
     k_face_polygon<<<blocks(nf, T), T, 0, s>>>(nf, d_points, d_fptr, d_fpts, c->fn, c->fa, c->fc, vsn3, cen);
     SEMO_CHECK_LAUNCH();
-    k_cell_volume<<<blocks(nc, T), T, 0, s>>>(nc, nf, c->cf_ptr, c->cf_idx, vsn3, cen, c->vol, c->cc, c->flag);
+    k_cell_volume<<<blocks(nc, T), T, 0, s>>>(nc, nf, c->cf_ptr, c->cf_idx, vsn3, cen, c->vol, c->ivol, c->cc,
+                                              c->flag);
     SEMO_CHECK_LAUNCH();
     k_face_weights<<<blocks(nf, T), T, 0, s>>>(nf, ni, nc, c->own, c->nei, c->cc, c->fn, c->fc, c->wc, c->mpn,
                                                 c->alf, c->epn, c->skew, c->pf, c->nfv);
@@ -260,7 +265,7 @@ void geometry_build(semo_ctx* c, const double* d_points, const int* d_fptr, cons
     SEMO_CHECK_LAUNCH();
     stencil_weights(c);
     if (ni > 0) {
-        k_face_consts<<<blocks(ni, T), T, 0, s>>>(ni, nf, c->fa, c->mpn, c->alf, c->wc, c->fk);
+        k_face_consts<<<blocks(ni, T), T, 0, s>>>(ni, nf, c->fa, c->mpn, c->alf, c->wc, c->epn, c->fk);
         SEMO_CHECK_LAUNCH();
     }
     int hflag[2] = {0, 0};

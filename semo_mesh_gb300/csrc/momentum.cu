@@ -39,8 +39,6 @@ struct MomArgs {
     double* sc;
 };
 
-__device__ __forceinline__ double kept(double a) { return (fabs(a) < DBL_MIN) ? 0.0 : a; }
-
 __global__ void __launch_bounds__(256) k_mface(MomArgs m) {
     const FaceArgs& a = m.a;
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -56,28 +54,25 @@ __global__ void __launch_bounds__(256) k_mface(MomArgs m) {
     const double muF = 1.0 / (g.wL * __ldg(m.mu + N + o) + g.wR * __ldg(m.mu + N + q));
     // first-order upwind on UnF (eqMomentum.cpp:613-620)
     // face pressure, skew-corrected and limited by both cells (eqMomentum.cpp:617-659)
-    double PF = g.wL * __ldg(a.P + o) + g.wR * __ldg(a.P + q);
-    PF += g.wL * __ldg(G + o) * g.s0;
-    PF += g.wR * __ldg(G + q) * g.s0;
-    PF += g.wL * __ldg(G + N + o) * g.s1;
-    PF += g.wR * __ldg(G + N + q) * g.s1;
-    PF += g.wL * __ldg(G + 2 * N + o) * g.s2;
-    PF += g.wR * __ldg(G + 2 * N + q) * g.s2;
+    const double pl = __ldg(a.P + o) + __ldg(G + o) * g.s0 + __ldg(G + N + o) * g.s1 + __ldg(G + 2 * N + o) * g.s2;
+    const double pr = __ldg(a.P + q) + __ldg(G + q) * g.s0 + __ldg(G + N + q) * g.s1 + __ldg(G + 2 * N + q) * g.s2;
+    double PF = g.wL * pl + g.wR * pr;
     PF = clamp_k(PF, __ldg(M + 9 * N + o), __ldg(M + 8 * N + o));
     PF = clamp_k(PF, __ldg(M + 9 * N + q), __ldg(M + 8 * N + q));
     const double UL = __ldg(a.U + o), VL = __ldg(a.V + o), WL = __ldg(a.W + o);
     const double UR = __ldg(a.U + q), VR = __ldg(a.V + q), WR = __ldg(a.W + q);
     // the upwind weights are 0 or 1: selections, not FP64 arithmetic
-    const bool up = UnF > 0.0;
+    const bool up = positive(UnF);
     const double UF = up ? UL : UR, VFh = up ? VL : VR, WFh = up ? WL : WR;
     const double area = g.area, mf = UnF * area;
     const double ad = muF * g.kA;   // alpha muF / |PN| * area
     const double rlm = RhoL * mf, rrm = RhoR * mf;
     // coefficients (eqMomentum.cpp:694-712)
-    const double dO = up ? rlm + ad : ad;
-    const double dN = up ? -ad : rrm - ad;
-    a.val[a.lr[f]] = kept(up ? -ad : rlm - ad);
-    a.val[a.rl[f]] = kept(up ? -(rrm + ad) : -ad);
+    const double ads = signed_by(ad, !up), cl = rlm + ads, cr = rrm + ads;   // + ad upwind, - ad downwind
+    const double dO = up ? cl : ad;
+    const double dN = up ? -ad : cr;
+    a.val[a.lr[f]] = kept(up ? -ad : cl);
+    a.val[a.rl[f]] = kept(up ? -cr : -ad);
     // convection + pressure, over-relaxed diffusion with its non-orthogonal
     // part on (n - alpha e), and SEMO's extra grad.n term (eqMomentum.cpp:739-779)
     const double t0 = g.n0 - g.ae0, t1 = g.n1 - g.ae1, t2 = g.n2 - g.ae2;
@@ -93,14 +88,16 @@ __global__ void __launch_bounds__(256) k_mface(MomArgs m) {
         const double uf = (c == 0) ? UF : (c == 1 ? VFh : WFh);
         const double dl = (c == 0) ? UR - UL : (c == 1 ? VR - VL : WR - WL);
         const double nc = (c == 0) ? g.n0 : (c == 1 ? g.n1 : g.n2);
-        const double pn = pa * nc;
-        // (wL gL + wR gR).t = wL (gL.t) + wR (gR.t): the projections serve both terms
+        // (wL gL + wR gR).t = wL (gL.t) + wR (gR.t): the projections serve both
+        // sides, and a side's grad.n joins them before the product with mu A
         const double glt = gl0 * t0 + gl1 * t1 + gl2 * t2, grt = gr0 * t0 + gr1 * t1 + gr2 * t2;
-        const double diff = ad * dl + ma * (g.wL * glt + g.wR * grt);
-        const double dLn = ma * (gl0 * g.n0 + gl1 * g.n1 + gl2 * g.n2);
-        const double dRn = ma * (gr0 * g.n0 + gr1 * g.n1 + gr2 * g.n2);
-        sc[(2 + c) * NF + f] = (rlm * uf + pn) - diff - dLn;
-        sc[(5 + c) * NF + f] = (rrm * uf + pn) - diff - dRn;
+        const double x = g.wL * glt + g.wR * grt;
+        double yl = x, yr = x;
+        yl += gl0 * g.n0; yl += gl1 * g.n1; yl += gl2 * g.n2;
+        yr += gr0 * g.n0; yr += gr1 * g.n1; yr += gr2 * g.n2;
+        const double pd = pa * nc - ad * dl;
+        sc[(2 + c) * NF + f] = (rlm * uf + pd) - ma * yl;
+        sc[(5 + c) * NF + f] = (rrm * uf + pd) - ma * yr;
     }
 }
 
@@ -149,7 +146,9 @@ __global__ void k_mbface(int nb, int ni, int nf, int nc, const int* __restrict__
     }
 }
 
-__global__ void k_mcell(int nc, int ni, int nf, double dt, const int* __restrict__ cfp, const int* __restrict__ cfi,
+// 4 FP64 additions a face and ~30 a cell (0.072 -> 0.049 ms at 75^3 without the
+// divisions by dt), then the 8 planes of face terms.
+__global__ void k_mcell(int nc, int ni, int nf, double idt, const int* __restrict__ cfp, const int* __restrict__ cfi,
                         const int* __restrict__ dig, const double* __restrict__ rho, const double* __restrict__ vol,
                         const double* __restrict__ U, const double* __restrict__ V, const double* __restrict__ W,
                         const double* __restrict__ old, int has_old, const double* __restrict__ sg,
@@ -160,13 +159,14 @@ __global__ void k_mcell(int nc, int ni, int nf, double dt, const int* __restrict
     const size_t N = nc, NF = nf;
     const double r = rho[i], v = vol[i];
     const double cur[3] = {U[i], V[i], W[i]};
-    double d = r * 1.5 * v / dt;
+    const double rv = r * v * idt;   // one product with 1/dt, not four divisions
+    double d = 1.5 * rv;
     double b[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const double o1 = has_old ? old[c * N + i] : cur[c];
         const double o2 = has_old ? old[(3 + c) * N + i] : cur[c];
-        b[c] = -r * (1.5 * cur[c] - 2.0 * o1 + 0.5 * o2) * v / dt;
+        b[c] = -rv * (1.5 * cur[c] - 2.0 * o1 + 0.5 * o2);
         b[c] += v * sg[c * N + i];
         if (sft) b[c] += v * sft[c * N + i];   // surface tension (eqMomentum.cpp:320-322)
     }
@@ -236,7 +236,7 @@ void assemble_momentum(semo_ctx* c, bool face_values_done) {
         FaceArgs& a = m.a;
         a.ni = ni; a.nf = nf; a.nc = nc;
         a.own = c->own; a.nei = c->nei; a.lr = c->A_lr; a.rl = c->A_rl;
-        a.fn = c->fn; a.epn = c->epn; a.skew = c->skew; a.alf = c->alf; a.fk = c->fk;
+        a.fn = c->fn; a.skew = c->skew; a.alf = c->alf; a.fk = c->fk;
         a.P = c->P; a.U = c->U; a.V = c->V; a.W = c->W; a.irho = c->irho; a.grad = c->grad; a.mm = c->mm; a.sg = c->sg;
         a.dt = c->phys.dt; a.g0 = c->phys.gravity[0]; a.g1 = c->phys.gravity[1]; a.g2 = c->phys.gravity[2];
         a.use_gravity = c->phys.use_gravity;
@@ -255,7 +255,7 @@ void assemble_momentum(semo_ctx* c, bool face_values_done) {
         SEMO_CHECK_LAUNCH();
     }
     StageScope sc(c, ST_MCELL);
-    k_mcell<<<blocks(nc, T), T, 0, s>>>(nc, ni, nf, c->phys.dt, c->cf_ptr, c->cf_idx, c->A_dig, c->rho, c->vol,
+    k_mcell<<<blocks(nc, T), T, 0, s>>>(nc, ni, nf, 1.0 / c->phys.dt, c->cf_ptr, c->cf_idx, c->A_dig, c->rho, c->vol,
                                          c->U, c->V, c->W, c->has_old ? c->old.p : nullptr, c->has_old ? 1 : 0,
                                          c->sg, (c->phys.sigma != 0.0 && c->sft_current) ? c->sft.p + 2 * (size_t)nc : nullptr,
                                          c->msc, c->Am_val, c->bm);

@@ -157,7 +157,7 @@ struct semo_ctx {
     semo::DBuf<double> bc_value;                  // npatch*5
     // geometry (SoA, 3-vectors stored as 3 planes of length nf or nc)
     semo::DBuf<double> fn, fa, fc, wc, mpn, alf, epn, skew, pf, nfv;
-    semo::DBuf<double> vol, cc, minv;             // cc: 3 planes; minv: 6 planes
+    semo::DBuf<double> vol, ivol, cc, minv;       // ivol: 1 / vol; cc: 3 planes; minv: 6 planes
     semo::DBuf<double> stw;                       // 3 planes of st_nnz: w_k * d_k (LSQ weight vectors)
     semo::DBuf<double> bfw;                       // 3 planes of nb: boundary-face LSQ weight vectors
     semo::DBuf<double> stws;                      // 3 planes of nc: per-cell sum of the stencil and boundary weights
@@ -168,7 +168,7 @@ struct semo_ctx {
     semo::DBuf<int> st_tpos;                      // per stencil entry (j, i): the entry's position in i's row (adjoint)
     int st_tpos_gen = -1;                         // mesh generation st_tpos was built for
     // derived per-face constants for the hot face kernel
-    semo::DBuf<double> fk;                        // 4 planes of ni: kA = alpha*area/magPN, kP = alpha/magPN, area, wC
+    semo::DBuf<double> fk;                        // 7 planes of ni: kA = alpha*area/magPN, kP = alpha/magPN, area, wC, alpha*ePN (3)
 
     // ---- CSR pattern (RCM order) ----
     semo::DBuf<int> A_ptr, A_col, A_dig, A_lr, A_rl;

@@ -140,14 +140,14 @@ __global__ void __launch_bounds__(256) k_vface(VofArgs m) {
     const int o = a.own[f], q = a.nei[f];
     const FaceGeo g = load_geo(a, f);
     const double UnF = face_unf(a, g, o, q);
-    const double wLu = (UnF > 0.0) ? 1.0 : 0.0, wRu = 1.0 - wLu;
-    const double vff = wLu * m.fvf[f] + wRu * m.fvf[a.ni + f];
+    const bool up = positive(UnF);   // the upwind weights are 0 or 1: selections
+    const double vff = up ? m.fvf[f] : m.fvf[a.ni + f];
     const double mf = UnF * g.area;
-    a.val[a.lr[f]] = kept(wRu * mf);
-    a.val[a.rl[f]] = kept(-(wLu * mf));
+    a.val[a.lr[f]] = up ? 0.0 : kept(mf);
+    a.val[a.rl[f]] = up ? kept(-mf) : 0.0;
     const size_t NF = a.nf;
-    m.sc[f] = wLu * mf;
-    m.sc[NF + f] = wRu * mf;
+    m.sc[f] = up ? mf : 0.0;
+    m.sc[NF + f] = up ? 0.0 : mf;
     m.sc[2 * NF + f] = vff * mf;
 }
 
@@ -253,7 +253,7 @@ void assemble_vof(semo_ctx* c) {
         FaceArgs& a = m.a;
         a.ni = ni; a.nf = nf; a.nc = nc;
         a.own = c->own; a.nei = c->nei; a.lr = c->A_lr; a.rl = c->A_rl;
-        a.fn = c->fn; a.epn = c->epn; a.skew = c->skew; a.alf = c->alf; a.fk = c->fk;
+        a.fn = c->fn; a.skew = c->skew; a.alf = c->alf; a.fk = c->fk;
         a.P = c->P; a.U = c->U; a.V = c->V; a.W = c->W; a.irho = c->irho; a.grad = c->grad; a.mm = c->mm; a.sg = c->sg;
         a.dt = c->phys.dt; a.g0 = c->phys.gravity[0]; a.g1 = c->phys.gravity[1]; a.g2 = c->phys.gravity[2];
         a.use_gravity = c->phys.use_gravity;
