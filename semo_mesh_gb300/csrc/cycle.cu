@@ -1493,263 +1493,395 @@ void prepare_cycle(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const std::shared_ptr<S
 // ---------------------------------- momentum and VOF: batched BiCGStab
 // NR right-hand sides (3 for the velocity components, 1 for the volume
 // fraction) share one matrix: every kernel walks the rows once and serves all
-// of them, so the operator is read once per product for the NR systems.  Right preconditioning by D^-1 (the momentum
-// matrix is dominated by its BDF2 diagonal at the time steps of interest).
+// of them, so the operator is read once per product for the NR systems.  Right
+// preconditioning by D^-1 (the momentum matrix is dominated by its BDF2 diagonal
+// at the time steps of interest): the iteration solves B xh = b, B = A D^-1, and
+// x = D^-1 xh at the end.  B's diagonal is 1 and is not stored: a product starts
+// from the row's own value and adds the off-diagonal entries.
+// What bounds the iteration is the FP64 unit (2 lanes a clock and
+// multiprocessor): 72 instructions a row and iteration of three systems, and
+// 548 bytes.  So D^-1 p and D^-1 s are never formed (the search directions
+// themselves are gathered), rho comes from the sums of the second product,
+// rho' = (rh,s) - omega (rh,t), which lets one kernel end an iteration and
+// begin the next, and every scalar is formed by the kernels that use it: five
+// kernels an iteration.
 // Per system j the scalars live at scal[16 j + k]:
-//   0 rho, 1 alpha, 2 omega, 3 beta, 4 (rh,v), 5 (t,s), 6 (t,t), 7 (r,r),
-//   8 (b,b), 9 active, 10 breakdown, 11 iterations
+//   0 rho, 1 alpha, 2 omega, 7 (r,r), 8 (b,b), 9 active, 10 breakdown,
+//   11 iterations, 12 the next rho
 constexpr int kMomScal = 16;
-__device__ __forceinline__ bool mom_active(const double* scal, int j) { return scal[kMomScal * j + 9] != 0.0; }
-
-template <int NR>
-__device__ __forceinline__ void sell_mv(const SellView<double>& A, int row, const double* __restrict__ x, size_t N,
-                                       double* y) {
-#pragma unroll
-    for (int j = 0; j < NR; ++j) y[j] = 0.0;
-    const int sl = row >> 5, l = row & 31;
-    const int b = A.sptr[sl], w = (A.sptr[sl + 1] - b) >> 5;
-    if (NR == 1 && w <= 8) {
-        // one right-hand side, short rows (the mesh's): every entry load
-        // first, then the gathers, so a row costs about two memory round
-        // trips instead of one per entry; the products are summed in entry
-        // order as below (0.85 -> 0.73 ms for the volume-fraction solve at
-        // 128^3; with three right-hand sides the batch's registers cost more
-        // than it gains: 1.63 -> 1.67 ms for the momentum solve)
-        int cj[8];
-        double vj[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-            if (q < w) { cj[q] = A.col[b + l + 32 * q]; vj[q] = A.val[b + l + 32 * q]; }
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-            if (q < w) {
-#pragma unroll
-                for (int j = 0; j < NR; ++j) y[j] += vj[q] * __ldg(x + j * N + cj[q]);
-            }
-        return;
-    }
-    for (int e = 0, k = b + l; e < w; ++e, k += 32) {
-        const int c = A.col[k];
-        const double v = A.val[k];
-#pragma unroll
-        for (int j = 0; j < NR; ++j) y[j] += v * __ldg(x + j * N + c);
-    }
+// Grid: at most 152 blocks (one a GB300 multiprocessor; not taken from the
+// device, so that every sum's bits are the same on any GPU), because each block
+// adds up the partial sums of all (12 sums of three systems: 1 us with 152
+// partials, 9 us with four blocks of 256 threads a multiprocessor, at 16 clocks
+// an FP64 warp instruction).  Threads: what deals n out in equal sweeps.
+constexpr int kBiBlocks = 152, kBiThreads = 512, kBiStream = 1024;
+struct BiGrid { int blocks, threads; };
+inline BiGrid bi_grid(int n, int most) {
+    const int64_t sweeps = std::max<int64_t>(1, ((int64_t)n + kBiBlocks * most - 1) / (kBiBlocks * most));
+    const int64_t per = ((int64_t)n + kBiBlocks * sweeps - 1) / (kBiBlocks * sweeps);
+    const int t = (int)std::max<int64_t>(128, (per + 31) / 32 * 32);
+    return BiGrid{(int)std::min<int64_t>(kBiBlocks, ((int64_t)n + t - 1) / t), t};
 }
 
-// x = 0, r = rh = b, p = v = 0;  part = (b,b) per system
+// The off-diagonal entries of B in slices of 32 rows, entry j of row 32 s + l at
+// the slice's start + 32 j + l; padding entries point at the row with value 0.
+// All slices W wide: every entry load, then every gather of a system.
+template <int W>
+struct OffEven {
+    const int* __restrict__ col;
+    const double* __restrict__ val;
+    int n;
+    template <int NR>
+    __device__ __forceinline__ void mv(int row, unsigned act, const double* __restrict__ x, double* y) const {
+        const int k = (row >> 5) * (32 * W) + (row & 31);
+        int cj[W];
+        double vj[W];
+#pragma unroll
+        for (int q = 0; q < W; ++q) { cj[q] = col[k + 32 * q]; vj[q] = val[k + 32 * q]; }
+#pragma unroll
+        for (int j = 0; j < NR; ++j) {
+            if (!(act >> j & 1)) continue;
+            const double* const xs = x + (size_t)j * n;
+            double g[W];
+#pragma unroll
+            for (int q = 0; q < W; ++q) g[q] = __ldg(xs + cj[q]);
+            y[j] = __ldg(xs + row);
+#pragma unroll
+            for (int q = 0; q < W; ++q) y[j] += vj[q] * g[q];
+        }
+    }
+};
+struct OffSell {
+    const int* __restrict__ sptr;
+    const int* __restrict__ col;
+    const double* __restrict__ val;
+    int n;
+    template <int NR>
+    __device__ __forceinline__ void mv(int row, unsigned act, const double* __restrict__ x, double* y) const {
+        const int sl = row >> 5, b = sptr[sl] + (row & 31), w = (sptr[sl + 1] - sptr[sl]) >> 5;
+#pragma unroll
+        for (int j = 0; j < NR; ++j) y[j] = __ldg(x + (size_t)j * n + row);
+        for (int e = 0, k = b; e < w; e += 4, k += 128) {   // four entries in flight
+            int cj[4];
+            double vj[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (e + q < w) { cj[q] = col[k + 32 * q]; vj[q] = val[k + 32 * q]; }
+#pragma unroll
+            for (int j = 0; j < NR; ++j) {
+                if (!(act >> j & 1)) continue;
+                double g[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (e + q < w) g[q] = __ldg(x + (size_t)j * n + cj[q]);
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (e + q < w) y[j] += vj[q] * g[q];
+            }
+        }
+    }
+};
+__global__ void k_off_width(int n, const int* __restrict__ ptr, int* __restrict__ slice_len, int* __restrict__ most) {
+    const int row = blockIdx.x * blockDim.x + threadIdx.x;
+    const int len = (row < n) ? ptr[row + 1] - ptr[row] - 1 : 0;
+    const int w = __reduce_max_sync(0xffffffffu, len);
+    if ((threadIdx.x & 31) == 0 && row < ((n + 31) & ~31)) {
+        slice_len[row >> 5] = 32 * w;
+        if (*most < w) atomicMax(most, w);
+    }
+}
+// B's off-diagonal values (and, into a new layout, columns: scol not null).  width 0: slices as sptr says
+__global__ void k_off_fill(int n, const int* __restrict__ ptr, const int* __restrict__ col,
+                           const int* __restrict__ dig, const double* __restrict__ val,
+                           const double* __restrict__ dinv, const int* __restrict__ sptr, int width,
+                           int* __restrict__ scol, double* __restrict__ sval) {
+    const int row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row >= ((n + 31) & ~31)) return;
+    const int sl = row >> 5, l = row & 31;
+    const int b = width ? 32 * width * sl : sptr[sl], w = width ? width : (sptr[sl + 1] - b) >> 5;
+    const int rb = (row < n) ? ptr[row] : 0, len = (row < n) ? ptr[row + 1] - rb - 1 : 0;
+    const int d = (row < n) ? dig[row] - rb : 0;   // the diagonal's place in the row
+    for (int j = 0; j < w; ++j) {
+        const int k = b + 32 * j + l;
+        int c = min(row, n - 1);
+        double v = 0.0;
+        if (j < len) {
+            const int e = rb + j + (j >= d);
+            c = col[e];
+            v = val[e] * dinv[c];
+        }
+        if (scol) scol[k] = c;
+        sval[k] = v;
+    }
+}
+struct OffDiag {
+    int n = 0, nslices = 0, width = 0;
+    DBuf<int> sptr, col;
+    DBuf<double> val;
+    // run f on the view that suits the layout
+    template <class F>
+    void with(F&& f) const {
+        switch (width) {
+            case 4: f(OffEven<4>{col.p, val.p, n}); break;
+            case 5: f(OffEven<5>{col.p, val.p, n}); break;
+            case 6: f(OffEven<6>{col.p, val.p, n}); break;
+            default: f(OffSell{sptr.p, col.p, val.p, n});
+        }
+    }
+};
+// the layout of a pattern, without values and columns; hpin: two pinned ints.
+// Slices are made equally wide under the rule of build_sell16_struct
+void build_offdiag(cudaStream_t s, const int* ptr, int n, OffDiag& S, int* hpin) {
+    S.n = n;
+    S.nslices = (n + 31) / 32;
+    S.width = 0;
+    S.sptr.alloc(S.nslices + 2, s);   // and the widest slice
+    SEMO_CUDA(cudaMemsetAsync(S.sptr.p + S.nslices, 0, 2 * sizeof(int), s));
+    k_off_width<<<blocks((int64_t)S.nslices * 32, 256), 256, 0, s>>>(n, ptr, S.sptr.p, S.sptr.p + S.nslices + 1);
+    SEMO_CHECK_LAUNCH();
+    SEMO_CUDA(cudaMemcpyAsync(hpin + 1, S.sptr.p + S.nslices + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+    int total = device_scan(s, S.sptr.p, S.nslices + 1, hpin);   // its sync lands hpin[1] too
+    const int64_t even = 32 * (int64_t)hpin[1] * S.nslices;
+    if (hpin[1] >= 4 && hpin[1] <= 6 && even <= (int64_t)total + total / 8 && even < INT_MAX) {
+        S.width = hpin[1];
+        total = (int)even;
+    }
+    S.col.alloc(std::max(total, 1), s);
+    S.val.alloc(std::max(total, 1), s);
+}
+
+__device__ __forceinline__ unsigned bi_active(const double* scal, int nr) {
+    unsigned a = 0;
+    for (int j = 0; j < nr; ++j)
+        a |= (scal[kMomScal * j + 9] != 0.0 && scal[kMomScal * j + 10] == 0.0 ? 1u : 0u) << j;
+    return a;
+}
+// part[k * kBiBlocks + block] = sum over the block of v[k], a warp a sum (sh: K * blockDim.x doubles)
+template <int K>
+__device__ __forceinline__ void bi_put(const double* v, double* sh, double* __restrict__ part) {
+    __syncthreads();   // sh may still be read
+#pragma unroll
+    for (int k = 0; k < K; ++k) sh[k * blockDim.x + threadIdx.x] = v[k];
+    __syncthreads();
+    for (int k = threadIdx.x >> 5; k < K; k += blockDim.x >> 5) {
+        const double* const a = sh + k * blockDim.x + (threadIdx.x & 31);
+        double t = a[0];
+        for (unsigned m = 32; m < blockDim.x; m += 32) t += a[m];
+        t = warp_sum(t);
+        if ((threadIdx.x & 31) == 0) part[k * kBiBlocks + blockIdx.x] = t;
+    }
+}
+// tot[k] = sum of the nb partial sums k, k < K, in shared memory for the whole block
+template <int K>
+__device__ __forceinline__ void bi_get(const double* __restrict__ part, int nb, double* tot) {
+    for (int k = threadIdx.x >> 5; k < K; k += blockDim.x >> 5) {
+        const double t = parts_sum(part + k * kBiBlocks, nb);
+        if ((threadIdx.x & 31) == 0) tot[k] = t;
+    }
+    __syncthreads();
+}
+
+// xh = 0, r = p = b, dinv;  part = (b,b) per system
 template <int NR>
-__global__ void __launch_bounds__(kRedThreads) k_bi_init(int n, const double* __restrict__ b, double* __restrict__ x,
-                                                         double* __restrict__ r, double* __restrict__ rh,
-                                                         double* __restrict__ p, double* __restrict__ v,
-                                                         double* __restrict__ part) {
-    __shared__ double sh[kRedThreads];
+__global__ void __launch_bounds__(kBiStream) k_bi_init(int n, const int* __restrict__ dig,
+                                                       const double* __restrict__ val, const double* __restrict__ b,
+                                                       double* __restrict__ dinv, double* __restrict__ xh,
+                                                       double* __restrict__ r, double* __restrict__ p,
+                                                       double* __restrict__ part) {
+    __shared__ double sh[NR * kBiStream];
     double bb[NR] = {};
     const size_t N = n;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        dinv[i] = 1.0 / val[dig[i]];
+#pragma unroll
         for (int j = 0; j < NR; ++j) {
             const double bi = b[j * N + i];
-            x[j * N + i] = 0.0; r[j * N + i] = bi; rh[j * N + i] = bi; p[j * N + i] = 0.0; v[j * N + i] = 0.0;
+            xh[j * N + i] = 0.0; r[j * N + i] = bi; p[j * N + i] = bi;
             bb[j] += bi * bi;
         }
-    for (int j = 0; j < NR; ++j) {
-        const double t = block_sum(bb[j], sh);
-        if (threadIdx.x == 0) part[j * kRedBlocks + blockIdx.x] = t;
     }
+    bi_put<NR>(bb, sh, part);
 }
 template <int NR>
 __global__ void k_bi_fin0(const double* __restrict__ part, int nb, double* __restrict__ scal, double tol2) {
-    __shared__ double sh[kRedThreads];
-    for (int j = 0; j < NR; ++j) {
-        const double bb = sum_parts(part + j * kRedBlocks, nb, sh);
-        if (threadIdx.x == 0) {
-            double* S = scal + kMomScal * j;
-            for (int k = 0; k < kMomScal; ++k) S[k] = 0.0;
-            S[0] = bb; S[1] = 1.0; S[2] = 1.0; S[3] = 0.0; S[7] = bb; S[8] = bb;
-            S[9] = (bb > 0.0 && !(bb <= tol2 * bb)) ? 1.0 : 0.0;
-        }
+    __shared__ double tot[NR];
+    bi_get<NR>(part, nb, tot);
+    if (threadIdx.x < NR) {
+        const double bb = tot[threadIdx.x];
+        double* S = scal + kMomScal * threadIdx.x;
+        for (int k = 0; k < kMomScal; ++k) S[k] = 0.0;
+        S[0] = bb; S[1] = 1.0; S[2] = 1.0; S[7] = bb; S[8] = bb;
+        S[9] = (bb > 0.0 && !(bb <= tol2 * bb)) ? 1.0 : 0.0;
     }
+    if (threadIdx.x == 0) scal[3 * kMomScal] = 0.0;   // iterations of the loop
 }
-// p = r + beta (p - omega v);  ph = D^-1 p
-template <int NR>
-__global__ void k_bi_p(int n, const double* __restrict__ dinv, const double* __restrict__ r, double* __restrict__ p,
-                       const double* __restrict__ v, double* __restrict__ ph, const double* __restrict__ scal) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const size_t N = n;
-    const double di = dinv[i];
-    for (int j = 0; j < NR; ++j) {
-        if (!mom_active(scal, j)) continue;
-        const double beta = scal[kMomScal * j + 3], omega = scal[kMomScal * j + 2];
-        const double pi = r[j * N + i] + beta * (p[j * N + i] - omega * v[j * N + i]);
-        p[j * N + i] = pi;
-        ph[j * N + i] = di * pi;
-    }
-}
-// y = A x for the three systems;  part = (rh, y) per system
-template <int NR>
-__global__ void __launch_bounds__(kRedThreads) k_bi_mv1(SellView<double> A, const double* __restrict__ x,
-                                                        double* __restrict__ y, const double* __restrict__ rh,
-                                                        const double* __restrict__ scal, double* __restrict__ part) {
-    __shared__ double sh[kRedThreads];
-    const size_t N = A.n;
-    double d[NR] = {};
-    for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n; row += gridDim.x * blockDim.x) {
-        double s[NR];
-        sell_mv<NR>(A, row, x, N, s);
-        for (int j = 0; j < NR; ++j) {
-            if (!mom_active(scal, j)) continue;
-            y[j * N + row] = s[j];
-            d[j] += rh[j * N + row] * s[j];
-        }
-    }
-    for (int j = 0; j < NR; ++j) {
-        const double t = block_sum(d[j], sh);
-        if (threadIdx.x == 0) part[j * kRedBlocks + blockIdx.x] = t;
-    }
-}
-template <int NR>
-__global__ void k_bi_fin1(const double* __restrict__ part, int nb, double* __restrict__ scal) {
-    __shared__ double sh[kRedThreads];
-    for (int j = 0; j < NR; ++j) {
-        const double rv = sum_parts(part + j * kRedBlocks, nb, sh);
-        if (threadIdx.x == 0) {
-            double* S = scal + kMomScal * j;
-            if (S[9] != 0.0) {
-                S[4] = rv;
-                if (rv == 0.0 || !isfinite(rv)) { S[10] = 1.0; S[9] = 0.0; }
-                else S[1] = S[0] / rv;
-            }
-        }
-    }
-}
-// s = r - alpha v (in place in r);  sh = D^-1 s
-template <int NR>
-__global__ void k_bi_s(int n, const double* __restrict__ dinv, double* __restrict__ r, const double* __restrict__ v,
-                       double* __restrict__ shv, const double* __restrict__ scal) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const size_t N = n;
-    const double di = dinv[i];
-    for (int j = 0; j < NR; ++j) {
-        if (!mom_active(scal, j)) continue;
-        const double si = r[j * N + i] - scal[kMomScal * j + 1] * v[j * N + i];
-        r[j * N + i] = si;
-        shv[j * N + i] = di * si;
-    }
-}
-// t = A sh;  part = (t,s), (t,t) per system
-template <int NR>
-__global__ void __launch_bounds__(kRedThreads) k_bi_mv2(SellView<double> A, const double* __restrict__ x,
-                                                        double* __restrict__ t, const double* __restrict__ s,
-                                                        const double* __restrict__ scal, double* __restrict__ part) {
-    __shared__ double sh[kRedThreads];
-    const size_t N = A.n;
-    double ts[NR] = {}, tt[NR] = {};
-    for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n; row += gridDim.x * blockDim.x) {
-        double y[NR];
-        sell_mv<NR>(A, row, x, N, y);
-        for (int j = 0; j < NR; ++j) {
-            if (!mom_active(scal, j)) continue;
-            t[j * N + row] = y[j];
-            ts[j] += y[j] * s[j * N + row];
-            tt[j] += y[j] * y[j];
-        }
-    }
-    for (int j = 0; j < NR; ++j) {
-        const double a = block_sum(ts[j], sh);
-        const double b = block_sum(tt[j], sh);
-        if (threadIdx.x == 0) { part[(2 * j) * kRedBlocks + blockIdx.x] = a; part[(2 * j + 1) * kRedBlocks + blockIdx.x] = b; }
-    }
-}
-template <int NR>
-__global__ void k_bi_fin2(const double* __restrict__ part, int nb, double* __restrict__ scal) {
-    __shared__ double sh[kRedThreads];
-    for (int j = 0; j < NR; ++j) {
-        const double ts = sum_parts(part + (2 * j) * kRedBlocks, nb, sh);
-        const double tt = sum_parts(part + (2 * j + 1) * kRedBlocks, nb, sh);
-        if (threadIdx.x == 0) {
-            double* S = scal + kMomScal * j;
-            if (S[9] != 0.0) { S[5] = ts; S[6] = tt; S[2] = (tt > 0.0) ? ts / tt : 0.0; }
-        }
-    }
-}
-// x += alpha ph + omega sh;  r = s - omega t;  part = (rh,r), (r,r)
-template <int NR>
-__global__ void __launch_bounds__(kRedThreads) k_bi_xr(int n, double* __restrict__ x, const double* __restrict__ ph,
-                                                       const double* __restrict__ shv, double* __restrict__ r,
-                                                       const double* __restrict__ t, const double* __restrict__ rh,
+// v = B p;  part = (rh,v) per system
+template <int NR, class M>
+__global__ void __launch_bounds__(kBiThreads) k_bi_mv1(M B, const double* __restrict__ p, double* __restrict__ v,
+                                                       const double* __restrict__ rh,
                                                        const double* __restrict__ scal, double* __restrict__ part) {
-    __shared__ double sh[kRedThreads];
-    const size_t N = n;
-    double a[NR] = {}, b[NR] = {};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        for (int j = 0; j < NR; ++j) {
-            if (!mom_active(scal, j)) continue;
-            const double alpha = scal[kMomScal * j + 1], omega = scal[kMomScal * j + 2];
-            x[j * N + i] += alpha * ph[j * N + i] + omega * shv[j * N + i];
-            const double ri = r[j * N + i] - omega * t[j * N + i];
-            r[j * N + i] = ri;
-            a[j] += rh[j * N + i] * ri;
-            b[j] += ri * ri;
-        }
-    for (int j = 0; j < NR; ++j) {
-        const double u = block_sum(a[j], sh);
-        const double w = block_sum(b[j], sh);
-        if (threadIdx.x == 0) { part[(2 * j) * kRedBlocks + blockIdx.x] = u; part[(2 * j + 1) * kRedBlocks + blockIdx.x] = w; }
-    }
-}
-template <int NR>
-__global__ void k_bi_fin3(const double* __restrict__ part, int nb, double* __restrict__ scal, double tol2) {
-    __shared__ double sh[kRedThreads];
-    for (int j = 0; j < NR; ++j) {
-        const double rho1 = sum_parts(part + (2 * j) * kRedBlocks, nb, sh);
-        const double rr = sum_parts(part + (2 * j + 1) * kRedBlocks, nb, sh);
-        if (threadIdx.x == 0) {
-            double* S = scal + kMomScal * j;
-            if (S[9] != 0.0) {
-                S[11] += 1.0;                                        // iterations of this system
-                S[7] = rr;
-                if (rr <= tol2 * S[8]) {
-                    S[9] = 0.0;                                     // converged
-                } else if (rho1 == 0.0 || S[2] == 0.0 || !isfinite(rr)) {
-                    S[10] = 1.0; S[9] = 0.0;                        // breakdown
-                } else {
-                    S[3] = (rho1 / S[0]) * (S[1] / S[2]);
-                    S[0] = rho1;
-                }
-            }
-        }
-    }
-}
-// r = b - A x;  part = (r,r) per system
-template <int NR>
-__global__ void __launch_bounds__(kRedThreads) k_bi_res(SellView<double> A, const double* __restrict__ x,
-                                                        const double* __restrict__ b, double* __restrict__ part) {
-    __shared__ double sh[kRedThreads];
-    const size_t N = A.n;
+    pdl_enter();
+    __shared__ double sh[NR * kBiThreads];
+    const size_t N = B.n;
+    const unsigned act = bi_active(scal, NR);
     double d[NR] = {};
-    for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n; row += gridDim.x * blockDim.x) {
+    for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < B.n; row += gridDim.x * blockDim.x) {
         double y[NR];
-        sell_mv<NR>(A, row, x, N, y);
-        for (int j = 0; j < NR; ++j) { const double ri = b[j * N + row] - y[j]; d[j] += ri * ri; }
+        B.template mv<NR>(row, act, p, y);
+#pragma unroll
+        for (int j = 0; j < NR; ++j) {
+            if (!(act >> j & 1)) continue;
+            v[j * N + row] = y[j];
+            d[j] += rh[j * N + row] * y[j];
+        }
     }
+    bi_put<NR>(d, sh, part);
+}
+// alpha = rho / (rh,v);  s = r - alpha v (in place in r)
+template <int NR>
+__global__ void __launch_bounds__(kBiStream) k_bi_s(int n, double* __restrict__ r, const double* __restrict__ v,
+                                                    double* __restrict__ scal, const double* __restrict__ part,
+                                                    int nb) {
+    pdl_enter();
+    __shared__ double tot[NR];
+    bi_get<NR>(part, nb, tot);
+    const size_t N = n;
+#pragma unroll
     for (int j = 0; j < NR; ++j) {
-        const double t = block_sum(d[j], sh);
-        if (threadIdx.x == 0) part[j * kRedBlocks + blockIdx.x] = t;
+        double* const S = scal + kMomScal * j;
+        const double rv = tot[j];
+        if (S[9] == 0.0) continue;   // no block reads what this kernel writes
+        const bool bad = rv == 0.0 || !isfinite(rv);
+        const double alpha = S[0] / rv;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            if (bad) S[10] = 1.0;
+            else S[1] = alpha;
+        }
+        if (bad) continue;
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+            r[j * N + i] -= alpha * v[j * N + i];
     }
+}
+// t = B s;  part = (t,s), (t,t), (rh,s), (rh,t) per system
+template <int NR, class M>
+__global__ void __launch_bounds__(kBiThreads) k_bi_mv2(M B, const double* __restrict__ s, double* __restrict__ t,
+                                                       const double* __restrict__ rh,
+                                                       const double* __restrict__ scal, double* __restrict__ part) {
+    pdl_enter();
+    __shared__ double sh[4 * kBiThreads];
+    const size_t N = B.n;
+    const unsigned act = bi_active(scal, NR);
+    double d[4 * NR] = {};
+    for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < B.n; row += gridDim.x * blockDim.x) {
+        double y[NR];
+        B.template mv<NR>(row, act, s, y);
+#pragma unroll
+        for (int j = 0; j < NR; ++j) {
+            if (!(act >> j & 1)) continue;
+            const double si = s[j * N + row], ri = rh[j * N + row];
+            t[j * N + row] = y[j];
+            d[4 * j] += y[j] * si;
+            d[4 * j + 1] += y[j] * y[j];
+            d[4 * j + 2] += ri * si;
+            d[4 * j + 3] += ri * y[j];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < NR; ++j) bi_put<4>(d + 4 * j, sh, part + 4 * j * kBiBlocks);
+}
+// omega = (t,s) / (t,t), the next rho and beta = (rho' / rho) (alpha / omega) =
+// alpha ((rh,s) / omega - (rh,t)) / rho;  xh += alpha p + omega s;  r = s - omega t;
+// p = r + beta (p - omega v);  part = (r,r) per system
+template <int NR>
+__global__ void __launch_bounds__(kBiStream) k_bi_xrp(int n, double* __restrict__ xh, double* __restrict__ p,
+                                                      double* __restrict__ r, const double* __restrict__ v,
+                                                      const double* __restrict__ t, double* __restrict__ scal,
+                                                      const double* __restrict__ parts, int nb,
+                                                      double* __restrict__ part) {
+    pdl_enter();
+    __shared__ double sh[NR * kBiStream], tot[4 * NR];
+    bi_get<4 * NR>(parts, nb, tot);
+    const unsigned act = bi_active(scal, NR);
+    const size_t N = n;
+    double rr[NR] = {};
+#pragma unroll
+    for (int j = 0; j < NR; ++j) {
+        if (!(act >> j & 1)) continue;
+        double* const S = scal + kMomScal * j;   // no block reads what this kernel writes
+        const double ts = tot[4 * j], tt = tot[4 * j + 1];
+        const double omega = (tt > 0.0) ? ts / tt : 0.0, alpha = S[1];
+        const double rho = tot[4 * j + 2] - omega * tot[4 * j + 3];
+        const double beta = (rho / S[0]) * (alpha / omega);
+        if (blockIdx.x == 0 && threadIdx.x == 0) { S[2] = omega; S[12] = rho; }
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+            const size_t k = j * N + i;
+            const double pi = p[k], si = r[k], vi = v[k], ti = t[k], xi = xh[k];
+            xh[k] = xi + (alpha * pi + omega * si);
+            const double ri = si - omega * ti;
+            r[k] = ri;
+            p[k] = ri + beta * (pi - omega * vi);
+            rr[j] += ri * ri;
+        }
+    }
+    bi_put<NR>(rr, sh, part);
+}
+// The end of an iteration: each system's state, and whether the loop goes on (a
+// system is active and the cap is not reached; scal[3 * 16] counts iterations)
+template <int NR>
+__global__ void k_bi_check(cudaGraphConditionalHandle h, double* __restrict__ scal, const double* __restrict__ part,
+                           int nb, double tol2, int max_iter) {
+    pdl_enter();
+    __shared__ double tot[NR];
+    bi_get<NR>(part, nb, tot);
+    if (threadIdx.x != 0) return;
+    double* const it = scal + 3 * kMomScal;
+    it[0] += 1.0;
+    bool any = false;
+    for (int j = 0; j < NR; ++j) {
+        double* S = scal + kMomScal * j;
+        if (S[9] == 0.0) continue;
+        if (S[10] != 0.0) { S[9] = 0.0; continue; }             // (rh,v) was 0 or not finite
+        const double rr = tot[j];
+        S[11] += 1.0;                                           // iterations of this system
+        S[7] = rr;
+        if (rr <= tol2 * S[8]) {
+            S[9] = 0.0;                                         // converged
+        } else if (S[12] == 0.0 || S[2] == 0.0 || !isfinite(rr)) {
+            S[10] = 1.0; S[9] = 0.0;                            // breakdown
+        } else {
+            S[0] = S[12];
+            any = true;
+        }
+    }
+    cudaGraphSetConditional(h, (any && it[0] < (double)max_iter) ? 1u : 0u);
+}
+// x = D^-1 xh (0 where no iteration was made);  part = (r,r) of r = b - B xh per system
+template <int NR, class M>
+__global__ void __launch_bounds__(kBiThreads) k_bi_res(M B, const double* __restrict__ xh,
+                                                       const double* __restrict__ dinv, const double* __restrict__ b,
+                                                       const double* __restrict__ scal, double* __restrict__ x,
+                                                       double* __restrict__ part) {
+    __shared__ double sh[NR * kBiThreads];
+    const size_t N = B.n;
+    double d[NR] = {};
+    for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < B.n; row += gridDim.x * blockDim.x) {
+        double y[NR];
+        B.template mv<NR>(row, (1u << NR) - 1, xh, y);
+        const double di = dinv[row];
+#pragma unroll
+        for (int j = 0; j < NR; ++j) {
+            const double ri = b[j * N + row] - y[j];
+            d[j] += ri * ri;
+            x[j * N + row] = scal[kMomScal * j + 11] == 0.0 ? 0.0 : di * __ldg(xh + j * N + row);
+        }
+    }
+    bi_put<NR>(d, sh, part);
 }
 template <int NR>
 __global__ void k_bi_fin_res(const double* __restrict__ part, int nb, double* __restrict__ out) {
-    __shared__ double sh[kRedThreads];
-    for (int j = 0; j < NR; ++j) {
-        const double rr = sum_parts(part + j * kRedBlocks, nb, sh);
-        if (threadIdx.x == 0) out[j] = rr;
-    }
-}
-__global__ void k_dinv_dig(int n, const int* __restrict__ dig, const double* __restrict__ val,
-                           double* __restrict__ dinv) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dinv[i] = 1.0 / val[dig[i]];
+    __shared__ double tot[NR];
+    bi_get<NR>(part, nb, tot);
+    if (threadIdx.x < NR) out[threadIdx.x] = tot[threadIdx.x];
 }
 
 // The instantiated iteration graph of a batched BiCGStab, kept while every
@@ -1757,11 +1889,11 @@ __global__ void k_dinv_dig(int n, const int* __restrict__ dig, const double* __r
 // are reused from call to call, so the momentum and volume-fraction solves of
 // successive outer iterations launch it without capturing it again).
 struct BiGraphKey {
-    int nr = 0, n = 0, max_iter = 0;
+    int nr = 0, n = 0, max_iter = 0, width = 0;
     double tol2 = 0.0;
     const void* ptrs[8] = {};
     bool operator==(const BiGraphKey& o) const {
-        if (nr != o.nr || n != o.n || max_iter != o.max_iter || tol2 != o.tol2) return false;
+        if (nr != o.nr || n != o.n || max_iter != o.max_iter || width != o.width || tol2 != o.tol2) return false;
         for (int k = 0; k < 8; ++k)
             if (ptrs[k] != o.ptrs[k]) return false;
         return true;
@@ -1784,22 +1916,12 @@ struct BiGraph {
     ~BiGraph() { reset(); }
 };
 struct MomState {
-    Sell<double> A;
-    int gen = -1;                 // mesh generation the SELL layout was built for
+    OffDiag B;
+    int gen = -1;                 // mesh generation the layout was built for
     DBuf<double> dinv, vec, part, scal;
     BiGraph graph[2];             // NR = 1, NR = 3
 };
 
-// end of one batched BiCGStab iteration on the device: go on while a system
-// is active and the cap is not reached (scal[3*16+0] counts iterations)
-template <int NR>
-__global__ void k_bi_check(cudaGraphConditionalHandle h, double* __restrict__ scal, int max_iter) {
-    double* it = scal + 3 * kMomScal;
-    it[0] += 1.0;
-    bool any = false;
-    for (int j = 0; j < NR; ++j) any |= scal[kMomScal * j + 9] != 0.0;
-    cudaGraphSetConditional(h, (any && it[0] < (double)max_iter) ? 1u : 0u);
-}
 MomState& mom_state(semo_ctx* c) {
     if (!c->mom_apply) c->mom_apply = std::shared_ptr<void>(new MomState(), [](void* p) { delete (MomState*)p; });
     return *(MomState*)c->mom_apply.get();
@@ -1933,41 +2055,39 @@ semo_status bicgstab_jacobi(semo_ctx* c, int stage, const KrylovPattern& pat, co
     cudaStream_t s = c->stream;
     const int n = pat.n;
     const size_t N = n;
-    const int nb = red_blocks(n);
+    const BiGrid gm = bi_grid(n, kBiThreads), gs = bi_grid(n, kBiStream);
     MomState& st = mom_state(c);
     st.dinv.alloc(N, s);
-    st.vec.alloc(7 * 3 * N, s);       // r, rh, p, v, ph, sh, t (room for 3 systems)
-    st.part.alloc(6 * kRedBlocks, s);
+    st.vec.alloc(5 * 3 * N, s);       // r, p, v, t, xh (room for 3 systems)
+    st.part.alloc((size_t)(12 + 3) * kBiBlocks, s);
     st.scal.alloc(4 * kMomScal, s);
     double* r = st.vec.p;
-    double* rh = r + NR * N;
-    double* p = rh + NR * N;
+    double* p = r + NR * N;
     double* v = p + NR * N;
-    double* ph = v + NR * N;
-    double* shv = ph + NR * N;
-    double* t = shv + NR * N;
+    double* t = v + NR * N;
+    double* xh = t + NR * N;
+    double* const prr = st.part.p + 12 * kBiBlocks;
     // the recurrence residual is driven to half the tolerance so that the true
     // residual, checked at the end, lands under it
     const double tol2 = 0.25 * c->prm.mom_tol * c->prm.mom_tol;
     SEMO_CUDA(cudaEventRecord(c->ev[0], s));
-    if (pat.gen < 0 || st.gen != pat.gen) {
-        build_sell<double, double>(s, pat.ptr, pat.col, val, n, st.A, c->hpin_scan);
-        st.gen = pat.gen;
-    } else {   // same pattern (the mesh's): refill the values into the kept layout
-        k_sell_fill<double, double><<<blocks((int64_t)st.A.nslices * 32, 256), 256, 0, s>>>(
-            n, pat.ptr, pat.col, val, st.A.sptr, st.A.col, st.A.val);
-        SEMO_CHECK_LAUNCH();
+    const bool fresh = pat.gen < 0 || st.gen != pat.gen;   // the mesh's layout is kept
+    if (fresh) {
+        st.gen = -1;
+        build_offdiag(s, pat.ptr, n, st.B, c->hpin_scan);
     }
-    k_dinv_dig<<<blocks(n, 256), 256, 0, s>>>(n, pat.dig, val, st.dinv);
+    k_bi_init<NR><<<gs.blocks, gs.threads, 0, s>>>(n, pat.dig, val, b, st.dinv, xh, r, p, st.part);
     SEMO_CHECK_LAUNCH();
+    k_off_fill<<<blocks((int64_t)st.B.nslices * 32, 256), 256, 0, s>>>(n, pat.ptr, pat.col, pat.dig, val, st.dinv,
+                                                                       st.B.sptr, st.B.width,
+                                                                       fresh ? st.B.col.p : nullptr, st.B.val);
+    SEMO_CHECK_LAUNCH();
+    st.gen = pat.gen;
     SEMO_CUDA(cudaEventRecord(c->ev[1], s));
-    const SellView<double> A = st.A.view();
-    k_bi_init<NR><<<nb, kRedThreads, 0, s>>>(n, b, x, r, rh, p, v, st.part);
-    SEMO_CHECK_LAUNCH();
-    k_bi_fin0<NR><<<1, 256, 0, s>>>(st.part, nb, st.scal, tol2);
+    k_bi_fin0<NR><<<1, 32 * NR, 0, s>>>(st.part, gs.blocks, st.scal, tol2);
     SEMO_CHECK_LAUNCH();
     // The iterations run as one graph: a conditional WHILE node around one
-    // iteration (8 kernels + k_bi_check), launched without a host round trip
+    // iteration (4 kernels and k_bi_check), launched without a host round trip
     // first: systems whose right-hand side is zero, already converged or not
     // finite start inactive (k_bi_fin0), every kernel skips them, and the
     // host reads the outcome once, after the true residuals.
@@ -1977,7 +2097,8 @@ semo_status bicgstab_jacobi(semo_ctx* c, int stage, const KrylovPattern& pat, co
     key.n = n;
     key.max_iter = c->prm.mom_max_iter;
     key.tol2 = tol2;
-    const void* kp[8] = {A.sptr, A.col, A.val, st.dinv.p, st.vec.p, st.part.p, st.scal.p, x};
+    key.width = st.B.width;
+    const void* kp[8] = {st.B.sptr.p, st.B.col.p, st.B.val.p, st.vec.p, st.part.p, st.scal.p, b, nullptr};
     std::copy(kp, kp + 8, key.ptrs);
     if (!G.e || !(G.key == key)) {
         G.reset();
@@ -1995,24 +2116,17 @@ semo_status bicgstab_jacobi(semo_ctx* c, int stage, const KrylovPattern& pat, co
         const long long before = __atomic_load_n(&g_kernel_launches, __ATOMIC_RELAXED);
         SEMO_CUDA(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
         try {
-            k_bi_p<NR><<<blocks(n, 256), 256, 0, s>>>(n, st.dinv, r, p, v, ph, st.scal);
-            SEMO_CHECK_LAUNCH();
-            k_bi_mv1<NR><<<nb, kRedThreads, 0, s>>>(A, ph, v, rh, st.scal, st.part);
-            SEMO_CHECK_LAUNCH();
-            k_bi_fin1<NR><<<1, 256, 0, s>>>(st.part, nb, st.scal);
-            SEMO_CHECK_LAUNCH();
-            k_bi_s<NR><<<blocks(n, 256), 256, 0, s>>>(n, st.dinv, r, v, shv, st.scal);
-            SEMO_CHECK_LAUNCH();
-            k_bi_mv2<NR><<<nb, kRedThreads, 0, s>>>(A, shv, t, r, st.scal, st.part);
-            SEMO_CHECK_LAUNCH();
-            k_bi_fin2<NR><<<1, 256, 0, s>>>(st.part, nb, st.scal);
-            SEMO_CHECK_LAUNCH();
-            k_bi_xr<NR><<<nb, kRedThreads, 0, s>>>(n, x, ph, shv, r, t, rh, st.scal, st.part);
-            SEMO_CHECK_LAUNCH();
-            k_bi_fin3<NR><<<1, 256, 0, s>>>(st.part, nb, st.scal, tol2);
-            SEMO_CHECK_LAUNCH();
-            k_bi_check<NR><<<1, 1, 0, s>>>(handle, st.scal, c->prm.mom_max_iter);
-            SEMO_CHECK_LAUNCH();
+            st.B.with([&](auto B) {
+                launch_pdl(k_bi_mv1<NR, decltype(B)>, gm.blocks, gm.threads, s, B, p, v, b, st.scal.p, st.part.p);
+            });
+            launch_pdl(k_bi_s<NR>, gs.blocks, gs.threads, s, n, r, v, st.scal.p, st.part.p, gm.blocks);
+            st.B.with([&](auto B) {
+                launch_pdl(k_bi_mv2<NR, decltype(B)>, gm.blocks, gm.threads, s, B, r, t, b, st.scal.p, st.part.p);
+            });
+            launch_pdl(k_bi_xrp<NR>, gs.blocks, gs.threads, s, n, xh, p, r, v, t, st.scal.p, st.part.p, gm.blocks,
+                       prr);
+            launch_pdl(k_bi_check<NR>, 1, 32 * NR, s, handle, st.scal.p, prr, gs.blocks, tol2,
+                       c->prm.mom_max_iter);
         } catch (...) {
             cudaGraph_t junk = nullptr;
             cudaStreamEndCapture(s, &junk);
@@ -2025,23 +2139,22 @@ semo_status bicgstab_jacobi(semo_ctx* c, int stage, const KrylovPattern& pat, co
         SEMO_CUDA(cudaGraphInstantiate(&G.e, G.g, 0));
         G.key = key;
     }
-    SEMO_CUDA(cudaMemsetAsync(st.scal.p + 3 * kMomScal, 0, sizeof(double) * kMomScal, s));
     SEMO_CUDA(cudaGraphLaunch(G.e, s));
-    // true FP64 residuals of the returned solutions
-    k_bi_res<NR><<<nb, kRedThreads, 0, s>>>(A, x, b, st.part);
+    // the solutions, and their true FP64 residuals (in scal's last places of the third system)
+    st.B.with([&](auto B) {
+        k_bi_res<NR, decltype(B)><<<gm.blocks, gm.threads, 0, s>>>(B, xh, st.dinv, b, st.scal, x, st.part);
+        SEMO_CHECK_LAUNCH();
+    });
+    k_bi_fin_res<NR><<<1, 32 * NR, 0, s>>>(st.part, gm.blocks, st.scal.p + 3 * kMomScal - 3);
     SEMO_CHECK_LAUNCH();
-    k_bi_fin_res<NR><<<1, 256, 0, s>>>(st.part, nb, st.scal.p + 3 * kMomScal - 3);
-    SEMO_CHECK_LAUNCH();
-    // pinned: the systems' scalars and the iteration count hpin[0, 64), the
-    // true residuals hpin[64, 64 + NR)
+    // pinned: the systems' scalars, the residuals and the iteration count
     double* const hs = c->hpin;
-    double* const tr = c->hpin + 4 * kMomScal;
+    double* const tr = hs + 3 * kMomScal - 3;
     SEMO_CUDA(cudaMemcpyAsync(hs, st.scal.p, sizeof(double) * 4 * kMomScal, cudaMemcpyDeviceToHost, s));
-    SEMO_CUDA(cudaMemcpyAsync(tr, st.scal.p + 3 * kMomScal - 3, sizeof(double) * NR, cudaMemcpyDeviceToHost, s));
     SEMO_CUDA(cudaEventRecord(c->ev[2], s));
     SEMO_CUDA(cudaEventSynchronize(c->ev[2]));
     const int it = (int)hs[3 * kMomScal];
-    __atomic_add_fetch(&g_kernel_launches, 9LL * it, __ATOMIC_RELAXED);
+    __atomic_add_fetch(&g_kernel_launches, 5LL * it, __ATOMIC_RELAXED);
     int iters[NR] = {};
     for (int j = 0; j < NR; ++j) {
         if (!std::isfinite(hs[kMomScal * j + 8])) throw Error(SEMO_ERR_NAN, "non-finite right-hand side");
