@@ -1651,9 +1651,10 @@ void build_offdiag(cudaStream_t s, const int* ptr, int n, OffDiag& S, int* hpin)
 }
 
 __device__ __forceinline__ unsigned bi_active(const double* scal, int nr) {
+    // 0.0 or 1.0, told apart by the high word: a comparison is an FP64 instruction of every thread
     unsigned a = 0;
     for (int j = 0; j < nr; ++j)
-        a |= (scal[kMomScal * j + 9] != 0.0 && scal[kMomScal * j + 10] == 0.0 ? 1u : 0u) << j;
+        a |= (__double2hiint(scal[kMomScal * j + 9]) != 0 && __double2hiint(scal[kMomScal * j + 10]) == 0 ? 1u : 0u) << j;
     return a;
 }
 // part[k * kBiBlocks + block] = sum over the block of v[k], a warp a sum (sh: K * blockDim.x doubles)
@@ -1737,27 +1738,34 @@ __global__ void __launch_bounds__(kBiThreads) k_bi_mv1(M B, const double* __rest
     }
     bi_put<NR>(d, sh, part);
 }
-// alpha = rho / (rh,v);  s = r - alpha v (in place in r)
+// alpha = rho / (rh,v);  s = r - alpha v (in place in r).  One thread a system
+// forms the scalars here and in k_bi_xrp: three divisions in every thread took
+// 5 and 25 us
 template <int NR>
 __global__ void __launch_bounds__(kBiStream) k_bi_s(int n, double* __restrict__ r, const double* __restrict__ v,
                                                     double* __restrict__ scal, const double* __restrict__ part,
                                                     int nb) {
     pdl_enter();
-    __shared__ double tot[NR];
+    __shared__ double tot[NR], sal[NR];
+    __shared__ int go[NR];
     bi_get<NR>(part, nb, tot);
-    const size_t N = n;
-#pragma unroll
-    for (int j = 0; j < NR; ++j) {
-        double* const S = scal + kMomScal * j;
-        const double rv = tot[j];
-        if (S[9] == 0.0) continue;   // no block reads what this kernel writes
-        const bool bad = rv == 0.0 || !isfinite(rv);
-        const double alpha = S[0] / rv;
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (threadIdx.x < NR) {
+        double* const S = scal + kMomScal * threadIdx.x;   // no block reads what this kernel writes
+        const double rv = tot[threadIdx.x], alpha = S[0] / rv;
+        const bool act = S[9] != 0.0, bad = rv == 0.0 || !isfinite(rv);
+        go[threadIdx.x] = act && !bad;
+        sal[threadIdx.x] = alpha;
+        if (blockIdx.x == 0 && act) {
             if (bad) S[10] = 1.0;
             else S[1] = alpha;
         }
-        if (bad) continue;
+    }
+    __syncthreads();
+    const size_t N = n;
+#pragma unroll
+    for (int j = 0; j < NR; ++j) {
+        if (!go[j]) continue;
+        const double alpha = sal[j];
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
             r[j * N + i] -= alpha * v[j * N + i];
     }
@@ -1789,8 +1797,7 @@ __global__ void __launch_bounds__(kBiThreads) k_bi_mv2(M B, const double* __rest
 #pragma unroll
     for (int j = 0; j < NR; ++j) bi_put<4>(d + 4 * j, sh, part + 4 * j * kBiBlocks);
 }
-// omega = (t,s) / (t,t), the next rho and beta = (rho' / rho) (alpha / omega) =
-// alpha ((rh,s) / omega - (rh,t)) / rho;  xh += alpha p + omega s;  r = s - omega t;
+// omega = (t,s) / (t,t), the next rho and beta = (rho' / rho) (alpha / omega);  xh += alpha p + omega s;  r = s - omega t;
 // p = r + beta (p - omega v);  part = (r,r) per system
 template <int NR>
 __global__ void __launch_bounds__(kBiStream) k_bi_xrp(int n, double* __restrict__ xh, double* __restrict__ p,
@@ -1799,20 +1806,26 @@ __global__ void __launch_bounds__(kBiStream) k_bi_xrp(int n, double* __restrict_
                                                       const double* __restrict__ parts, int nb,
                                                       double* __restrict__ part) {
     pdl_enter();
-    __shared__ double sh[NR * kBiStream], tot[4 * NR];
+    __shared__ double sh[NR * kBiStream], tot[4 * NR], sal[NR], som[NR], sbe[NR];
     bi_get<4 * NR>(parts, nb, tot);
+    if (threadIdx.x < NR) {
+        const int j = threadIdx.x;
+        double* const S = scal + kMomScal * j;   // no block reads what this kernel writes
+        const double tt = tot[4 * j + 1], omega = (tt > 0.0) ? tot[4 * j] / tt : 0.0, alpha = S[1];
+        const double rho = tot[4 * j + 2] - omega * tot[4 * j + 3];
+        sal[j] = alpha;
+        som[j] = omega;
+        sbe[j] = (rho / S[0]) * (alpha / omega);
+        if (blockIdx.x == 0 && S[9] != 0.0 && S[10] == 0.0) { S[2] = omega; S[12] = rho; }
+    }
+    __syncthreads();
     const unsigned act = bi_active(scal, NR);
     const size_t N = n;
     double rr[NR] = {};
 #pragma unroll
     for (int j = 0; j < NR; ++j) {
         if (!(act >> j & 1)) continue;
-        double* const S = scal + kMomScal * j;   // no block reads what this kernel writes
-        const double ts = tot[4 * j], tt = tot[4 * j + 1];
-        const double omega = (tt > 0.0) ? ts / tt : 0.0, alpha = S[1];
-        const double rho = tot[4 * j + 2] - omega * tot[4 * j + 3];
-        const double beta = (rho / S[0]) * (alpha / omega);
-        if (blockIdx.x == 0 && threadIdx.x == 0) { S[2] = omega; S[12] = rho; }
+        const double alpha = sal[j], omega = som[j], beta = sbe[j];
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
             const size_t k = j * N + i;
             const double pi = p[k], si = r[k], vi = v[k], ti = t[k], xi = xh[k];
@@ -1833,27 +1846,33 @@ __global__ void k_bi_check(cudaGraphConditionalHandle h, double* __restrict__ sc
     pdl_enter();
     __shared__ double tot[NR];
     bi_get<NR>(part, nb, tot);
-    if (threadIdx.x != 0) return;
-    double* const it = scal + 3 * kMomScal;
-    it[0] += 1.0;
     bool any = false;
-    for (int j = 0; j < NR; ++j) {
-        double* S = scal + kMomScal * j;
-        if (S[9] == 0.0) continue;
-        if (S[10] != 0.0) { S[9] = 0.0; continue; }             // (rh,v) was 0 or not finite
-        const double rr = tot[j];
-        S[11] += 1.0;                                           // iterations of this system
-        S[7] = rr;
-        if (rr <= tol2 * S[8]) {
-            S[9] = 0.0;                                         // converged
-        } else if (S[12] == 0.0 || S[2] == 0.0 || !isfinite(rr)) {
-            S[10] = 1.0; S[9] = 0.0;                            // breakdown
+    if (threadIdx.x < NR) {
+        double* S = scal + kMomScal * threadIdx.x;
+        const double rr = tot[threadIdx.x];
+        if (S[9] == 0.0) {
+        } else if (S[10] != 0.0) {
+            S[9] = 0.0;                                         // (rh,v) was 0 or not finite
         } else {
-            S[0] = S[12];
-            any = true;
+            S[11] += 1.0;                                       // iterations of this system
+            S[7] = rr;
+            if (rr <= tol2 * S[8]) {
+                S[9] = 0.0;                                     // converged
+            } else if (S[12] == 0.0 || S[2] == 0.0 || !isfinite(rr)) {
+                S[10] = 1.0; S[9] = 0.0;                        // breakdown
+            } else {
+                S[0] = S[12];
+                any = true;
+            }
         }
     }
-    cudaGraphSetConditional(h, (any && it[0] < (double)max_iter) ? 1u : 0u);
+    any = __syncthreads_or(any);
+    if (threadIdx.x == 0) {
+        double* const it = scal + 3 * kMomScal;
+        const double done = it[0] + 1.0;
+        it[0] = done;
+        cudaGraphSetConditional(h, (any && done < (double)max_iter) ? 1u : 0u);
+    }
 }
 // x = D^-1 xh (0 where no iteration was made);  part = (r,r) of r = b - B xh per system
 template <int NR, class M>
@@ -1872,7 +1891,7 @@ __global__ void __launch_bounds__(kBiThreads) k_bi_res(M B, const double* __rest
         for (int j = 0; j < NR; ++j) {
             const double ri = b[j * N + row] - y[j];
             d[j] += ri * ri;
-            x[j * N + row] = scal[kMomScal * j + 11] == 0.0 ? 0.0 : di * __ldg(xh + j * N + row);
+            x[j * N + row] = __double2hiint(scal[kMomScal * j + 11]) == 0 ? 0.0 : di * __ldg(xh + j * N + row);
         }
     }
     bi_put<NR>(d, sh, part);
