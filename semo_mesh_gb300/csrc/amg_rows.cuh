@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <cstring>
 
 namespace semo {
 namespace amg {
@@ -48,6 +49,47 @@ __device__ __forceinline__ long long fixed_product(float a, float b, int sc) {
         if (rem > half || (rem == half && (q & 1ull))) ++q;
     }
     return ((ua ^ ub) >> 31) ? -(long long)q : (long long)q;
+}
+
+// the same for doubles: the 53-bit significands multiply exactly into 106 bits,
+// so the product is rounded once, where (a b) 2^sc in FP64 rounds twice and
+// takes three instructions of the FP64 unit, 16 clocks a warp each
+__host__ __device__ __forceinline__ long long fixed_product(double a, double b, int sc) {
+#ifdef __CUDA_ARCH__
+    const uint64_t ua = (uint64_t)__double_as_longlong(a), ub = (uint64_t)__double_as_longlong(b);
+#else
+    uint64_t ua, ub;
+    memcpy(&ua, &a, 8);
+    memcpy(&ub, &b, 8);
+#endif
+    int ea = (int)(ua >> 52) & 0x7ff, eb = (int)(ub >> 52) & 0x7ff;
+    const uint64_t ma = (ua & 0xfffffffffffffull) | (ea ? 0x10000000000000ull : 0ull);
+    const uint64_t mb = (ub & 0xfffffffffffffull) | (eb ? 0x10000000000000ull : 0ull);
+    ea = ea ? ea : 1;
+    eb = eb ? eb : 1;
+    const unsigned __int128 m = (unsigned __int128)ma * mb;
+    const uint64_t hi = (uint64_t)(m >> 64), lo = (uint64_t)m;
+    const int sh = 2150 - ea - eb - sc;   // |a b| 2^sc = m 2^-sh
+    uint64_t q, rem, half;
+    if (sh <= 0) {   // m < 2^62 then, by the scale's bound
+        q = sh > -64 ? lo << -sh : 0ull;
+        rem = 0ull;
+        half = 1ull;
+    } else if (sh < 64) {
+        q = (hi << (64 - sh)) | (lo >> sh);
+        rem = lo << (64 - sh);   // the bits below the unit, at the top of a word
+        half = 1ull << 63;
+    } else if (sh < 128) {
+        const int s = sh - 64;
+        q = s ? hi >> s : hi;
+        rem = s ? (hi << (64 - s)) | (lo >> s) | (lo << (64 - s) ? 1ull : 0ull) : lo;
+        half = 1ull << 63;
+    } else {
+        q = rem = 0ull;   // below half a unit (m < 2^106)
+        half = 1ull;
+    }
+    if (rem > half || (rem == half && (q & 1ull))) ++q;
+    return ((ua ^ ub) >> 63) ? -(long long)q : (long long)q;
 }
 
 // A magnitude in FP32 with an exponent of its own: at most m 2^e.  The products'
@@ -161,7 +203,6 @@ __device__ int hash_row(int lane, int ht, RowTable tb, int ab, int ae, const int
     Mag bound{0.0f, kMagNone};
     for (int ka = ab + lane; ka < ae; ka += 32) mag_add(bound, mag_mul(mag_of(aval[ka]), bmag[acol[ka]]));
     const int sc = mag_scale(mag_warp_sum(bound));   // the row's scale 2^sc (a fixed tree: deterministic)
-    const double up_scale = __longlong_as_double((long long)(1023 + sc) << 52);   // 2^sc (FP64 values)
     __syncwarp();
     int distinct = 0;
     bool full = false;
@@ -182,9 +223,10 @@ __device__ int hash_row(int lane, int ht, RowTable tb, int ab, int ae, const int
         }
         const int total = __shfl_sync(0xffffffffu, incl, 31);
         const int excl = incl - blen;
-        for (int t0 = 0; t0 < total; t0 += 32) {
-            const int t = t0 + lane;
-            const bool act = t < total;
+        // a step's products are fetched while the one before is summed
+        int c = -1;
+        V av = V(0), bv = V(0);
+        auto fetch = [&](int t) {
             // owner lane: the last lane whose B-row run starts at or before t
             int j = 0;
 #pragma unroll
@@ -193,27 +235,31 @@ __device__ int hash_row(int lane, int ht, RowTable tb, int ab, int ae, const int
                 if (x <= t) j += step;
             }
             const int q = __shfl_sync(0xffffffffu, bb, j) + (t - __shfl_sync(0xffffffffu, excl, j));
-            const V av = __shfl_sync(0xffffffffu, avk, j);
-            const int c = act ? bcol[q] : -1;
+            av = __shfl_sync(0xffffffffu, avk, j);
+            c = t < total ? bcol[q] : -1;
+            if (t < total) bv = bval[q];
+        };
+        fetch(lane);
+        for (int t0 = 0; t0 < total; t0 += 32) {
+            const bool act = c >= 0;
+            const int cc = c;
+            const V a0 = av, b0 = bv;
+            if (t0 + 32 < total) fetch(t0 + 32 + lane);
             int slot = -1;
             bool fresh = false;
             if (act) {
-                uint32_t h = hash_u32((uint32_t)c) & hmask;
+                uint32_t h = hash_u32((uint32_t)cc) & hmask;
                 for (int probe = 0; probe < ht; ++probe) {
-                    const int prev = atomicCAS(tb.keys + h, -1, c);
+                    const int prev = atomicCAS(tb.keys + h, -1, cc);
                     if (prev == -1) { slot = (int)h; fresh = true; break; }
-                    if (prev == c) { slot = (int)h; break; }
+                    if (prev == cc) { slot = (int)h; break; }
                     h = (h + 1) & hmask;
                 }
             }
             distinct += __popc(__ballot_sync(0xffffffffu, fresh));
             const bool lost = __any_sync(0xffffffffu, act && slot < 0);
-            if (!lost && act) {
-                long long fx;
-                if constexpr (sizeof(V) == 4) fx = fixed_product(av, bval[q], sc);
-                else fx = __double2ll_rn((av * bval[q]) * up_scale);
-                shared_add64(tb.vals + slot, (unsigned long long)fx);   // two's complement: signed sum mod 2^64
-            }
+            if (!lost && act)   // two's complement: signed sum mod 2^64
+                shared_add64(tb.vals + slot, (unsigned long long)fixed_product(a0, b0, sc));
             __syncwarp();
             if (lost || distinct > (ht * 3) / 4) { full = true; break; }
         }
@@ -241,6 +287,119 @@ __device__ int hash_row(int lane, int ht, RowTable tb, int ab, int ae, const int
         oval[rank] = fixed_value((long long)tb.cvals[x], sc, V(0));
     }
     return m;
+}
+
+// Four short rows by one warp, 8 lanes and a table of 32 slots each (tb: the
+// group's, with room for 32 slots): row [ab, ae) of the lane's group, ab == ae
+// for none.  The sums are hash_row's.  A row of 26 products leaves a warp's lanes
+// idle in all but one step and costs its latency, ~5 us, alone.  Returns the
+// length, or -1 (nothing written) when more than 24 slots are taken; *size: the
+// sum of |values|.
+constexpr int kGroup = 8, kGroupSlots = 32;
+__device__ __forceinline__ Mag mag_group_sum(Mag s) {
+#pragma unroll
+    for (int o = kGroup / 2; o > 0; o >>= 1) {
+        const float m = __shfl_xor_sync(0xffffffffu, s.m, o);
+        const int e = __shfl_xor_sync(0xffffffffu, s.e, o);
+        const int top = max(e, s.e);   // the same in both lanes
+        s.m = s.m * pow2_down(s.e - top) + m * pow2_down(e - top);
+        s.e = top;
+    }
+    return s;
+}
+template <class V>
+__device__ int hash_rows_short(int lane, RowTable tb, int ab, int ae, const int* acol, const V* aval, RowSpan rb,
+                               const int* bcol, const V* bval, const Mag* bmag, int* ocol, V* oval, Mag* size) {
+    const int sub = lane & (kGroup - 1), first = lane & ~(kGroup - 1);
+    const unsigned group = ((1u << kGroup) - 1u) << first;
+    __syncwarp();
+#pragma unroll
+    for (int t = sub; t < kGroupSlots; t += kGroup) { tb.keys[t] = -1; tb.vals[t] = 0ull; }
+    Mag bound{0.0f, kMagNone};
+    for (int ka = ab + sub; ka < ae; ka += kGroup) mag_add(bound, mag_mul(mag_of(aval[ka]), bmag[acol[ka]]));
+    const int sc = mag_scale(mag_group_sum(bound));
+    __syncwarp();
+    int distinct = 0;
+    bool full = false;
+    for (int k0 = ab; __any_sync(0xffffffffu, k0 < ae && !full); k0 += kGroup) {
+        const int k = k0 + sub;
+        const bool ka = k < ae && !full;
+        const int a = ka ? acol[k] : 0;
+        const V avk = ka ? aval[k] : V(0);
+        const int bb = ka ? rb.begin(a) : 0;
+        const int blen = ka ? rb.count(a) : 0;
+        int incl = blen;
+#pragma unroll
+        for (int o = 1; o < kGroup; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o, kGroup);
+            if (sub >= o) incl += t;
+        }
+        const int total = __shfl_sync(0xffffffffu, incl, kGroup - 1, kGroup);
+        const int excl = incl - blen;
+        int c = -1;
+        V av = V(0), bv = V(0);
+        auto fetch = [&](int t) {
+            int j = 0;
+#pragma unroll
+            for (int step = kGroup / 2; step >= 1; step >>= 1) {
+                const int x = __shfl_sync(0xffffffffu, excl, j + step, kGroup);
+                if (x <= t) j += step;
+            }
+            const int q = __shfl_sync(0xffffffffu, bb, j, kGroup) + (t - __shfl_sync(0xffffffffu, excl, j, kGroup));
+            av = __shfl_sync(0xffffffffu, avk, j, kGroup);
+            c = t < total ? bcol[q] : -1;
+            if (t < total) bv = bval[q];
+        };
+        fetch(sub);
+        for (int t0 = 0; __any_sync(0xffffffffu, t0 < total && !full); t0 += kGroup) {
+            const bool act = c >= 0 && !full;
+            const int cc = c;
+            const V a0 = av, b0 = bv;
+            fetch(t0 + kGroup + sub);
+            int slot = -1;
+            bool fresh = false;
+            if (act) {
+                uint32_t h = hash_u32((uint32_t)cc) & (kGroupSlots - 1);
+                for (int probe = 0; probe < kGroupSlots; ++probe) {
+                    const int prev = atomicCAS(tb.keys + h, -1, cc);
+                    if (prev == -1) { slot = (int)h; fresh = true; break; }
+                    if (prev == cc) { slot = (int)h; break; }
+                    h = (h + 1) & (kGroupSlots - 1);
+                }
+            }
+            distinct += __popc(__ballot_sync(0xffffffffu, fresh) & group);
+            const bool lost = (__ballot_sync(0xffffffffu, act && slot < 0) & group) != 0;
+            if (act && slot >= 0) shared_add64(tb.vals + slot, (unsigned long long)fixed_product(a0, b0, sc));
+            full |= lost || distinct > (kGroupSlots * 3) / 4;
+        }
+    }
+    __syncwarp();
+    int m = 0;
+#pragma unroll
+    for (int t0 = 0; t0 < kGroupSlots; t0 += kGroup) {
+        const bool occ = tb.keys[t0 + sub] >= 0;
+        const unsigned bal = (__ballot_sync(0xffffffffu, occ) & group) >> first;
+        if (occ) {
+            const int pos = m + __popc(bal & ((1u << sub) - 1u));
+            tb.ckeys[pos] = tb.keys[t0 + sub];
+            tb.cvals[pos] = tb.vals[t0 + sub];
+        }
+        m += __popc(bal);
+    }
+    __syncwarp();
+    Mag sum{0.0f, kMagNone};
+    if (!full)
+        for (int x = sub; x < m; x += kGroup) {
+            const int ce = tb.ckeys[x];
+            int rank = 0;
+            for (int u = 0; u < m; ++u) rank += (tb.ckeys[u] < ce);
+            const V v = fixed_value((long long)tb.cvals[x], sc, V(0));
+            ocol[rank] = ce;
+            oval[rank] = v;
+            mag_add(sum, mag_of(v));
+        }
+    *size = mag_group_sum(sum);
+    return full ? -1 : m;
 }
 
 }  // namespace amg

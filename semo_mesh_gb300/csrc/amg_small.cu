@@ -207,7 +207,6 @@ __device__ int hash_row_block(RowTable tb, Mag* shm, int* cnt2, int ab, int ae, 
     if (threadIdx.x < 2) cnt2[threadIdx.x] = 0;
     __syncthreads();
     const int sc = mag_scale(mag_warp_sum(shm[lane]));   // kWarps == 32: the same tree in every warp
-    const double up_scale = __longlong_as_double((long long)(1023 + sc) << 52);
     for (int k = ab + wid; k < ae; k += kWarps) {
         const int a = acol[k], b0 = rb.begin(a), b1 = b0 + rb.count(a);
         const V av = aval[k];
@@ -218,10 +217,7 @@ __device__ int hash_row_block(RowTable tb, Mag* shm, int* cnt2, int ab, int ae, 
                 const int prev = atomicCAS(tb.keys + h, -1, c);
                 if (prev == -1) atomicAdd(cnt2, 1);
                 if (prev == -1 || prev == c) {
-                    long long fx;
-                    if constexpr (sizeof(V) == 4) fx = fixed_product(av, bval[q], sc);
-                    else fx = __double2ll_rn((av * bval[q]) * up_scale);
-                    shared_add64(tb.vals + h, (unsigned long long)fx);
+                    shared_add64(tb.vals + h, (unsigned long long)fixed_product(av, bval[q], sc));
                     break;
                 }
                 h = (h + 1) & (kBigSlots - 1);
@@ -272,12 +268,17 @@ __device__ void block_product(const SmallArgs<V>& a, int level, int c0, int c1, 
     // a chunk with such a row has no room.
     constexpr int kMostProducts = 1 << 21;
     bool many = false;
-    for (int i = c0 + wid; i < c1; i += kWarps) {
+    // short rows (a mesh's): 8 lanes a row, here and in the sums
+    const bool brief = c1 > c0 && (long long)aptr[c1] - aptr[c0] <= (long long)kGroup * (c1 - c0);
+    const int vs = brief ? kGroup : 32, rpw = 32 / vs, sub = lane & (vs - 1);
+    for (int r0 = c0 + wid * rpw; r0 < c1; r0 += kWarps * rpw) {
+        const int i = r0 + lane / vs;
         long long p = 0;
-        for (int k = aptr[i] + lane; k < aptr[i + 1]; k += 32) p += rb.count(acol[k]);
-        p = group_sum(p, 32);
+        if (i < c1)
+            for (int k = aptr[i] + sub; k < aptr[i + 1]; k += vs) p += rb.count(acol[k]);
+        p = group_sum(p, vs);
         many |= p >= kMostProducts;
-        if (lane == 0) cnt[i] = (int)min(p, (long long)kMostProducts);
+        if (i < c1 && sub == 0) cnt[i] = (int)min(p, (long long)kMostProducts);
     }
     __syncthreads();
     long long chunk = 0;
@@ -308,22 +309,47 @@ __device__ void block_product(const SmallArgs<V>& a, int level, int c0, int c1, 
     tb.cvals = tb.vals + kSlots;
     // rows from which the block does better together: few rows leave most warps idle
     const int alone = c1 - c0 >= kWarps / 4 ? kBlockProducts : 128;
-    for (int i = c0 + wid; i < c1; i += kWarps) {
-        const int s = b0 + start[i], most = cnt[i];
-        __syncwarp();   // every lane has read the row's places before lane 0 writes them
-        const int m = most > alone ? -1
-                                   : hash_row<V>(lane, table_size(most, kSlots), tb, aptr[i], aptr[i + 1], acol, aval,
-                                                 rb, bcol, bval, bmag, a.scol + s, a.sval + s);
-        if (m < 0) {
-            if (lane == 0) later[c0 + atomicAdd(nlater, 1)] = i;
-            continue;
+    RowTable tg = tb;   // the lane's group's part
+    tg.keys += (lane / kGroup) * kGroupSlots;
+    tg.ckeys += (lane / kGroup) * kGroupSlots;
+    tg.vals += (lane / kGroup) * kGroupSlots;
+    tg.cvals += (lane / kGroup) * kGroupSlots;
+    for (int r0 = c0 + wid * rpw; r0 < c1; r0 += kWarps * rpw) {
+        unsigned wide = 1u;   // rows from r0 on that the whole warp sums
+        if (brief) {
+            const int i = r0 + lane / kGroup;
+            const bool mine = i < c1;
+            const int s = mine ? b0 + start[i] : 0, ab = mine ? aptr[i] : 0, ae = mine ? aptr[i + 1] : 0;
+            __syncwarp();   // every lane has read the row's places before they are written
+            Mag t;
+            const int m = hash_rows_short<V>(lane, tg, ab, ae, acol, aval, rb, bcol, bval, bmag, a.scol + s,
+                                             a.sval + s, &t);
+            if (mine && sub == 0 && m >= 0) {
+                start[i] = s;
+                cnt[i] = m;
+                if (size) size[i] = t;
+            }
+            const unsigned failed = __ballot_sync(0xffffffffu, m < 0);
+            wide = (failed & 1u) | (failed >> 8 & 1u) << 1 | (failed >> 16 & 1u) << 2 | (failed >> 24 & 1u) << 3;
         }
-        Mag t{0.0f, kMagNone};
-        if (size) {
-            __syncwarp();
-            t = row_size(a.sval + s, m, lane);
+        for (; wide; wide &= wide - 1) {
+            const int i = r0 + __ffs(wide) - 1;
+            const int s = b0 + start[i], most = cnt[i];
+            __syncwarp();   // every lane has read the row's places before lane 0 writes them
+            const int m = most > alone ? -1
+                                       : hash_row<V>(lane, table_size(most, kSlots), tb, aptr[i], aptr[i + 1], acol,
+                                                     aval, rb, bcol, bval, bmag, a.scol + s, a.sval + s);
+            if (m < 0) {
+                if (lane == 0) later[c0 + atomicAdd(nlater, 1)] = i;
+                continue;
+            }
+            Mag t{0.0f, kMagNone};
+            if (size) {
+                __syncwarp();
+                t = row_size(a.sval + s, m, lane);
+            }
+            if (lane == 0) { start[i] = s; cnt[i] = m; if (size) size[i] = t; }
         }
-        if (lane == 0) { start[i] = s; cnt[i] = m; if (size) size[i] = t; }
     }
     __syncthreads();
     const int todo = *nlater;
