@@ -59,11 +59,19 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     }
     return v;
 }
-// sum of a kernel's nb partial sums, by one warp (every lane gets it)
+// sum of a kernel's nb partial sums, by one warp (every lane gets it); four
+// chains of additions and eight loads in flight: the kernels that begin with it
+// wait for it
 __device__ __forceinline__ double parts_sum(const double* part, int nb) {
-    double s = 0.0;
-    for (int i = threadIdx.x & 31; i < nb; i += 32) s += part[i];
-    return __shfl_sync(0xffffffffu, warp_sum(s), 0);
+    double s[4] = {};
+    for (int i = threadIdx.x & 31; i < nb; i += 256) {
+        double v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = i + 32 * k < nb ? part[i + 32 * k] : 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s[k & 3] += v[k];
+    }
+    return __shfl_sync(0xffffffffu, warp_sum((s[0] + s[1]) + (s[2] + s[3])), 0);
 }
 // blocks of a reducing kernel over n rows
 inline int red_blocks(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>(kRedBlocks, (n + kRedThreads - 1) / kRedThreads)); }
@@ -72,7 +80,7 @@ inline int red_blocks(int64_t n) { return (int)std::max<int64_t>(1, std::min<int
 // CSR with VS lanes per row.
 template <class V, int VS>
 struct CsrView {
-    static constexpr int kVS = VS;
+    static constexpr int kVS = VS, kEven = 0;
     const int* __restrict__ ptr;
     const int* __restrict__ col;
     const V* __restrict__ val;
@@ -94,7 +102,7 @@ struct CsrView {
 // sptr[s] + 32j + l; padding entries point at column 0 with value 0.
 template <class V>
 struct SellView {
-    static constexpr int kVS = 1;
+    static constexpr int kVS = 1, kEven = 0;
     const int* __restrict__ sptr;
     const int* __restrict__ col;
     const V* __restrict__ val;
@@ -239,22 +247,38 @@ struct Sell16UView {
     const unsigned short* __restrict__ dcol;
     const V* __restrict__ val;
     int n;
+    // a row in registers: its entries, then the gathered values
+    template <class F>
+    struct Row {
+        int cj[W];
+        V vj[W];
+        typename F::Raw xj[W];
+    };
+    template <class F>
+    __device__ __forceinline__ void entries(int row, Row<F>& t) const {
+        const int k = (row >> 5) * (32 * W) + (row & 31);
+#pragma unroll
+        for (int q = 0; q < W; ++q) { t.cj[q] = row + (short)dcol[k + 32 * q]; t.vj[q] = val[k + 32 * q]; }
+    }
+    template <class F>
+    __device__ __forceinline__ void gather(Row<F>& t, const F& x) const {
+#pragma unroll
+        for (int q = 0; q < W; ++q) t.xj[q] = x.load(t.cj[q]);
+    }
+    template <class F>
+    __device__ __forceinline__ V sum(const Row<F>& t, const F& x) const {
+        V s = V(0);
+#pragma unroll
+        for (int q = 0; q < W; ++q) s += t.vj[q] * x.value(t.xj[q]);
+        return s;
+    }
     template <class F>
     __device__ __forceinline__ V dot(int row, int, const F& x) const {
-        V s = V(0);
-        if (row < n) {
-            const int k = (row >> 5) * (32 * W) + (row & 31);
-            int cj[W];
-            V vj[W];
-            typename F::Raw xj[W];
-#pragma unroll
-            for (int q = 0; q < W; ++q) { cj[q] = row + (short)dcol[k + 32 * q]; vj[q] = val[k + 32 * q]; }
-#pragma unroll
-            for (int q = 0; q < W; ++q) xj[q] = x.load(cj[q]);
-#pragma unroll
-            for (int q = 0; q < W; ++q) s += vj[q] * x.value(xj[q]);
-        }
-        return s;
+        if (row >= n) return V(0);
+        Row<F> t;
+        entries(row, t);
+        gather(t, x);
+        return sum(t, x);
     }
 };
 
@@ -455,7 +479,7 @@ __global__ void __launch_bounds__(256) k_post1(M A, const V* __restrict__ dinv, 
 // finest-level post-smoothing step 1 (SELL), also folding in the CG dots
 // z.r and z.q (q = A p of the previous iteration); grid-stride, fixed grid
 template <class M, class V>
-__global__ void __launch_bounds__(kRedThreads) k_post1_dots(M A, const V* __restrict__ dinv,
+__global__ void __launch_bounds__(kRedThreads, 4) k_post1_dots(M A, const V* __restrict__ dinv,
                                                             const V* __restrict__ b, V c1, V c2,
                                                             const V* __restrict__ y, const V* __restrict__ d,
                                                             V* __restrict__ z, const double* __restrict__ r,
@@ -464,20 +488,50 @@ __global__ void __launch_bounds__(kRedThreads) k_post1_dots(M A, const V* __rest
     pdl_enter();
     __shared__ double sh[kRedThreads];
     double zr = 0.0, zq = 0.0;
-    const int per_block = blockDim.x / M::kVS, lane = threadIdx.x % M::kVS;
-    for (int row0 = blockIdx.x * per_block; row0 < A.n; row0 += gridDim.x * per_block) {
-        const int row = row0 + threadIdx.x / M::kVS;   // every lane runs the dot's shuffles
-        const bool mine = row < A.n && lane == 0;
-        const V yi = mine ? y[row] : V(0), dv = mine ? d[row] : V(0), di = mine ? dinv[row] : V(0);
-        const V bi = mine ? b[row] : V(0);
-        const double ri = mine ? r[row] : 0.0, qi = mine ? q[row] : 0.0;
-        const V s = A.dot(row, lane, Vec<V, V>{y});
-        if (mine) {
-            const V zi = yi + c1 * dv + c2 * (di * (bi - s));
-            z[row] = zi;
-            const double zd = widen<double>(zi);
-            zr += zd * ri;
-            zq += zd * qi;
+    if constexpr (M::kEven != 0 && sizeof(V) == 4) {
+        // two rows a thread in flight: with one the fixed grid's half-filled
+        // multiprocessors wait for memory
+        const int stride = gridDim.x * blockDim.x;
+        const Vec<V, V> yv{y};
+        for (int row0 = blockIdx.x * blockDim.x + threadIdx.x; row0 < A.n; row0 += 2 * stride) {
+            const int rows[2] = {row0, row0 + stride < A.n ? row0 + stride : row0};
+            typename M::template Row<Vec<V, V>> t[2];
+            V yi[2], dv[2], di[2], bi[2];
+            double ri[2], qi[2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) A.entries(rows[k], t[k]);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                A.gather(t[k], yv);
+                yi[k] = y[rows[k]]; dv[k] = d[rows[k]]; di[k] = dinv[rows[k]]; bi[k] = b[rows[k]];
+                ri[k] = r[rows[k]]; qi[k] = q[rows[k]];
+            }
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                if (k == 1 && rows[1] == row0) break;
+                const V zi = yi[k] + c1 * dv[k] + c2 * (di[k] * (bi[k] - A.sum(t[k], yv)));
+                z[rows[k]] = zi;
+                const double zd = widen<double>(zi);
+                zr += zd * ri[k];
+                zq += zd * qi[k];
+            }
+        }
+    } else {
+        const int per_block = blockDim.x / M::kVS, lane = threadIdx.x % M::kVS;
+        for (int row0 = blockIdx.x * per_block; row0 < A.n; row0 += gridDim.x * per_block) {
+            const int row = row0 + threadIdx.x / M::kVS;   // every lane runs the dot's shuffles
+            const bool mine = row < A.n && lane == 0;
+            const V yi = mine ? y[row] : V(0), dv = mine ? d[row] : V(0), di = mine ? dinv[row] : V(0);
+            const V bi = mine ? b[row] : V(0);
+            const double ri = mine ? r[row] : 0.0, qi = mine ? q[row] : 0.0;
+            const V s = A.dot(row, lane, Vec<V, V>{y});
+            if (mine) {
+                const V zi = yi + c1 * dv + c2 * (di * (bi - s));
+                z[row] = zi;
+                const double zd = widen<double>(zi);
+                zr += zd * ri;
+                zq += zd * qi;
+            }
         }
     }
     zr = block_sum(zr, sh);
@@ -531,6 +585,10 @@ __device__ __forceinline__ double sum_parts(const double* part, int nb, double* 
     for (int i = threadIdx.x; i < nb; i += blockDim.x) s += part[i];
     return block_sum(s, sh);
 }
+template <class M, class F, int kEven = M::kEven>
+struct OuterRow { using type = typename M::template Row<F>; };
+template <class M, class F>
+struct OuterRow<M, F, 0> { struct type {}; };
 // The scalars of an iteration are formed by the kernels that use them, each
 // block adding the producer's partial sums itself (one warp): a kernel of their
 // own for beta, alpha and r.r cost ~2.75 us each.  Block 0 keeps what later
@@ -545,6 +603,25 @@ __global__ void __launch_bounds__(kRedThreads, 4) k_outer_mv(M A, const Z* __res
                                                           double* __restrict__ ppq) {
     pdl_enter();
     __shared__ double sh[kRedThreads], sbeta;
+    const int stride = gridDim.x * blockDim.x;
+    int row = blockIdx.x * blockDim.x + threadIdx.x;
+    const Vec<double, Z> zv{z};
+    // a row's values, on equal slices with its entries; the first row's are under
+    // way while beta is formed
+    double q0 = 0.0, p0 = 0.0;
+    Z zi = Z(0);
+    auto fetch = [&](auto& t) {
+        if (row >= A.n) return;
+        q0 = q[row];
+        p0 = p[row];
+        zi = z[row];
+        if constexpr (M::kEven != 0) {
+            A.entries(row, t);
+            A.gather(t, zv);
+        }
+    };
+    typename OuterRow<M, Vec<double, Z>>::type t;
+    fetch(t);
     if (threadIdx.x < 32) {
         const double rz = parts_sum(part, nb);
         // Polak-Ribiere: beta = z.(r_k - r_{k-1}) / (z_{k-1}.r_{k-1}) = -alpha_{k-1} z.q_{k-1} / rz_prev
@@ -557,16 +634,17 @@ __global__ void __launch_bounds__(kRedThreads, 4) k_outer_mv(M A, const Z* __res
     __syncthreads();
     const double beta = sbeta;
     double pq = 0.0;
-    const int stride = gridDim.x * blockDim.x;
-    for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.n; row += stride) {
-        const double q0 = q[row], p0 = p[row];
-        const Z zi = z[row];
-        const double w = A.dot(row, 0, Vec<double, Z>{z});
+    while (row < A.n) {
+        double w;
+        if constexpr (M::kEven != 0) w = A.sum(t, zv);
+        else w = A.dot(row, 0, zv);
         const double qi = w + beta * q0;
         const double pi = widen<double>(zi) + beta * p0;
         q[row] = qi;
         p[row] = pi;
         pq += pi * qi;
+        row += stride;
+        fetch(t);
     }
     pq = block_sum(pq, sh);
     if (threadIdx.x == 0) ppq[blockIdx.x] = pq;
@@ -581,6 +659,18 @@ __global__ void __launch_bounds__(kRedThreads) k_xr(int n, double* __restrict__ 
                                                     double* __restrict__ part) {
     pdl_enter();
     __shared__ double sh[kRedThreads], salpha;
+    // two rows a thread in flight, the first two while alpha is formed
+    const int stride = gridDim.x * blockDim.x;
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double xv[2], pv[2], rr[2], qv[2];
+    auto fetch = [&] {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int j = i + k * stride;
+            if (j < n) { xv[k] = x[j]; pv[k] = p[j]; rr[k] = r[j]; qv[k] = q[j]; }
+        }
+    };
+    fetch();
     if (threadIdx.x < 32) {
         const double pq = parts_sum(ppq, nb), rz = scal[0];
         if (threadIdx.x == 0) {
@@ -596,12 +686,19 @@ __global__ void __launch_bounds__(kRedThreads) k_xr(int n, double* __restrict__ 
     __syncthreads();
     const double alpha = salpha;
     double s = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        x[i] += alpha * p[i];
-        const double ri = r[i] - alpha * q[i];
-        r[i] = ri;
-        rv[i] = narrow<V>(ri);
-        s += ri * ri;
+    while (i < n) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int j = i + k * stride;
+            if (j >= n) break;
+            x[j] = xv[k] + alpha * pv[k];
+            const double ri = rr[k] - alpha * qv[k];
+            r[j] = ri;
+            rv[j] = narrow<V>(ri);
+            s += ri * ri;
+        }
+        i += 2 * stride;
+        fetch();
     }
     s = block_sum(s, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = s;
