@@ -844,16 +844,19 @@ __global__ void __launch_bounds__(kT, 1) k_small_setup(SmallArgs<V> a) {
 #undef SMALL_SYNC
 }
 
-// Explicit FP64 inverse of the coarsest level (Gauss-Jordan, partial
-// pivoting), matrix and inverse in shared memory, one block.  The pivot is
-// searched by one warp and the arithmetic is k_gauss_jordan's, which walks
-// global memory with one thread searching (a coarsest level of 40 rows: 0.42
-// ms there, 0.05 here).
+// Explicit FP64 inverse of the coarsest level, one block: Gauss-Jordan in place
+// with partial pivoting, the rows left where they are (a row is a pivot once).
+// A thread holds rows q, q + 16, q + 32, q + 48 of one column in registers; a
+// step passes the pivot's column and scaled row through shared memory.  Its bound
+// is the FP64 unit of one multiprocessor: n^2 multiply-adds a step.  One thread
+// divides: the reciprocal of the pivot in every thread was 2.6 us of each step,
+// and matrix and inverse side by side in shared memory twice the multiply-adds.
 template <class V>
 __global__ void __launch_bounds__(kT, 1) k_small_inverse(SmallArgs<V> a) {
+    static_assert(kGjMax == 64 && kT == 1024, "16 threads a column, 4 rows a thread");
+    __shared__ double column[2][kGjMax], row[kGjMax], sinv;
+    __shared__ int spiv, order[kGjMax], place[kGjMax];   // step -> pivot row; its inverse
     extern __shared__ double dense[];
-    __shared__ int piv;
-    __shared__ double pval;
     SmallCtl* const ctl = a.ctl;
     if (ctl->status || ctl->abort || ctl->nlev < 1) return;
     const int l = ctl->nlev - 1, n = ctl->lev[l].n;
@@ -861,59 +864,77 @@ __global__ void __launch_bounds__(kT, 1) k_small_inverse(SmallArgs<V> a) {
     const int* ptr = l ? reinterpret_cast<const int*>(a.arena + ctl->lev[l].Aptr) : a.ptr;
     const int* col = l ? reinterpret_cast<const int*>(a.arena + ctl->lev[l].Acol) : a.col;
     const V* val = l ? reinterpret_cast<const V*>(a.arena + ctl->lev[l].Aval) : a.val;
-    double* const A = dense;
-    double* const I = dense + kGjMax * kGjMax;
-    for (int t = threadIdx.x; t < n * n; t += kT) { A[t] = 0.0; I[t] = (t / n == t % n) ? 1.0 : 0.0; }
+    for (int t = threadIdx.x; t < n * n; t += kT) dense[t] = 0.0;
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += kT)
-        for (int k = ptr[i]; k < ptr[i + 1]; ++k) A[i * n + col[k]] = (double)val[k];
+        for (int k = ptr[i]; k < ptr[i + 1]; ++k) dense[i * n + col[k]] = (double)val[k];
     __syncthreads();
+    const int k = threadIdx.x & 63, q = threadIdx.x >> 6, lane = threadIdx.x & 31;
+    double m[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int r = q + 16 * j;
+        m[j] = (k < n && r < n) ? dense[r * n + k] : 0.0;
+        if (k == 0) column[0][r] = m[j];
+    }
+    __syncthreads();
+    unsigned long long used = 0;   // pivot rows so far (the first warp's)
     for (int c = 0; c < n; ++c) {
-        if (threadIdx.x < 32) {   // the first largest |a_rc|, r >= c
-            double best = -1.0;
+        const double* const f = column[c & 1];
+        if (threadIdx.x < 32) {
+            // the first largest |a_rc| of the rows left; magnitudes compare as integers
+            unsigned long long best = 0;
             int p = n;
-            for (int r = c + (int)threadIdx.x; r < n; r += 32) {
-                const double v = fabs(A[r * n + c]);
-                if (v > best) { best = v; p = r; }
+            for (int r = lane; r < n; r += 32) {
+                const unsigned long long v = (unsigned long long)__double_as_longlong(f[r]) & 0x7fffffffffffffffull;
+                if (!(used >> r & 1) && (p == n || v > best)) { best = v; p = r; }
             }
+#pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
-                const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+                const unsigned long long ob = __shfl_xor_sync(0xffffffffu, best, o);
                 const int op = __shfl_xor_sync(0xffffffffu, p, o);
-                if (ob > best || (ob == best && op < p)) { best = ob; p = op; }
+                if (op < n && (p == n || ob > best || (ob == best && op < p))) { best = ob; p = op; }
             }
-            if (threadIdx.x == 0) {
-                if (p >= n) p = c;   // a column of NaNs
-                piv = p;
-                pval = A[p * n + c];
-                if (!(best > 0.0)) ctl->singular = 1;
+            used |= 1ull << p;   // c < n rows are used, so one is left
+            if (lane == 0) {
+                const double pv = f[p];
+                if (!(fabs(pv) > 0.0)) ctl->singular = 1;
+                spiv = p;
+                sinv = 1.0 / pv;
+                order[c] = p;
+                place[p] = c;
             }
         }
         __syncthreads();
-        if (pval == 0.0) return;
-        const int p = piv;
-        const double ip = 1.0 / pval;
-        for (int t = threadIdx.x; t < 2 * n; t += kT) {   // swap rows c and p, scale row c
-            double* const M = t < n ? A : I;
-            const int k = t < n ? t : t - n;
-            const double x = M[p * n + k];
-            if (p != c) M[p * n + k] = M[c * n + k];
-            M[c * n + k] = x * ip;
+        const int p = spiv;
+        const double ip = sinv;
+        if (f[p] == 0.0) return;
+        if (q == (p & 15) && k < n) {
+            const double x = p < 32 ? (p < 16 ? m[0] : m[1]) : (p < 48 ? m[2] : m[3]);
+            row[k] = k == c ? ip : x * ip;
         }
         __syncthreads();
-        for (int t = threadIdx.x; t < n * n; t += kT) {
-            const int r = t / n, k = t % n;
-            if (r == c) continue;
-            const double f = A[r * n + c];
-            if (k != c) A[r * n + k] -= f * A[c * n + k];
-            I[r * n + k] -= f * I[c * n + k];
+        if (k < n) {
+            const double rk = row[k];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int r = q + 16 * j;
+                if (r >= n) continue;
+                if (r == p) m[j] = rk;
+                else m[j] = (k == c ? 0.0 : m[j]) - f[r] * rk;
+                if (k == c + 1) column[(c + 1) & 1][r] = m[j];
+            }
         }
-        __syncthreads();
-        for (int r = threadIdx.x; r < n; r += kT)
-            if (r != c) A[r * n + c] = 0.0;
         __syncthreads();
     }
+    // row order[i] of the array is row i of the inverse, its column c belongs to right-hand side order[c]
     double* const out = reinterpret_cast<double*>(a.arena + ctl->cinv);
-    for (int t = threadIdx.x; t < n * n; t += kT) out[t] = I[t];
+    if (k < n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = q + 16 * j;
+            if (r < n) out[place[r] * n + order[k]] = m[j];
+        }
 }
 
 }  // namespace
@@ -963,8 +984,7 @@ SmallResult small_setup(semo_ctx* c, Amg<V>& h, float eps, double omega, const i
     void* args[] = {&a};
     SEMO_CUDA(cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(kT), args, kTableBytes, s));
     SEMO_CHECK_LAUNCH();
-    const int gj = 2 * kGjMax * kGjMax * (int)sizeof(double);
-    SEMO_CUDA(cudaFuncSetAttribute(k_small_inverse<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, gj));
+    const int gj = kGjMax * kGjMax * (int)sizeof(double);
     k_small_inverse<V><<<1, kT, gj, s>>>(a);
     SEMO_CHECK_LAUNCH();
     if (!c->hpin_small) SEMO_CUDA(cudaMallocHost(&c->hpin_small, sizeof(SmallCtl)));

@@ -646,7 +646,7 @@ __device__ __forceinline__ void bapply(const M* __restrict__ minv, int64_t i, co
 }
 
 // device scalars: 0 rho, 1 alpha, 2 omega, 3 beta, 4 <r,r>, 5 <rh,r>,
-// 6 <b,b>, 7 breakdown; partials: 2 x kRedBlocks
+// 6 <b,b>, 7 breakdown; partials: 2 x kRedBlocks of the products, 2 x of the residual
 __global__ void k_bi_init_sc(double* __restrict__ sc) {
     sc[0] = 1.0; sc[1] = 1.0; sc[2] = 1.0; sc[3] = 0.0; sc[7] = 0.0;
 }
@@ -722,24 +722,38 @@ __global__ void k_bi_mv(int nc, const int* __restrict__ off32, const int* __rest
     }
 }
 
-// alpha = rho / <rh, v>
-__global__ void k_bi_alpha(const double* __restrict__ part, double* __restrict__ sc) {
-    __shared__ double sh[32];
-    double a = 0.0;
-    for (int i = threadIdx.x; i < kRedBlocks; i += blockDim.x) a += part[i];
-    a = block_sum(a, sh);
-    if (threadIdx.x == 0) {
-        const double al = sc[0] / a;
-        if (!isfinite(al)) sc[7] = 1.0;
-        sc[1] = isfinite(al) ? al : 0.0;
-    }
+// sum of kRedBlocks partial sums, by one warp (every lane gets it)
+__device__ __forceinline__ double parts_sum(const double* part) {
+    double s[4] = {};
+    for (int i = threadIdx.x & 31; i < kRedBlocks; i += 128)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s[k] += i + 32 * k < kRedBlocks ? part[i + 32 * k] : 0.0;
+    double t = (s[0] + s[1]) + (s[2] + s[3]);
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
 }
 
-// z += alpha y; s = r - alpha v
-__global__ void k_bi_s(int nc, const double* __restrict__ sc, const double* __restrict__ r,
-                       const double* __restrict__ v, double* __restrict__ s, double* __restrict__ z,
-                       const double* __restrict__ y) {
-    const double alpha = sc[1];
+// The kernels that use alpha and omega add the partial sums themselves, and one
+// thread of a block divides; block 0 keeps what later kernels read, and no block
+// reads a scalar that this kernel writes.
+// alpha = rho / <rh, v>;  z += alpha y; s = r - alpha v
+__global__ void k_bi_s(int nc, const double* __restrict__ part, double* __restrict__ sc,
+                       const double* __restrict__ r, const double* __restrict__ v, double* __restrict__ s,
+                       double* __restrict__ z, const double* __restrict__ y) {
+    __shared__ double sal;
+    if (threadIdx.x < 32) {
+        const double a = parts_sum(part);
+        if (threadIdx.x == 0) {
+            const double al = sc[0] / a;
+            sal = isfinite(al) ? al : 0.0;
+            if (blockIdx.x == 0) {
+                if (!isfinite(al)) sc[7] = 1.0;
+                sc[1] = sal;
+            }
+        }
+    }
+    __syncthreads();
+    const double alpha = sal;
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < 5 * (int64_t)nc;
          q += (int64_t)gridDim.x * blockDim.x) {
         z[q] += alpha * y[q];
@@ -747,23 +761,21 @@ __global__ void k_bi_s(int nc, const double* __restrict__ sc, const double* __re
     }
 }
 
-// omega = <t, s> / <t, t>
-__global__ void k_bi_omega(const double* __restrict__ part, double* __restrict__ sc) {
-    __shared__ double sh[32];
-    double a = 0.0, b = 0.0;
-    for (int i = threadIdx.x; i < kRedBlocks; i += blockDim.x) { a += part[i]; b += part[kRedBlocks + i]; }
-    a = block_sum(a, sh);
+// omega = <t, s> / <t, t>;  z += omega y; r = s - omega t; partials (rpart) <r,r>, <rh,r>
+__global__ void k_bi_r(int nc, const double* __restrict__ part, double* __restrict__ sc,
+                       const double* __restrict__ s, const double* __restrict__ t, const double* __restrict__ y,
+                       const double* __restrict__ rh, double* __restrict__ z, double* __restrict__ r,
+                       double* __restrict__ rpart) {
+    __shared__ double sh[32], som;
+    if (threadIdx.x < 32) {
+        const double a = parts_sum(part), b = parts_sum(part + kRedBlocks);
+        if (threadIdx.x == 0) {
+            som = (b > 0.0) ? a / b : 0.0;
+            if (blockIdx.x == 0) sc[2] = som;
+        }
+    }
     __syncthreads();
-    b = block_sum(b, sh);
-    if (threadIdx.x == 0) sc[2] = (b > 0.0) ? a / b : 0.0;
-}
-
-// z += omega y; r = s - omega t; partials <r,r>, <rh,r>
-__global__ void k_bi_r(int nc, const double* __restrict__ sc, const double* __restrict__ s,
-                       const double* __restrict__ t, const double* __restrict__ y, const double* __restrict__ rh,
-                       double* __restrict__ z, double* __restrict__ r, double* __restrict__ part) {
-    __shared__ double sh[32];
-    const double omega = sc[2];
+    const double omega = som;
     double d1 = 0.0, d2 = 0.0;
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < 5 * (int64_t)nc;
          q += (int64_t)gridDim.x * blockDim.x) {
@@ -774,10 +786,10 @@ __global__ void k_bi_r(int nc, const double* __restrict__ sc, const double* __re
         d2 += rh[q] * rv;
     }
     d1 = block_sum(d1, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = d1;
+    if (threadIdx.x == 0) rpart[blockIdx.x] = d1;
     __syncthreads();
     d2 = block_sum(d2, sh);
-    if (threadIdx.x == 0) part[kRedBlocks + blockIdx.x] = d2;
+    if (threadIdx.x == 0) rpart[kRedBlocks + blockIdx.x] = d2;
 }
 
 __global__ void k_bi_fin_r(const double* __restrict__ part, double* __restrict__ sc) {
@@ -936,8 +948,8 @@ struct CplSolver {
     int nch = 0;
     int64_t rows32 = 0;            // slot rows (of 32 lanes)
     semo::DBuf<int> width, off32, col;
-    semo::DBuf<float> val32, minv32, cp32;    // cp: restricted residual and pressure correction (2 nc)
-    semo::DBuf<double> val64, minv64, cp64;
+    semo::DBuf<float> val32, minv32;
+    semo::DBuf<double> val64, minv64;
     semo::DBuf<double> vec;                   // 8 Krylov vectors of 5 nc
     semo::DBuf<double> part, sc, r64, app;    // app: pressure-equation values on the scalar pattern
     semo::DBuf<double> dinv64, rs;            // mixed mode: FP64 D^-1 blocks; the scaled residual D^-1 r
@@ -968,7 +980,7 @@ CplArgs make_args(semo_ctx* c) {
 // preconditioner, to rtol of ||src||; z is left in the 8th Krylov vector
 // (interleaved).  One host read of the residual per iteration.
 template <class M, class P>
-int bicgstab_inner(semo_ctx* c, CplSolver& S, const M* val, const M* minv, P* cpbuf, const double* src,
+int bicgstab_inner(semo_ctx* c, CplSolver& S, const M* val, const M* minv, const double* src,
                    double rtol, int maxit, double* rel_out, bool* breakdown) {
     using namespace semo;
     cudaStream_t s = c->stream;
@@ -982,11 +994,9 @@ int bicgstab_inner(semo_ctx* c, CplSolver& S, const M* val, const M* minv, P* cp
     double* h = c->hpin;
     // y = M^-1 in
     auto precond = [&](const double* in) {
-        P* bp = cpbuf;
-        P* zp = cpbuf + nc;
-        k_cpr_restrict<M, P><<<kRedBlocks, kT, 0, s>>>(nc, minv, in, bp);
+        k_cpr_restrict<M, P><<<kRedBlocks, kT, 0, s>>>(nc, minv, in, cpr_rhs<P>(c));
         SEMO_CHECK_LAUNCH();
-        cpr_vcycle<P>(c, bp, zp);
+        const P* const zp = cpr_vcycle<P>(c);
         k_cpr_second<M, P><<<kRedBlocks, kT, 0, s>>>(nc, S.off32, S.width, S.col, val, minv, in, zp, y);
         SEMO_CHECK_LAUNCH();
     };
@@ -1012,18 +1022,14 @@ int bicgstab_inner(semo_ctx* c, CplSolver& S, const M* val, const M* minv, P* cp
         precond(p);
         k_bi_mv<M, false><<<kRedBlocks, kT, 0, s>>>(nc, S.off32, S.width, S.col, val, y, v, rh, part);
         SEMO_CHECK_LAUNCH();
-        k_bi_alpha<<<1, kT, 0, s>>>(part, sc);
-        SEMO_CHECK_LAUNCH();
-        k_bi_s<<<kRedBlocks, kT, 0, s>>>(nc, sc, r, v, sv, z, y);
+        k_bi_s<<<kRedBlocks, kT, 0, s>>>(nc, part, sc, r, v, sv, z, y);
         SEMO_CHECK_LAUNCH();
         precond(sv);
         k_bi_mv<M, true><<<kRedBlocks, kT, 0, s>>>(nc, S.off32, S.width, S.col, val, y, t, sv, part);
         SEMO_CHECK_LAUNCH();
-        k_bi_omega<<<1, kT, 0, s>>>(part, sc);
+        k_bi_r<<<kRedBlocks, kT, 0, s>>>(nc, part, sc, sv, t, y, rh, z, r, part + 2 * kRedBlocks);
         SEMO_CHECK_LAUNCH();
-        k_bi_r<<<kRedBlocks, kT, 0, s>>>(nc, sc, sv, t, y, rh, z, r, part);
-        SEMO_CHECK_LAUNCH();
-        k_bi_fin_r<<<1, kT, 0, s>>>(part, sc);
+        k_bi_fin_r<<<1, kT, 0, s>>>(part + 2 * kRedBlocks, sc);
         SEMO_CHECK_LAUNCH();
         ++it;
         SEMO_CUDA(cudaMemcpyAsync(h, sc, 8 * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1087,13 +1093,12 @@ void coupled_assemble(semo_ctx* c) {
 }
 
 template <class M, class P>
-void prepare_blocks(semo_ctx* c, CplSolver& S, DBuf<M>& val, DBuf<M>& minv, DBuf<P>& cp, bool scaled) {
+void prepare_blocks(semo_ctx* c, CplSolver& S, DBuf<M>& val, DBuf<M>& minv, bool scaled) {
     cudaStream_t s = c->stream;
     const int nc = c->nc;
     const bool pattern = S.val32.n == 0 && S.val64.n == 0;
     val.alloc(25 * 32 * (size_t)S.rows32, s);
     minv.alloc(25 * (size_t)nc, s);
-    cp.alloc(2 * (size_t)nc, s);
     S.app.alloc((size_t)c->nnz, s);
     if (scaled) {
         // the copy holds D^-1 A: its block-Jacobi stage is the identity, and
@@ -1142,7 +1147,7 @@ semo_status coupled_solve(semo_ctx* c, semo_solve_info* info) {
     }
     SEMO_CUDA(cudaEventRecord(e0, s));
     StageScope stage(c, ST_CSOLVE);
-    S.part.alloc(2 * kRedBlocks, s);
+    S.part.alloc(4 * kRedBlocks, s);
     S.sc.alloc(8, s);
     // block SELL layout: the pattern once per mesh
     if (S.gen != c->mesh_gen) {
@@ -1160,8 +1165,8 @@ semo_status coupled_solve(semo_ctx* c, semo_solve_info* info) {
     }
     SEMO_CUDA(cudaMemsetAsync(c->flag.p + 12, 0, sizeof(int), s));
     const size_t n5 = 5 * (size_t)nc;
-    if (mixed) prepare_blocks<float, float>(c, S, S.val32, S.minv32, S.cp32, kScaleMixed);
-    else prepare_blocks<double, double>(c, S, S.val64, S.minv64, S.cp64, false);
+    if (mixed) prepare_blocks<float, float>(c, S, S.val32, S.minv32, kScaleMixed);
+    else prepare_blocks<double, double>(c, S, S.val64, S.minv64, false);
     SEMO_CUDA(cudaEventRecord(e1, s));
     int* const singular = c->hpin_scan + 3;
     SEMO_CUDA(cudaMemcpyAsync(singular, c->flag.p + 12, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1202,10 +1207,10 @@ semo_status coupled_solve(semo_ctx* c, semo_solve_info* info) {
                 SEMO_CHECK_LAUNCH();
                 src = S.rs;
             }
-            it = bicgstab_inner<float, float>(c, S, S.val32, S.minv32, S.cp32, src, std::max(1e-5, 0.5 * tol / rel),
+            it = bicgstab_inner<float, float>(c, S, S.val32, S.minv32, src, std::max(1e-5, 0.5 * tol / rel),
                                        maxit - total, &inner_rel, &brk);
         } else {
-            it = bicgstab_inner<double, double>(c, S, S.val64, S.minv64, S.cp64, S.r64, 0.5 * tol / rel, maxit - total,
+            it = bicgstab_inner<double, double>(c, S, S.val64, S.minv64, S.r64, 0.5 * tol / rel, maxit - total,
                                         &inner_rel, &brk);
         }
         k_add_il<<<kRedBlocks, kT, 0, s>>>(nc, S.vec.p + 7 * n5, c->cpl_x);
@@ -1242,7 +1247,7 @@ double coupled_update(semo_ctx* c) {
     cudaStream_t s = c->stream;
     StageScope sc(c, ST_CUPDATE);
     CplSolver& S = solver_state(c);
-    S.part.alloc(2 * kRedBlocks, s);
+    S.part.alloc(4 * kRedBlocks, s);
     S.sc.alloc(8, s);
     c->cpl_lim.upload(c->cphys.limits, 10, s);
     k_cupdate<<<kRedBlocks, kT, 0, s>>>(c->nc, c->cphys.urf, c->cpl_lim, c->cpl_x, c->cpl_f, S.part);

@@ -564,14 +564,35 @@ __global__ void k_copy_t(int n, const V* __restrict__ a, V* __restrict__ b) {
     if (i < n) b[i] = a[i];
 }
 
-// coarsest level: x = A^-1 b with the explicit FP64 inverse, one block
+// coarsest level: x = A^-1 b with the explicit FP64 inverse, one block, 4 lanes a
+// row with eight entries each in flight (a thread a row: 15 us for 61 rows)
 template <class V>
-__global__ void k_coarse_solve(int n, const double* __restrict__ inv, const V* __restrict__ b, V* __restrict__ x) {
+__global__ void __launch_bounds__(256) k_coarse_solve(int n, const double* __restrict__ inv, const V* __restrict__ b,
+                                                      V* __restrict__ x) {
     pdl_enter();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int sub = threadIdx.x & 3, rows = blockDim.x >> 2;
+    for (int i0 = 0; i0 < n; i0 += rows) {
+        const int i = i0 + (threadIdx.x >> 2);
         double s = 0.0;
-        for (int k = 0; k < n; ++k) s += inv[(size_t)i * n + k] * (double)b[k];
-        x[i] = (V)s;
+        if (i < n) {
+            const double* const m = inv + (size_t)i * n;
+            for (int k0 = sub; k0 < n; k0 += 32) {
+                double v[8];
+                V w[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int k = min(k0 + 4 * u, n - 1);
+                    v[u] = m[k];
+                    w[u] = b[k];
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (k0 + 4 * u < n) s += v[u] * widen<double>(w[u]);
+            }
+        }
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        if (i < n && sub == 0) x[i] = (V)s;
     }
 }
 
@@ -2484,14 +2505,14 @@ void cpr_setup(semo_ctx* c, const int* ptr, const int* col, const double* val, i
 
 // x = one V-cycle (zero start, both smoothing sweeps on every level) applied to b
 template <class V>
-void cpr_vcycle(semo_ctx* c, const V* b, V* x) {
+V* cpr_rhs(semo_ctx* c) { return cpr_h<V>(cpr_state(c)).lev[0].b.p; }
+template <class V>
+const V* cpr_vcycle(semo_ctx* c) {
     CprState& S = cpr_state(c);
     Amg<V>& h = cpr_h<V>(S);
     Cycle<V>& cy = cpr_cy<V>(S);
     cudaStream_t s = c->stream;
     AmgLevel<V>& L = h.lev[0];
-    const int n = L.A.n;
-    SEMO_CUDA(cudaMemcpyAsync(L.b.p, b, sizeof(V) * n, cudaMemcpyDeviceToDevice, s));
     vcycle_from(c, h, cy, 0);
     if (h.lev.size() > 1 && c->prm.cheb_degree == 2 && !cy.lev[0].gs) {
         // the last step vcycle_from leaves to the fused CG kernels on the finest level
@@ -2501,11 +2522,13 @@ void cpr_vcycle(semo_ctx* c, const V* b, V* x) {
         });
         SEMO_CHECK_LAUNCH();
     }
-    SEMO_CUDA(cudaMemcpyAsync(x, L.x.p, sizeof(V) * n, cudaMemcpyDeviceToDevice, s));
+    return L.x.p;
 }
 template void cpr_setup<float>(semo_ctx*, const int*, const int*, const double*, int, int64_t);
 template void cpr_setup<double>(semo_ctx*, const int*, const int*, const double*, int, int64_t);
-template void cpr_vcycle<float>(semo_ctx*, const float*, float*);
-template void cpr_vcycle<double>(semo_ctx*, const double*, double*);
+template float* cpr_rhs<float>(semo_ctx*);
+template double* cpr_rhs<double>(semo_ctx*);
+template const float* cpr_vcycle<float>(semo_ctx*);
+template const double* cpr_vcycle<double>(semo_ctx*);
 
 }  // namespace semo

@@ -388,9 +388,12 @@ void lsq_gradients5(semo_ctx* c, const double* f0, const double* f1, const doubl
 // cycle.cu: AMG on the pressure equation of the coupled system (value type float or double)
 template <class V>
 void cpr_setup(semo_ctx* c, const int* ptr, const int* col, const double* val, int n, int64_t nnz);
-// x = one V-cycle on b (device arrays of n)
+// one V-cycle: the right-hand side is written to cpr_rhs (n values, on the
+// context's stream), the result read from what cpr_vcycle returns
 template <class V>
-void cpr_vcycle(semo_ctx* c, const V* b, V* x);
+V* cpr_rhs(semo_ctx* c);
+template <class V>
+const V* cpr_vcycle(semo_ctx* c);
 
 // coupled.cu: compressible coupled 5x5 system
 void coupled_assemble(semo_ctx* c);
