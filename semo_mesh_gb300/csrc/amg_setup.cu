@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "amg_rows.cuh"
+#include "convert.cuh"
 #include "semo_internal.h"
 
 namespace semo {
@@ -116,17 +117,19 @@ __global__ void k_diag(int n, const int* __restrict__ ptr, const int* __restrict
                        V* __restrict__ dia, V* __restrict__ dinv, double* __restrict__ ratio, int* __restrict__ flag) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    double d = 0.0, rs = 0.0;
+    V d = V(0);
+    double rs = 0.0;
     for (int k = ptr[i]; k < ptr[i + 1]; ++k) {
-        const double v = (double)val[k];
+        const V v = val[k];
         if (col[k] == i) d = v;
-        rs += fabs(v);
+        rs += fabs(widen<double>(v));
     }
-    if (!(d > 0.0) && !(d < 0.0)) atomicExch(flag + 2, 1);   // zero diagonal
-    if (!isfinite(d) || !isfinite(rs)) atomicExch(flag + 3, 1);
-    dia[i] = (V)d;
-    dinv[i] = (V)(1.0 / d);
-    ratio[i] = rs / fabs(d);
+    if (!(d > V(0)) && !(d < V(0))) atomicExch(flag + 2, 1);   // zero diagonal
+    if (!isfinite(d) || ((__double2hiint(rs) >> 20) & 0x7ff) == 0x7ff) atomicExch(flag + 3, 1);
+    dia[i] = d;
+    const double inv = 1.0 / widen<double>(d);
+    dinv[i] = narrow<V>(inv);
+    ratio[i] = rs * fabs(inv);
 }
 
 __global__ void __launch_bounds__(kRedThreads) k_max(int n, const double* __restrict__ a, double* __restrict__ part) {
@@ -179,7 +182,7 @@ __global__ void k_strength(int n, const int* __restrict__ ptr, const int* __rest
     row_lane<VS>(i, lane);
     int has = 0;
     if (i < n) {
-        const V ed = (V)(eps2 * (double)dia[i]);
+        const V ed = narrow<V>(eps2 * widen<double>(dia[i]));
         for (int k = ptr[i] + lane; k < ptr[i + 1]; k += VS) {
             const int j = col[k];
             const V v = val[k];
@@ -306,37 +309,87 @@ __global__ void k_prolong_count(int n, const int* __restrict__ ptr, const int* _
     }
     cnt[i] = c;
 }
+// The row's aggregates and their sums, in entry order, in a list whose first
+// kFillListed places are in shared memory and the others at the row's places in
+// P, where the row ends up sorted.  What bounds it is the FP64 unit, so FP32
+// values become doubles and back by integer instructions: the conversions were
+// more than half of its instructions.
+constexpr int kFillThreads = 128, kFillListed = 8;
 template <class V>
-__global__ void k_prolong_fill(int n, const int* __restrict__ ptr, const int* __restrict__ col,
-                               const V* __restrict__ val, const unsigned char* __restrict__ strong,
-                               const int* __restrict__ agg, double omega, const int* __restrict__ pptr,
-                               int* __restrict__ pcol, V* __restrict__ pval) {
+__global__ void __launch_bounds__(kFillThreads) k_prolong_fill(int n, const int* __restrict__ ptr,
+                                                               const int* __restrict__ col,
+                                                               const V* __restrict__ val,
+                                                               const unsigned char* __restrict__ strong,
+                                                               const int* __restrict__ agg, double omega,
+                                                               const int* __restrict__ pptr, int* __restrict__ pcol,
+                                                               V* __restrict__ pval) {
+    __shared__ int lagg[kFillListed * kFillThreads];
+    __shared__ V lsum[kFillListed * kFillThreads];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    const int rb = ptr[i], re = ptr[i + 1];
+    int* const sagg = lagg + threadIdx.x;
+    V* const ssum = lsum + threadIdx.x;
+    int* const oagg = pcol + pptr[i];   // as many places as the row has aggregates
+    V* const osum = pval + pptr[i];
+    constexpr int kAhead = 8;   // entries loaded at once
+    int j[kAhead];
+    V x[kAhead];
+    bool st[kAhead];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int k = min(k0 + u, re - 1);
+            j[u] = col[k];
+            x[u] = val[k];
+            st[u] = strong[k] != 0;
+        }
+    };
     double df = 0.0;
-    for (int k = ptr[i]; k < ptr[i + 1]; ++k)
-        if (col[k] == i || !strong[k]) df += (double)val[k];
-    df = -omega * (1.0 / df);
-    const int rb = pptr[i];
-    int m = rb;
-    for (int k = ptr[i]; k < ptr[i + 1]; ++k) {
-        const int j = col[k];
-        if (j != i && !strong[k]) continue;
-        const int g = agg[j];
-        if (g < 0) continue;
-        const double v = (j == i) ? (1.0 - omega) : df * (double)val[k];
-        int t = rb;
-        while (t < m && pcol[t] != g) ++t;
-        if (t < m) pval[t] = (V)((double)pval[t] + v);
-        else { pcol[m] = g; pval[m] = (V)v; ++m; }
+    for (int k0 = rb; k0 < re; k0 += kAhead) {
+        load(k0);
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (k0 + u < re && (j[u] == i || !st[u])) df += widen<double>(x[u]);
     }
-    for (int s = rb + 1; s < m; ++s) {   // insertion sort by column
-        const int cv = pcol[s];
-        const V vv = pval[s];
-        int t = s - 1;
-        while (t >= rb && pcol[t] > cv) { pcol[t + 1] = pcol[t]; pval[t + 1] = pval[t]; --t; }
-        pcol[t + 1] = cv;
-        pval[t + 1] = vv;
+    df = -omega * (1.0 / df);
+    int m = 0;
+    for (int k0 = rb; k0 < re; k0 += kAhead) {
+        if (re - rb > kAhead) load(k0);
+        int g[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) g[u] = (k0 + u < re && (j[u] == i || st[u])) ? agg[j[u]] : -1;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            if (g[u] < 0) continue;
+            const double v = (j[u] == i) ? (1.0 - omega) : df * widen<double>(x[u]);
+            int t = 0;
+            while (t < m && (t < kFillListed ? sagg[t * kFillThreads] : oagg[t]) != g[u]) ++t;
+            V* const at = t < kFillListed ? ssum + t * kFillThreads : osum + t;
+            if (t < m) { *at = narrow<V>(widen<double>(*at) + v); continue; }
+            (t < kFillListed ? sagg[t * kFillThreads] : oagg[t]) = g[u];
+            *at = narrow<V>(v);
+            ++m;
+        }
+    }
+    if (m <= kFillListed) {
+        for (int e = 0; e < m; ++e) {
+            const int g = sagg[e * kFillThreads];
+            int rank = 0;
+            for (int u = 0; u < m; ++u) rank += sagg[u * kFillThreads] < g;
+            oagg[rank] = g;
+            osum[rank] = ssum[e * kFillThreads];
+        }
+    } else {
+        for (int e = 0; e < kFillListed; ++e) { oagg[e] = sagg[e * kFillThreads]; osum[e] = ssum[e * kFillThreads]; }
+        for (int e = 1; e < m; ++e) {   // insertion sort by aggregate
+            const int g = oagg[e];
+            const V v = osum[e];
+            int t = e - 1;
+            while (t >= 0 && oagg[t] > g) { oagg[t + 1] = oagg[t]; osum[t + 1] = osum[t]; --t; }
+            oagg[t + 1] = g;
+            osum[t + 1] = v;
+        }
     }
 }
 // the same rows with VS lanes: first[k] marks an entry whose aggregate has not
@@ -978,8 +1031,8 @@ void amg_setup(semo_ctx* c, Amg<V>& h, const int* ptr, const int* col, const dou
         // filling: the lane version rescans the row per output entry, which
         // only pays for the longest rows; both give the same values and order
         if (lanes < 32) {
-            k_prolong_fill<V><<<blocks(nl, 256), 256, 0, s>>>(nl, L.A.ptr, L.A.col, L.A.val, strong, agg, omega,
-                                                              L.P.ptr, L.P.col, L.P.val);
+            k_prolong_fill<V><<<blocks(nl, kFillThreads), kFillThreads, 0, s>>>(
+                nl, L.A.ptr, L.A.col, L.A.val, strong, agg, omega, L.P.ptr, L.P.col, L.P.val);
         } else {
             with_row_lanes(L.A.nnz, nl, [&](auto vs) {
                 constexpr int VS = decltype(vs)::value;
