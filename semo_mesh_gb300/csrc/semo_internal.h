@@ -165,8 +165,8 @@ struct semo_ctx {
     semo::DBuf<int2> stf;
     semo::DBuf<int> stfe;
     semo::DBuf<double> stfs, bfg;
-    semo::DBuf<int> st_tpos;                      // per stencil entry (j, i): the entry's position in i's row (adjoint)
-    int st_tpos_gen = -1;                         // mesh generation st_tpos was built for
+    semo::DBuf<double> st_wt;                     // per stencil entry (j, i): the weights of (i, j), 3 planes (adjoint)
+    int st_wt_gen = -1;                           // mesh generation st_wt was built for
     // derived per-face constants for the hot face kernel
     semo::DBuf<double> fk;                        // 7 planes of ni: kA = alpha*area/magPN, kP = alpha/magPN, area, wC, alpha*ePN (3)
 
