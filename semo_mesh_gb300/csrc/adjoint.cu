@@ -22,8 +22,8 @@
 //                 adjoints of the cell's own gradients (mapped through the
 //                 symmetric M^-1 of its LSQ fit) and of its clamped limits;
 //   k_adj_gather  over the cell's vertex stencil (symmetric, so the cells
-//                 whose gradients read cell j are j's own stencil; the weights
-//                 w_ij are kept in j's order, st_wt), its
+//                 whose gradients read cell j are j's own stencil; the weight
+//                 w_ij is read at its position in i's row, st_tpos), its
 //                 boundary faces (through the boundary-value rules) and the
 //                 limit adjoints of the stencil cells whose extremum it holds.
 #include <cuda_runtime.h>
@@ -35,10 +35,10 @@ namespace {
 
 using namespace semo::face;
 
-// for every entry (j, i) of j's stencil row the weights of entry (i, j) of i's row
-// (3 planes of stn); flag when the stencil is not symmetric
-__global__ void k_stencil_transpose(int nc, const int* __restrict__ stp, const int* __restrict__ sti, int64_t stn,
-                                    const double* __restrict__ stw, double* __restrict__ wt, int* __restrict__ flag) {
+// position of j in i's stencil row for every entry (j, i) of j's row; -1 (and
+// flag) when the stencil is not symmetric
+__global__ void k_stencil_tpos(int nc, const int* __restrict__ stp, const int* __restrict__ sti,
+                               int* __restrict__ tpos, int* __restrict__ flag) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nc) return;
     for (int k = stp[j]; k < stp[j + 1]; ++k) {
@@ -46,9 +46,8 @@ __global__ void k_stencil_transpose(int nc, const int* __restrict__ stp, const i
         int t = -1;
         for (int kk = stp[i]; kk < stp[i + 1]; ++kk)
             if (sti[kk] == j) { t = kk; break; }
-        if (t < 0) { atomicExch(flag, 1); continue; }
-#pragma unroll
-        for (int d = 0; d < 3; ++d) wt[d * stn + k] = stw[d * stn + t];
+        tpos[k] = t;
+        if (t < 0) atomicExch(flag, 1);
     }
 }
 
@@ -173,18 +172,17 @@ __global__ void __launch_bounds__(128) k_adj_cell(AdjCellArgs a) {
 
 struct AdjGatherArgs {
     int nc, ni, nf, nb;
-    int64_t stn;
-    const int *stp, *sti, *cfp, *cfi, *bpatch, *bct, *arg;
-    const double *wt, *stws, *bfw, *fn, *gdir, *gm, *lim;
+    const int *stp, *sti, *tpos, *cfp, *cfi, *bpatch, *bct, *arg;
+    const double *stw, *stws, *bfw, *fn, *gdir, *gm, *lim;
     double* out;   // 4 planes: dJ/dU, dJ/dV, dJ/dW, dJ/dP
 };
 
 // What bounds it is the FP64 unit (12 multiply-adds an entry) and the loads of 18
-// values an entry.  A limit adjoint reaches j from about one entry in 27, but from
-// some lane of a warp at most entries, so the places are listed first and added
-// afterwards (6 a cell on average instead of 109 additions a warp), and the
-// weights are read in j's own order: at their places in the neighbours' rows every
-// read was a sector of its own.
+// values an entry; an entry's three weights lie together, a sector or two where
+// three planes were three.  A limit adjoint reaches j from
+// about one entry in 27, but from some lane of a warp at most entries, so the
+// places are listed first and added afterwards (6 a cell on average instead of 109
+// additions a warp).
 constexpr int kAdjThreads = 128, kAdjListed = 16;
 __global__ void __launch_bounds__(kAdjThreads) k_adj_gather(AdjGatherArgs a) {
     __shared__ unsigned short listed[kAdjListed * kAdjThreads];   // 8 x place in the row + component
@@ -212,7 +210,9 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_gather(AdjGatherArgs a) {
     int np = 0;
     for (int k = kb; k < ke; ++k) {
         const int i = __ldg(a.sti + k);
-        const double w[3] = {__ldg(a.wt + k), __ldg(a.wt + a.stn + k), __ldg(a.wt + 2 * a.stn + k)};
+        const int t = __ldg(a.tpos + k);
+        const double* const wt = a.stw + 3 * (int64_t)t;
+        const double w[3] = {__ldg(wt), __ldg(wt + 1), __ldg(wt + 2)};
 #pragma unroll
         for (int q = 0; q < 4; ++q)
 #pragma unroll
@@ -267,18 +267,17 @@ void vjp_fields(semo_ctx* c, const double* lam, double* out) {
     const int nc = c->nc, nf = c->nf, ni = c->ni, nb = c->nb;
     const size_t N = nc;
     cudaStream_t s = c->stream;
-    // the stencil's transposed weights, once per mesh
-    if (c->st_wt_gen != c->mesh_gen) {
-        c->st_wt.alloc(3 * (size_t)std::max<int64_t>(c->st_nnz, 1), s);
+    // the stencil's transpose positions, once per mesh
+    if (c->st_tpos_gen != c->mesh_gen) {
+        c->st_tpos.alloc((size_t)std::max<int64_t>(c->st_nnz, 1), s);
         SEMO_CUDA(cudaMemsetAsync(c->flag.p + 13, 0, sizeof(int), s));
-        k_stencil_transpose<<<nblocks(nc, 128), 128, 0, s>>>(nc, c->st_ptr, c->st_idx, c->st_nnz, c->stw, c->st_wt,
-                                                             c->flag.p + 13);
+        k_stencil_tpos<<<nblocks(nc, 128), 128, 0, s>>>(nc, c->st_ptr, c->st_idx, c->st_tpos, c->flag.p + 13);
         SEMO_CHECK_LAUNCH();
         int* const bad = c->hpin_scan + 2;
         SEMO_CUDA(cudaMemcpyAsync(bad, c->flag.p + 13, sizeof(int), cudaMemcpyDeviceToHost, s));
         SEMO_CUDA(cudaStreamSynchronize(s));
         if (*bad) throw Error(SEMO_ERR_MESH, "vertex stencil is not symmetric");
-        c->st_wt_gen = c->mesh_gen;
+        c->st_tpos_gen = c->mesh_gen;
     }
     // checkpointed recomputation: face values, gradients, limits and their
     // arg-extrema from the current cell fields
@@ -305,10 +304,10 @@ void vjp_fields(semo_ctx* c, const double* lam, double* out) {
     k_adj_cell<<<nblocks(nc, 128), 128, 0, s>>>(a);
     SEMO_CHECK_LAUNCH();
     AdjGatherArgs g{};
-    g.nc = nc; g.ni = ni; g.nf = nf; g.nb = nb; g.stn = c->st_nnz;
-    g.stp = c->st_ptr; g.sti = c->st_idx; g.cfp = c->cf_ptr; g.cfi = c->cf_idx;
+    g.nc = nc; g.ni = ni; g.nf = nf; g.nb = nb;
+    g.stp = c->st_ptr; g.sti = c->st_idx; g.tpos = c->st_tpos; g.cfp = c->cf_ptr; g.cfi = c->cf_idx;
     g.bpatch = c->bpatch; g.bct = c->bc_type; g.arg = arg.p;
-    g.wt = c->st_wt; g.stws = c->stws; g.bfw = c->bfw; g.fn = c->fn; g.gdir = gdir.p; g.gm = gm.p; g.lim = lim.p;
+    g.stw = c->stw; g.stws = c->stws; g.bfw = c->bfw; g.fn = c->fn; g.gdir = gdir.p; g.gm = gm.p; g.lim = lim.p;
     g.out = out;
     k_adj_gather<<<nblocks(nc, kAdjThreads), kAdjThreads, 0, s>>>(g);
     SEMO_CHECK_LAUNCH();

@@ -173,7 +173,7 @@ __global__ void k_face_weights(int nf, int ni, int nc, const int* __restrict__ o
 // difference phi_k - phi_i.
 __global__ void k_lsq_setup(int nc, int nf, int ni, const int* __restrict__ stp, const int* __restrict__ sti,
                             const int* __restrict__ cfp, const int* __restrict__ cfi, const double* __restrict__ cc,
-                            const double* __restrict__ fc, int64_t stn, double* __restrict__ stw,
+                            const double* __restrict__ fc, double* __restrict__ stw,
                             double* __restrict__ bfw, double* __restrict__ minv, double* __restrict__ stws,
                             int* __restrict__ flag) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -188,7 +188,7 @@ __global__ void k_lsq_setup(int nc, int nf, int ni, const int* __restrict__ stp,
         const double wx = wk * dx, wy = wk * dy, wz = wk * dz;
         v0 += wx * dx; v1 += wx * dy; v2 += wx * dz;
         v9 += wy * dy; v10 += wy * dz; v17 += wz * dz;
-        stw[k] = wx; stw[stn + k] = wy; stw[2 * stn + k] = wz;
+        stw[3 * (int64_t)k] = wx; stw[3 * (int64_t)k + 1] = wy; stw[3 * (int64_t)k + 2] = wz;
         sx += wx; sy += wy; sz += wz;
     }
     const int nb = nf - ni;
@@ -261,7 +261,7 @@ void geometry_build(semo_ctx* c, const double* d_points, const int* d_fptr, cons
                                                 c->alf, c->epn, c->skew, c->pf, c->nfv);
     SEMO_CHECK_LAUNCH();
     k_lsq_setup<<<blocks(nc, T), T, 0, s>>>(nc, nf, ni, c->st_ptr, c->st_idx, c->cf_ptr, c->cf_idx, c->cc, c->fc,
-                                             c->st_nnz, c->stw, c->bfw, c->minv, c->stws, c->flag);
+                                             c->stw, c->bfw, c->minv, c->stws, c->flag);
     SEMO_CHECK_LAUNCH();
     stencil_weights(c);
     if (ni > 0) {

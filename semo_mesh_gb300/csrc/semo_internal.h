@@ -158,15 +158,15 @@ struct semo_ctx {
     // geometry (SoA, 3-vectors stored as 3 planes of length nf or nc)
     semo::DBuf<double> fn, fa, fc, wc, mpn, alf, epn, skew, pf, nfv;
     semo::DBuf<double> vol, ivol, cc, minv;       // ivol: 1 / vol; cc: 3 planes; minv: 6 planes
-    semo::DBuf<double> stw;                       // 3 planes of st_nnz: w_k * d_k (LSQ weight vectors)
+    semo::DBuf<double> stw;                       // w_k * d_k (LSQ weight vectors), an entry's three together
     semo::DBuf<double> bfw;                       // 3 planes of nb: boundary-face LSQ weight vectors
     semo::DBuf<double> stws;                      // 3 planes of nc: per-cell sum of the stencil and boundary weights
     // the fixed-point stencil weights of stencil.cu: entries, exponents, sums; boundary faces' weights
     semo::DBuf<int2> stf;
     semo::DBuf<int> stfe;
     semo::DBuf<double> stfs, bfg;
-    semo::DBuf<double> st_wt;                     // per stencil entry (j, i): the weights of (i, j), 3 planes (adjoint)
-    int st_wt_gen = -1;                           // mesh generation st_wt was built for
+    semo::DBuf<int> st_tpos;                      // per stencil entry (j, i): the entry's position in i's row (adjoint)
+    int st_tpos_gen = -1;                         // mesh generation st_tpos was built for
     // derived per-face constants for the hot face kernel
     semo::DBuf<double> fk;                        // 7 planes of ni: kA = alpha*area/magPN, kP = alpha/magPN, area, wC, alpha*ePN (3)
 

@@ -60,7 +60,7 @@ __global__ void k_stencil_weights(int nc, int ni, int nb, const int* __restrict_
                             {minv[2 * N + i], minv[4 * N + i], minv[5 * N + i]}};
     int e[3] = {0, 0, 0};
     for (int k = stp[i]; k < stp[i + 1]; ++k) {
-        const double w[3] = {stw[k], stw[stn + k], stw[2 * stn + k]};
+        const double w[3] = {stw[3 * (int64_t)k], stw[3 * (int64_t)k + 1], stw[3 * (int64_t)k + 2]};
 #pragma unroll
         for (int c = 0; c < 3; ++c) e[c] = max(e[c], exp_of(m[c][0] * w[0] + m[c][1] * w[1] + m[c][2] * w[2]));
     }
@@ -68,7 +68,7 @@ __global__ void k_stencil_weights(int nc, int ni, int nb, const int* __restrict_
 #pragma unroll
     for (int c = 0; c < 3; ++c) e[c] -= 1022;   // |g| < 2^e
     for (int k = stp[i]; k < stp[i + 1]; ++k) {
-        const double w[3] = {stw[k], stw[stn + k], stw[2 * stn + k]};
+        const double w[3] = {stw[3 * (int64_t)k], stw[3 * (int64_t)k + 1], stw[3 * (int64_t)k + 2]};
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const long long q = __double2ll_rn(ldexp(m[c][0] * w[0] + m[c][1] * w[1] + m[c][2] * w[2], kW - e[c]));

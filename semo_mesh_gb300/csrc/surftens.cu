@@ -43,15 +43,15 @@ using namespace semo::face;
 // stw, normal-matrix inverse in minv); boundary faces contribute nothing
 // (zero-gradient values: phi_b - phi_i = 0).
 __device__ __forceinline__ void lsq1(int i, int nc, const int* __restrict__ stp, const int* __restrict__ sti,
-                                     const double* __restrict__ stw, int64_t stn, const double* __restrict__ minv,
+                                     const double* __restrict__ stw, const double* __restrict__ minv,
                                      const double* __restrict__ phi, double g[3]) {
     const double pi = phi[i];
     double s0 = 0.0, s1 = 0.0, s2 = 0.0;
     for (int k = stp[i]; k < stp[i + 1]; ++k) {
         const double d = __ldg(phi + __ldg(sti + k)) - pi;
-        s0 += __ldg(stw + k) * d;
-        s1 += __ldg(stw + stn + k) * d;
-        s2 += __ldg(stw + 2 * stn + k) * d;
+        s0 += __ldg(stw + 3 * (int64_t)k) * d;
+        s1 += __ldg(stw + 3 * (int64_t)k + 1) * d;
+        s2 += __ldg(stw + 3 * (int64_t)k + 2) * d;
     }
     const double m0 = minv[i], m1 = minv[nc + i], m2 = minv[2 * nc + i];
     const double m3 = minv[3 * nc + i], m4 = minv[4 * nc + i], m5 = minv[5 * nc + i];
@@ -332,13 +332,13 @@ __global__ void k_sft_init(int nc, int ni, const int* __restrict__ cfp, const in
 }
 
 __global__ void k_sft_norm(int nc, const int* __restrict__ stp, const int* __restrict__ sti,
-                           const double* __restrict__ stw, int64_t stn, const double* __restrict__ minv,
+                           const double* __restrict__ stw, const double* __restrict__ minv,
                            const double* __restrict__ vol, const int* __restrict__ iface,
                            const double* __restrict__ ls0, double* __restrict__ ls1, double* __restrict__ vel0) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nc) return;
     double g[3];
-    lsq1(i, nc, stp, sti, stw, stn, minv, ls0, g);
+    lsq1(i, nc, stp, sti, stw, minv, ls0, g);
     double var = ls0[i];
     if (iface[i]) {
         const double mg = g[0] * g[0] + g[1] * g[1] + g[2] * g[2];
@@ -352,7 +352,7 @@ __global__ void k_sft_norm(int nc, const int* __restrict__ stp, const int* __res
 // One re-initialisation sweep, ls_in -> ls_out (Jacobi: every cell reads ls_in).
 __global__ void __launch_bounds__(128) k_sft_reinit(int nc, int ni, int nf, const int* __restrict__ stp,
                                                     const int* __restrict__ sti, const double* __restrict__ stw,
-                                                    int64_t stn, const double* __restrict__ minv,
+                                                    const double* __restrict__ minv,
                                                     const int* __restrict__ cfp, const int* __restrict__ cfi,
                                                     const int* __restrict__ own, const int* __restrict__ nei,
                                                     const double* __restrict__ cc, const double* __restrict__ pf,
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(128) k_sft_reinit(int nc, int ni, int nf, cons
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nc) return;
     double g[3];
-    lsq1(i, nc, stp, sti, stw, stn, minv, ls_in, g);
+    lsq1(i, nc, stp, sti, stw, minv, ls_in, g);
     const double m = sqrt(g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);
     double nv[3];
     for (int q = 0; q < 3; ++q) nv[q] = (m != 0.0) ? g[q] / m : 0.0;
@@ -392,12 +392,12 @@ __global__ void __launch_bounds__(128) k_sft_reinit(int nc, int ni, int nf, cons
 }
 
 __global__ void k_sft_normals(int nc, const int* __restrict__ stp, const int* __restrict__ sti,
-                              const double* __restrict__ stw, int64_t stn, const double* __restrict__ minv,
+                              const double* __restrict__ stw, const double* __restrict__ minv,
                               const double* __restrict__ ls, double* __restrict__ nrm) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nc) return;
     double g[3];
-    lsq1(i, nc, stp, sti, stw, stn, minv, ls, g);
+    lsq1(i, nc, stp, sti, stw, minv, ls, g);
     const double m = sqrt(g[0] * g[0] + g[1] * g[1] + g[2] * g[2]);
     for (int q = 0; q < 3; ++q) nrm[(size_t)q * nc + i] = (m > 1.e-15) ? g[q] / m : 0.0;
 }
@@ -516,17 +516,17 @@ void assemble_surface_tension(semo_ctx* c) {
     k_sft_init<<<B, T, 0, s>>>(nc, ni, c->cf_ptr, c->cf_idx, c->own, c->nei, c->wc, c->fa, c->vol, c->VF, lsb,
                                c->sft_iface, tau);
     SEMO_CHECK_LAUNCH();
-    k_sft_norm<<<B, T, 0, s>>>(nc, c->st_ptr, c->st_idx, c->stw, c->st_nnz, c->minv, c->vol, c->sft_iface, lsb, ls,
+    k_sft_norm<<<B, T, 0, s>>>(nc, c->st_ptr, c->st_idx, c->stw, c->minv, c->vol, c->sft_iface, lsb, ls,
                                vel0);
     SEMO_CHECK_LAUNCH();
     for (int it = 0; it < 4; ++it) {   // ls -> lsb -> ls -> lsb -> ls
         const double* in = (it & 1) ? lsb : ls;
         double* out = (it & 1) ? ls : lsb;
-        k_sft_reinit<<<B, T, 0, s>>>(nc, ni, nf, c->st_ptr, c->st_idx, c->stw, c->st_nnz, c->minv, c->cf_ptr,
+        k_sft_reinit<<<B, T, 0, s>>>(nc, ni, nf, c->st_ptr, c->st_idx, c->stw, c->minv, c->cf_ptr,
                                      c->cf_idx, c->own, c->nei, c->cc, c->pf, c->sft_iface, tau, vel0, in, out);
         SEMO_CHECK_LAUNCH();
     }
-    k_sft_normals<<<B, T, 0, s>>>(nc, c->st_ptr, c->st_idx, c->stw, c->st_nnz, c->minv, ls, nrm);
+    k_sft_normals<<<B, T, 0, s>>>(nc, c->st_ptr, c->st_idx, c->stw, c->minv, ls, nrm);
     SEMO_CHECK_LAUNCH();
     k_sft_kappa<<<B, T, 0, s>>>(nc, ni, nf, c->st_ptr, c->st_idx, c->cf_ptr, c->cf_idx, c->cc, c->pf, nrm, kap);
     SEMO_CHECK_LAUNCH();
