@@ -292,7 +292,8 @@ __device__ int hash_row(int lane, int ht, RowTable tb, int ab, int ae, const int
 // Four short rows by one warp, 8 lanes and a table of 32 slots each (tb: the
 // group's, with room for 32 slots): row [ab, ae) of the lane's group, ab == ae
 // for none.  The sums are hash_row's.  A row of 26 products leaves a warp's lanes
-// idle in all but one step and costs its latency, ~5 us, alone.  Returns the
+// idle in all but one step and costs its latency, ~5 us, alone (A P of 262,144
+// rows in the single-kernel setup 266 -> 118 us).  Returns the
 // length, or -1 (nothing written) when more than 24 slots are taken; *size: the
 // sum of |values|.
 constexpr int kGroup = 8, kGroupSlots = 32;

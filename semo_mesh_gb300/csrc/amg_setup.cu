@@ -313,7 +313,8 @@ __global__ void k_prolong_count(int n, const int* __restrict__ ptr, const int* _
 // kFillListed places are in shared memory and the others at the row's places in
 // P, where the row ends up sorted.  What bounds it is the FP64 unit, so FP32
 // values become doubles and back by integer instructions: the conversions were
-// more than half of its instructions.
+// more than half of its instructions (prolongation of a 128^3 hierarchy 1.11 ->
+// 0.90 ms).
 constexpr int kFillThreads = 128, kFillListed = 8;
 template <class V>
 __global__ void __launch_bounds__(kFillThreads) k_prolong_fill(int n, const int* __restrict__ ptr,

@@ -268,7 +268,8 @@ __device__ void block_product(const SmallArgs<V>& a, int level, int c0, int c1, 
     // a chunk with such a row has no room.
     constexpr int kMostProducts = 1 << 21;
     bool many = false;
-    // short rows (a mesh's): 8 lanes a row, here and in the sums
+    // short rows (a mesh's): 8 lanes a row, here and in the sums.  Up to 8 entries
+    // a row one step of the lanes holds a row; longer ones fill a warp by themselves
     const bool brief = c1 > c0 && (long long)aptr[c1] - aptr[c0] <= (long long)kGroup * (c1 - c0);
     const int vs = brief ? kGroup : 32, rpw = 32 / vs, sub = lane & (vs - 1);
     for (int r0 = c0 + wid * rpw; r0 < c1; r0 += kWarps * rpw) {
