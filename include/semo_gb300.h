@@ -360,7 +360,9 @@ semo_status semo_vjp_source(semo_ctx* ctx, const double* dJ_dx, double* lambda, 
    goes to the stencil cell holding the limit.  The face gradients are
    recomputed from the cell fields, not kept from the forward pass.  Needs a
    forward solve (semo_pressure_pass, or semo_assemble_pressure and
-   semo_solve_pressure).  Any output pointer may be NULL.  No reference
+   semo_solve_pressure) of the assembled matrix: after an assembly with other
+   values, or a caller's system in between, the result is
+   SEMO_ERR_NOT_CONVERGED or SEMO_ERR_STATE.  Any output pointer may be NULL.  No reference
    counterpart (SEMO has no adjoint). */
 semo_status semo_vjp_fields(semo_ctx* ctx, const double* dJ_dx, double* lambda, double* dJ_dU, double* dJ_dV,
                             double* dJ_dW, double* dJ_dP, semo_solve_info* info);

@@ -452,6 +452,7 @@ void assemble_pressure(semo_ctx* c) {
     assemble_gravity_stencil(c);
     double* coef = c->fscr.p;
     double* flux = c->fscr.p + nf;
+    if (!c->matrix_prebuilt) ++c->matrix_gen;
     if (ni > 0) {
         FaceArgs a;
         a.ni = ni; a.nf = nf; a.nc = nc;
@@ -484,6 +485,7 @@ void pressure_matrix(semo_ctx* c, cudaStream_t s) {
     const int T = 256;
     const int nc = c->nc, nf = c->nf, ni = c->ni, nb = c->nb;
     c->pm_coef.alloc(std::max(nf, 1), s);
+    ++c->matrix_gen;
     if (nf > 0) {
         k_pmat_face<<<blocks(nf, T), T, 0, s>>>(nf, ni, nb, c->own, c->nei, c->A_lr, c->A_rl, c->fk, c->irho,
                                                  c->bpatch, c->bc_type, c->mpn, c->alf, c->fa, c->bface,

@@ -426,6 +426,7 @@ semo_status semo_mesh_upload(semo_ctx* c, int n_points, const double* points, in
         c->A_lr.upload(alr.data(), alr.size(), s);
         c->A_rl.upload(arl.data(), arl.size(), s);
         c->A_val.alloc(c->nnz, s);
+        ++c->matrix_gen;
         c->b.alloc(nc, s);
         semo::DBuf<double> d_pts;
         semo::DBuf<int> d_fptr, d_fpts;

@@ -1377,8 +1377,13 @@ bool cluster_cg_fits(const semo_ctx* c, const Amg<V>& h, const Cycle<V>& cy, ClA
     return h.lev[0].A.n <= kClBlocks * kClThreads && cl_args<V>(h, 0, h.lev.size() > 1, a, &g);
 }
 
+// same: the hierarchy and outer were built from this matrix (ptr, col, val).
+// Without it they may belong to another one with as many rows, whose pattern
+// k_cluster_cg would not fit and whose residual is not this matrix's: the
+// iteration then runs on outer, and the residuals are formed with the caller's
+// matrix, so that a solution of the other system is not taken for converged.
 template <class V>
-void pcg(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const OuterOp& outer, const int* ptr, const int* col,
+void pcg(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const OuterOp& outer, bool same, const int* ptr, const int* col,
          const double* val, int n, const double* b, double* x, bool zero_guess, semo_solve_info* info) {
     cudaStream_t s = c->stream;
     Red R = red_area(c);
@@ -1398,7 +1403,7 @@ void pcg(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const OuterOp& outer, const int* 
     g.tol = c->prm.tol;
     g.max_iter = c->prm.max_iter;
     g.zero_guess = zero_guess;
-    if (cluster_cg_fits(c, h, cy, ca, g)) {   // the whole solve in one kernel
+    if (same && cluster_cg_fits(c, h, cy, ca, g)) {   // the whole solve in one kernel
         SEMO_CUDA(cudaMemsetAsync(R.scal, 0, sizeof(double) * 17, s));
         launch_cluster(k_cluster_cg<V>, s, kClBlocks, ca.smem, false, ca, g);
         SEMO_CUDA(cudaMemcpyAsync(h2, R.scal, sizeof(double) * 17, cudaMemcpyDeviceToHost, s));
@@ -1407,12 +1412,15 @@ void pcg(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const OuterOp& outer, const int* 
         return;
     }
     auto residual = [&] {
-        outer.with([&](auto A) {
-            if constexpr (decltype(A)::kEven > 0)
-                k_res64_even<decltype(A)::kEven><<<blocks(n, 256), 256, 0, s>>>(A, x, b, r);
-            else
-                k_res64<<<blocks((int64_t)n * 8, 256), 256, 0, s>>>(CsrView<double, 8>{ptr, col, val, n}, x, b, r);
-        });
+        bool done = false;
+        if (same)
+            outer.with([&](auto A) {
+                if constexpr (decltype(A)::kEven > 0) {
+                    k_res64_even<decltype(A)::kEven><<<blocks(n, 256), 256, 0, s>>>(A, x, b, r);
+                    done = true;
+                }
+            });
+        if (!done) k_res64<<<blocks((int64_t)n * 8, 256), 256, 0, s>>>(CsrView<double, 8>{ptr, col, val, n}, x, b, r);
         SEMO_CHECK_LAUNCH();
     };
     if (zero_guess) {
@@ -1509,6 +1517,9 @@ struct ApplyState {
     int src_n = 0;
     int64_t src_nnz = 0;
     int src_prec = -1;
+    // the generation of the mesh's matrix (semo_ctx::matrix_gen) that the
+    // hierarchy and outer were built from; -1: another matrix's
+    int of_gen = -1;
 };
 
 // flag[0] = 1 if a and b differ anywhere (bit patterns)
@@ -2028,6 +2039,7 @@ void pressure_setup(semo_ctx* c, const int* ptr, const int* col, const double* v
     c->sflag.alloc(16, s);
     SEMO_CUDA(cudaMemsetAsync(c->sflag.p, 0, 16 * sizeof(int), s));
     SEMO_CUDA(cudaEventRecord(c->setup_ev[0], s));
+    const bool mesh_matrix = ptr == c->A_ptr.p && col == c->A_col.p && val == c->A_val.p;
     {
         StageScope sc(c, ST_AMG_SETUP);
         // The hierarchy is a deterministic function of the matrix: when the
@@ -2048,6 +2060,7 @@ void pressure_setup(semo_ctx* c, const int* ptr, const int* col, const double* v
             SEMO_CUDA(cudaStreamSynchronize(s));
             reuse = *differs == 0;
         }
+        st.of_gen = -1;
         if (!reuse) {
             if (c->prm.precision == SEMO_PREC_MIXED) {
                 c->amg64.clear();
@@ -2081,6 +2094,7 @@ void pressure_setup(semo_ctx* c, const int* ptr, const int* col, const double* v
                 st.src_prec = c->prm.precision;
             }
         }
+        if (mesh_matrix) st.of_gen = c->matrix_gen;
     }
     SEMO_CUDA(cudaEventRecord(c->setup_ev[1], s));   // setup_ms is read from setup_ev after the solve
     (void)info;
@@ -2103,10 +2117,10 @@ void solve_system(semo_ctx* c, const int* ptr, const int* col, const double* val
     {
         StageScope sc(c, ST_PCG);
         if (c->prm.precision == SEMO_PREC_MIXED) {
-            pcg<float>(c, c->amg32, st.cy32, st.outer, ptr, col, val, n, b, x, zero_guess, info);
+            pcg<float>(c, c->amg32, st.cy32, st.outer, true, ptr, col, val, n, b, x, zero_guess, info);
             fill_info(c->amg32, nnz, info);
         } else {
-            pcg<double>(c, c->amg64, st.cy64, st.outer, ptr, col, val, n, b, x, zero_guess, info);
+            pcg<double>(c, c->amg64, st.cy64, st.outer, true, ptr, col, val, n, b, x, zero_guess, info);
             fill_info(c->amg64, nnz, info);
         }
     }
@@ -2328,18 +2342,27 @@ semo_status solve_csr_multi(semo_ctx* c, int n, const int* ptr, const int* col, 
 }
 
 // Adjoint solve on the hierarchy of the last forward solve (the pressure
-// matrix is symmetric, so A^T = A and the same preconditioner applies).
+// matrix is symmetric, so A^T = A and the same preconditioner applies).  The
+// matrix may have been assembled anew since, or the last solve a caller's
+// system: one of another size is refused, and otherwise the residual is that of
+// the assembled matrix, so that the solve of another one does not converge.
 void solve_transpose_reuse(semo_ctx* c, const double* g, double* lam, semo_solve_info* info) {
     const int n = c->nc;
     ApplyState& st = apply_state(c);
+    auto check = [&](const auto& h) {
+        if (!h.ready) throw Error(SEMO_ERR_STATE, "no hierarchy: run a forward solve first");
+        if (h.lev[0].A.n != n)
+            throw Error(SEMO_ERR_STATE, "the last solve was of a system of another size: run a forward solve first");
+    };
+    if (c->prm.precision == SEMO_PREC_MIXED) check(c->amg32);
+    else check(c->amg64);
+    const bool same = st.of_gen == c->matrix_gen;
     SEMO_CUDA(cudaEventRecord(c->ev[1], c->stream));
     if (c->prm.precision == SEMO_PREC_MIXED) {
-        if (!c->amg32.ready) throw Error(SEMO_ERR_STATE, "no hierarchy: run a forward solve first");
-        pcg<float>(c, c->amg32, st.cy32, st.outer, c->A_ptr, c->A_col, c->A_val, n, g, lam, true, info);
+        pcg<float>(c, c->amg32, st.cy32, st.outer, same, c->A_ptr, c->A_col, c->A_val, n, g, lam, true, info);
         fill_info(c->amg32, c->nnz, info);
     } else {
-        if (!c->amg64.ready) throw Error(SEMO_ERR_STATE, "no hierarchy: run a forward solve first");
-        pcg<double>(c, c->amg64, st.cy64, st.outer, c->A_ptr, c->A_col, c->A_val, n, g, lam, true, info);
+        pcg<double>(c, c->amg64, st.cy64, st.outer, same, c->A_ptr, c->A_col, c->A_val, n, g, lam, true, info);
         fill_info(c->amg64, c->nnz, info);
     }
     SEMO_CUDA(cudaEventRecord(c->ev[2], c->stream));

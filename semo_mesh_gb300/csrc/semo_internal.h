@@ -276,6 +276,7 @@ struct semo_ctx {
 
     bool mesh_ready = false, phys_ready = false, fields_ready = false, assembled = false;
     int mesh_gen = 0;                             // bumped by every mesh upload (cached layouts check it)
+    int matrix_gen = 0;                           // bumped whenever A_val is written (the hierarchy's user checks it)
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     // the pressure setup's own timing pair: the setup may run on the second
     // host thread while the momentum solve records ev[] on the main one
