@@ -58,7 +58,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(BUILD, exist_ok=True)
     headers = [os.path.join(CSRC, "semo_internal.h"), os.path.join(CSRC, "face_common.cuh"),
                os.path.join(CSRC, "amg_rows.cuh"), os.path.join(CSRC, "convert.cuh"),
-               os.path.join(CSRC, "cycle_cluster.cuh"),
+               os.path.join(CSRC, "cycle_cluster.cuh"), os.path.join(CSRC, "index.h"),
                os.path.join(os.path.dirname(HERE), "include", "semo_gb300.h")]
     procs = []
     objs = []

@@ -26,6 +26,7 @@
 #include <string>
 #include <vector>
 
+#include "index.h"
 #include "semo_internal.h"
 
 namespace semo {
@@ -84,9 +85,9 @@ __global__ void k_coo_rows(int n, const int* __restrict__ ptr, const int* __rest
                            const int* __restrict__ cols, const double* __restrict__ vals, int* __restrict__ col,
                            double* __restrict__ val, int* __restrict__ dig, CooFound* __restrict__ f) {
     if (f->longest > kCooMaxRow) return;   // the host converts it
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = g / kCooLanes, lane = g % kCooLanes;
-    const bool live = i < n;
+    const int64_t row = row_of(blockIdx.x, blockDim.x, threadIdx.x, kCooLanes);
+    const bool live = row < n;
+    const int i = live ? (int)row : 0, lane = threadIdx.x % kCooLanes;
     const int rb = live ? ptr[i] : 0, re = live ? ptr[i + 1] : 0;
     int first = INT_MAX;
     for (int e = rb + lane; e < re; e += kCooLanes) {

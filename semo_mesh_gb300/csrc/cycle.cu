@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "convert.cuh"
+#include "index.h"
 #include "semo_internal.h"
 
 namespace semo {
@@ -715,8 +716,7 @@ __global__ void k_conv(int n, const A* __restrict__ a, B* __restrict__ b) {
 // r = b - A x in FP64 (CSR, 8 lanes a row)
 __global__ void __launch_bounds__(256) k_res64(CsrView<double, 8> A, const double* __restrict__ x,
                                                const double* __restrict__ b, double* __restrict__ r) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    const int row = g / 8, lane = g % 8;
+    const int row = (int)min(row_of(blockIdx.x, blockDim.x, threadIdx.x, 8), (int64_t)A.n), lane = threadIdx.x % 8;
     const double s = A.dot(row, lane, Vec<double, double>{x});
     if (row < A.n && lane == 0) r[row] = b[row] - s;
 }
@@ -917,9 +917,8 @@ struct Sell16 {
 
 // SELL-32 structure with 16-bit columns of a square CSR pattern (slices that
 // fit no 16-bit encoding keep 32-bit columns).  hmost (two pinned ints, or
-// null): make the slices equally wide where Sell16UView has that width, every
-// slice has encoding 0 and it adds at most an eighth of padding -- more costs
-// what the known place gains.
+// null): make the slices equally wide where Sell16UView has that width and
+// every slice has encoding 0 (even_slots).
 std::shared_ptr<Sell16Struct> build_sell16_struct(cudaStream_t s, const int* ptr, const int* col, int n,
                                                   int* hpin, int* hmost) {
     auto S = std::make_shared<Sell16Struct>();
@@ -942,14 +941,12 @@ std::shared_ptr<Sell16Struct> build_sell16_struct(cudaStream_t s, const int* ptr
     SEMO_CHECK_LAUNCH();
     if (most) SEMO_CUDA(cudaMemcpyAsync(hmost, most, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
     const int wide = device_scan(s, S->wptr.p, S->nslices + 1, hpin);   // its sync lands hmost too
-    if (most && hmost[1] == 0 && hmost[0] >= 5 && hmost[0] <= 7) {
-        const int64_t even = 32 * (int64_t)hmost[0] * S->nslices;
-        if (even <= (int64_t)S->slots + S->slots / 8) {
-            S->width = hmost[0];
-            S->slots = (int)even;
-            k_sell16_even<<<blocks(S->nslices + 1, 256), 256, 0, s>>>(S->nslices, S->width, S->sptr.p);
-            SEMO_CHECK_LAUNCH();
-        }
+    const int64_t even = most && hmost[1] == 0 ? even_slots(hmost[0], 5, 7, S->nslices, S->slots) : 0;
+    if (even) {
+        S->width = hmost[0];
+        S->slots = (int)even;
+        k_sell16_even<<<blocks(S->nslices + 1, 256), 256, 0, s>>>(S->nslices, S->width, S->sptr.p);
+        SEMO_CHECK_LAUNCH();
     }
     S->dcol.alloc(std::max(S->slots, 1), s);
     S->wcol.alloc(std::max(wide, 1), s);
@@ -1714,7 +1711,7 @@ struct OffDiag {
     }
 };
 // the layout of a pattern, without values and columns; hpin: two pinned ints.
-// Slices are made equally wide under the rule of build_sell16_struct
+// Slices are made equally wide where OffEven has that width (even_slots)
 void build_offdiag(cudaStream_t s, const int* ptr, int n, OffDiag& S, int* hpin) {
     S.n = n;
     S.nslices = (n + 31) / 32;
@@ -1725,8 +1722,7 @@ void build_offdiag(cudaStream_t s, const int* ptr, int n, OffDiag& S, int* hpin)
     SEMO_CHECK_LAUNCH();
     SEMO_CUDA(cudaMemcpyAsync(hpin + 1, S.sptr.p + S.nslices + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
     int total = device_scan(s, S.sptr.p, S.nslices + 1, hpin);   // its sync lands hpin[1] too
-    const int64_t even = 32 * (int64_t)hpin[1] * S.nslices;
-    if (hpin[1] >= 4 && hpin[1] <= 6 && even <= (int64_t)total + total / 8 && even < INT_MAX) {
+    if (const int64_t even = even_slots(hpin[1], 4, 6, S.nslices, total)) {
         S.width = hpin[1];
         total = (int)even;
     }
