@@ -1579,22 +1579,25 @@ void prepare_cycle(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const std::shared_ptr<S
 // x = D^-1 xh at the end.  B's diagonal is 1 and is not stored: a product starts
 // from the row's own value and adds the off-diagonal entries.
 // What bounds the iteration is the FP64 unit (2 lanes a clock and
-// multiprocessor): 72 instructions a row and iteration of three systems, and
-// 548 bytes.  So D^-1 p and D^-1 s are never formed (the search directions
-// themselves are gathered), rho comes from the sums of the second product,
-// rho' = (rh,s) - omega (rh,t), which lets one kernel end an iteration and
-// begin the next, and every scalar is formed by the kernels that use it: five
-// kernels an iteration.  Momentum solve at 75^3 cells 0.391 -> 0.275 ms, three
-// right-hand sides of 67,080 caller's rows 0.60 -> 0.37.
+// multiprocessor): 69 instructions a row and iteration of three systems, and
+// 600 bytes.  So D^-1 p and D^-1 s are never formed (the search directions
+// themselves are gathered), and the scalars but beta are formed by the kernels
+// that use them: six kernels an iteration, and one for the residual of the
+// result.  Momentum solve at 75^3 cells 0.391 -> 0.277 ms, three right-hand sides
+// of 67,080 caller's rows 0.60 -> 0.385.  rho is the sum (rh,r) itself: as
+// (rh,s) - omega (rh,t), from the sums of the second product, it would save the
+// kernel that forms p, 3 us of a solve at 75^3, but on implicit transport systems
+// of 1,980 to 34,720 rows its error against extended precision was 3 to 40 times
+// as large (rms 1.3e-15 against 1.3e-16 at 34,720).
 // Per system j the scalars live at scal[16 j + k]:
-//   0 rho, 1 alpha, 2 omega, 7 (r,r), 8 (b,b), 9 active, 10 breakdown,
-//   11 iterations, 12 the next rho
+//   0 rho, 1 alpha, 2 omega, 3 beta, 7 (r,r), 8 (b,b), 9 active, 10 breakdown,
+//   11 iterations
 constexpr int kMomScal = 16;
 // Grid: at most 152 blocks (one a GB300 multiprocessor; not taken from the
 // device, so that every sum's bits are the same on any GPU), because each block
-// adds up the partial sums of all (12 sums of three systems: 1 us with 152
-// partials, 9 us with four blocks of 256 threads a multiprocessor, at 16 clocks
-// an FP64 warp instruction).  Threads: what deals n out in equal sweeps.
+// adds up the partial sums of all (12 sums: 1 us with 152 partials, 9 us with
+// four blocks of 256 threads a multiprocessor, at 16 clocks an FP64 warp
+// instruction; a kernel here needs 6).  Threads: what deals n out in equal sweeps.
 constexpr int kBiBlocks = 152, kBiThreads = 512, kBiStream = 1024;
 struct BiGrid { int blocks, threads; };
 inline BiGrid bi_grid(int n, int most) {
@@ -1819,8 +1822,8 @@ __global__ void __launch_bounds__(kBiThreads) k_bi_mv1(M B, const double* __rest
     bi_put<NR>(d, sh, part);
 }
 // alpha = rho / (rh,v);  s = r - alpha v (in place in r).  One thread a system
-// forms the scalars here and in k_bi_xrp: three divisions in every thread took
-// 5 and 25 us
+// forms the scalars here and in k_bi_xr: the divisions in every thread took 5 us
+// and more
 template <int NR>
 __global__ void __launch_bounds__(kBiStream) k_bi_s(int n, double* __restrict__ r, const double* __restrict__ v,
                                                     double* __restrict__ scal, const double* __restrict__ part,
@@ -1850,86 +1853,98 @@ __global__ void __launch_bounds__(kBiStream) k_bi_s(int n, double* __restrict__ 
             r[j * N + i] -= alpha * v[j * N + i];
     }
 }
-// t = B s;  part = (t,s), (t,t), (rh,s), (rh,t) per system
+// t = B s;  part = (t,s), (t,t) per system
 template <int NR, class M>
 __global__ void __launch_bounds__(kBiThreads) k_bi_mv2(M B, const double* __restrict__ s, double* __restrict__ t,
-                                                       const double* __restrict__ rh,
                                                        const double* __restrict__ scal, double* __restrict__ part) {
     pdl_enter();
-    __shared__ double sh[4 * kBiThreads];
+    __shared__ double sh[2 * NR * kBiThreads];
     const size_t N = B.n;
     const unsigned act = bi_active(scal, NR);
-    double d[4 * NR] = {};
+    double d[2 * NR] = {};
     for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < B.n; row += gridDim.x * blockDim.x) {
         double y[NR];
         B.template mv<NR>(row, act, s, y);
 #pragma unroll
         for (int j = 0; j < NR; ++j) {
             if (!(act >> j & 1)) continue;
-            const double si = s[j * N + row], ri = rh[j * N + row];
             t[j * N + row] = y[j];
-            d[4 * j] += y[j] * si;
-            d[4 * j + 1] += y[j] * y[j];
-            d[4 * j + 2] += ri * si;
-            d[4 * j + 3] += ri * y[j];
+            d[2 * j] += y[j] * s[j * N + row];
+            d[2 * j + 1] += y[j] * y[j];
         }
     }
-#pragma unroll
-    for (int j = 0; j < NR; ++j) bi_put<4>(d + 4 * j, sh, part + 4 * j * kBiBlocks);
+    bi_put<2 * NR>(d, sh, part);
 }
-// omega = (t,s) / (t,t), the next rho and beta = (rho' / rho) (alpha / omega);  xh += alpha p + omega s;  r = s - omega t;
-// p = r + beta (p - omega v);  part = (r,r) per system
+// omega = (t,s) / (t,t);  xh += alpha p + omega s;  r = s - omega t;  part = (r,r),
+// (rh,r) per system
 template <int NR>
-__global__ void __launch_bounds__(kBiStream) k_bi_xrp(int n, double* __restrict__ xh, double* __restrict__ p,
-                                                      double* __restrict__ r, const double* __restrict__ v,
-                                                      const double* __restrict__ t, double* __restrict__ scal,
-                                                      const double* __restrict__ parts, int nb,
-                                                      double* __restrict__ part) {
+__global__ void __launch_bounds__(kBiStream) k_bi_xr(int n, double* __restrict__ xh, const double* __restrict__ p,
+                                                     double* __restrict__ r, const double* __restrict__ t,
+                                                     const double* __restrict__ rh, double* __restrict__ scal,
+                                                     const double* __restrict__ parts, int nb,
+                                                     double* __restrict__ part) {
     pdl_enter();
-    __shared__ double sh[NR * kBiStream], tot[4 * NR], sal[NR], som[NR], sbe[NR];
-    bi_get<4 * NR>(parts, nb, tot);
+    __shared__ double sh[2 * kBiStream], tot[2 * NR], sal[NR], som[NR];
+    bi_get<2 * NR>(parts, nb, tot);
     if (threadIdx.x < NR) {
         const int j = threadIdx.x;
         double* const S = scal + kMomScal * j;   // no block reads what this kernel writes
-        const double tt = tot[4 * j + 1], omega = (tt > 0.0) ? tot[4 * j] / tt : 0.0, alpha = S[1];
-        const double rho = tot[4 * j + 2] - omega * tot[4 * j + 3];
-        sal[j] = alpha;
+        const double tt = tot[2 * j + 1], omega = (tt > 0.0) ? tot[2 * j] / tt : 0.0;
+        sal[j] = S[1];
         som[j] = omega;
-        sbe[j] = (rho / S[0]) * (alpha / omega);
-        if (blockIdx.x == 0 && S[9] != 0.0 && S[10] == 0.0) { S[2] = omega; S[12] = rho; }
+        if (blockIdx.x == 0 && S[9] != 0.0 && S[10] == 0.0) S[2] = omega;
     }
     __syncthreads();
     const unsigned act = bi_active(scal, NR);
     const size_t N = n;
-    double rr[NR] = {};
+    double d[2 * NR] = {};
 #pragma unroll
     for (int j = 0; j < NR; ++j) {
         if (!(act >> j & 1)) continue;
-        const double alpha = sal[j], omega = som[j], beta = sbe[j];
+        const double alpha = sal[j], omega = som[j];
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
             const size_t k = j * N + i;
-            const double pi = p[k], si = r[k], vi = v[k], ti = t[k], xi = xh[k];
-            xh[k] = xi + (alpha * pi + omega * si);
-            const double ri = si - omega * ti;
+            const double si = r[k], hi = rh[k];
+            xh[k] += alpha * p[k] + omega * si;
+            const double ri = si - omega * t[k];
             r[k] = ri;
-            p[k] = ri + beta * (pi - omega * vi);
-            rr[j] += ri * ri;
+            d[2 * j] += ri * ri;
+            d[2 * j + 1] += hi * ri;
         }
     }
-    bi_put<NR>(rr, sh, part);
+#pragma unroll
+    for (int j = 0; j < NR; ++j) bi_put<2>(d + 2 * j, sh, part + 2 * j * kBiBlocks);
 }
-// The end of an iteration: each system's state, and whether the loop goes on (a
-// system is active and the cap is not reached; scal[3 * 16] counts iterations)
+// p = r + beta (p - omega v)
+template <int NR>
+__global__ void __launch_bounds__(kBiStream) k_bi_p(int n, double* __restrict__ p, const double* __restrict__ r,
+                                                    const double* __restrict__ v, const double* __restrict__ scal) {
+    pdl_enter();
+    const unsigned act = bi_active(scal, NR);
+    const size_t N = n;
+#pragma unroll
+    for (int j = 0; j < NR; ++j) {
+        if (!(act >> j & 1)) continue;
+        const double omega = scal[kMomScal * j + 2], beta = scal[kMomScal * j + 3];
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+            const size_t k = j * N + i;
+            p[k] = r[k] + beta * (p[k] - omega * v[k]);
+        }
+    }
+}
+// The end of an iteration but for p: each system's state, the next rho and beta =
+// (rho' / rho) (alpha / omega), and whether the loop goes on (a system is active
+// and the cap is not reached; scal[3 * 16] counts iterations)
 template <int NR>
 __global__ void k_bi_check(cudaGraphConditionalHandle h, double* __restrict__ scal, const double* __restrict__ part,
                            int nb, double tol2, int max_iter) {
     pdl_enter();
-    __shared__ double tot[NR];
-    bi_get<NR>(part, nb, tot);
+    __shared__ double tot[2 * NR];
+    bi_get<2 * NR>(part, nb, tot);
     bool any = false;
     if (threadIdx.x < NR) {
         double* S = scal + kMomScal * threadIdx.x;
-        const double rr = tot[threadIdx.x];
+        const double rr = tot[2 * threadIdx.x], rho = tot[2 * threadIdx.x + 1];
         if (S[9] == 0.0) {
         } else if (S[10] != 0.0) {
             S[9] = 0.0;                                         // (rh,v) was 0 or not finite
@@ -1938,10 +1953,11 @@ __global__ void k_bi_check(cudaGraphConditionalHandle h, double* __restrict__ sc
             S[7] = rr;
             if (rr <= tol2 * S[8]) {
                 S[9] = 0.0;                                     // converged
-            } else if (S[12] == 0.0 || S[2] == 0.0 || !isfinite(rr)) {
+            } else if (rho == 0.0 || S[2] == 0.0 || !isfinite(rr)) {
                 S[10] = 1.0; S[9] = 0.0;                        // breakdown
             } else {
-                S[0] = S[12];
+                S[3] = (rho / S[0]) * (S[1] / S[2]);
+                S[0] = rho;
                 any = true;
             }
         }
@@ -2191,14 +2207,14 @@ semo_status bicgstab_jacobi(semo_ctx* c, int stage, const KrylovPattern& pat, co
     MomState& st = mom_state(c);
     st.dinv.alloc(N, s);
     st.vec.alloc(5 * 3 * N, s);       // r, p, v, t, xh (room for 3 systems)
-    st.part.alloc((size_t)(12 + 3) * kBiBlocks, s);
+    st.part.alloc((size_t)(6 + 6) * kBiBlocks, s);
     st.scal.alloc(4 * kMomScal, s);
     double* r = st.vec.p;
     double* p = r + NR * N;
     double* v = p + NR * N;
     double* t = v + NR * N;
     double* xh = t + NR * N;
-    double* const prr = st.part.p + 12 * kBiBlocks;
+    double* const prr = st.part.p + 6 * kBiBlocks;
     // the recurrence residual is driven to half the tolerance so that the true
     // residual, checked at the end, lands under it
     const double tol2 = 0.25 * c->prm.mom_tol * c->prm.mom_tol;
@@ -2219,7 +2235,7 @@ semo_status bicgstab_jacobi(semo_ctx* c, int stage, const KrylovPattern& pat, co
     k_bi_fin0<NR><<<1, 32 * NR, 0, s>>>(st.part, gs.blocks, st.scal, tol2);
     SEMO_CHECK_LAUNCH();
     // The iterations run as one graph: a conditional WHILE node around one
-    // iteration (4 kernels and k_bi_check), launched without a host round trip
+    // iteration (5 kernels and k_bi_check), launched without a host round trip
     // first: systems whose right-hand side is zero, already converged or not
     // finite start inactive (k_bi_fin0), every kernel skips them, and the
     // host reads the outcome once, after the true residuals.
@@ -2253,12 +2269,13 @@ semo_status bicgstab_jacobi(semo_ctx* c, int stage, const KrylovPattern& pat, co
             });
             launch_pdl(k_bi_s<NR>, gs.blocks, gs.threads, s, n, r, v, st.scal.p, st.part.p, gm.blocks);
             st.B.with([&](auto B) {
-                launch_pdl(k_bi_mv2<NR, decltype(B)>, gm.blocks, gm.threads, s, B, r, t, b, st.scal.p, st.part.p);
+                launch_pdl(k_bi_mv2<NR, decltype(B)>, gm.blocks, gm.threads, s, B, r, t, st.scal.p, st.part.p);
             });
-            launch_pdl(k_bi_xrp<NR>, gs.blocks, gs.threads, s, n, xh, p, r, v, t, st.scal.p, st.part.p, gm.blocks,
+            launch_pdl(k_bi_xr<NR>, gs.blocks, gs.threads, s, n, xh, p, r, t, b, st.scal.p, st.part.p, gm.blocks,
                        prr);
             launch_pdl(k_bi_check<NR>, 1, 32 * NR, s, handle, st.scal.p, prr, gs.blocks, tol2,
                        c->prm.mom_max_iter);
+            launch_pdl(k_bi_p<NR>, gs.blocks, gs.threads, s, n, p, r, v, st.scal.p);
         } catch (...) {
             cudaGraph_t junk = nullptr;
             cudaStreamEndCapture(s, &junk);
@@ -2286,7 +2303,7 @@ semo_status bicgstab_jacobi(semo_ctx* c, int stage, const KrylovPattern& pat, co
     SEMO_CUDA(cudaEventRecord(c->ev[2], s));
     SEMO_CUDA(cudaEventSynchronize(c->ev[2]));
     const int it = (int)hs[3 * kMomScal];
-    __atomic_add_fetch(&g_kernel_launches, 5LL * it, __ATOMIC_RELAXED);
+    __atomic_add_fetch(&g_kernel_launches, 6LL * it, __ATOMIC_RELAXED);
     int iters[NR] = {};
     for (int j = 0; j < NR; ++j) {
         if (!std::isfinite(hs[kMomScal * j + 8])) throw Error(SEMO_ERR_NAN, "non-finite right-hand side");
