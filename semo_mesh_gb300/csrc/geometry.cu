@@ -263,7 +263,6 @@ void geometry_build(semo_ctx* c, const double* d_points, const int* d_fptr, cons
     k_lsq_setup<<<blocks(nc, T), T, 0, s>>>(nc, nf, ni, c->st_ptr, c->st_idx, c->cf_ptr, c->cf_idx, c->cc, c->fc,
                                              c->stw, c->bfw, c->minv, c->stws, c->flag);
     SEMO_CHECK_LAUNCH();
-    stencil_weights(c);
     if (ni > 0) {
         k_face_consts<<<blocks(ni, T), T, 0, s>>>(ni, nf, c->fa, c->mpn, c->alf, c->wc, c->epn, c->fk);
         SEMO_CHECK_LAUNCH();

@@ -161,10 +161,6 @@ struct semo_ctx {
     semo::DBuf<double> stw;                       // w_k * d_k (LSQ weight vectors), an entry's three together
     semo::DBuf<double> bfw;                       // 3 planes of nb: boundary-face LSQ weight vectors
     semo::DBuf<double> stws;                      // 3 planes of nc: per-cell sum of the stencil and boundary weights
-    // the fixed-point stencil weights of stencil.cu: entries, exponents, sums; boundary faces' weights
-    semo::DBuf<int2> stf;
-    semo::DBuf<int> stfe;
-    semo::DBuf<double> stfs, bfg;
     semo::DBuf<int> st_tpos;                      // per stencil entry (j, i): the entry's position in i's row (adjoint)
     int st_tpos_gen = -1;                         // mesh generation st_tpos was built for
     // derived per-face constants for the hot face kernel
@@ -367,9 +363,7 @@ void assemble_face_values(semo_ctx* c, bool with_mu);
 // gravity source + one stencil pass (gradients of P,U,V,W,VF; min/max of U,V,W,VF,P)
 void assemble_gravity_stencil(semo_ctx* c);
 void assemble_gravity(semo_ctx* c);
-// stencil.cu: the mesh's fixed-point LSQ weights (after the LSQ setup)
-void stencil_weights(semo_ctx* c);
-// full: all five fields; else U, V, W only (P and VF planes left as they are)
+// stencil.cu; full: all five fields; else U, V, W only (P and VF planes left as they are)
 void stencil_pass(semo_ctx* c, bool full);
 // surftens.cu: curvature and surface-tension source (no-op when sigma == 0);
 // after assemble_face_values and a full stencil_pass
