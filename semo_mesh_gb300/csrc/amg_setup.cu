@@ -910,10 +910,11 @@ void amg_setup(semo_ctx* c, Amg<V>& h, const int* ptr, const int* col, const dou
     };
     SmallResult small = SmallResult::no_room;
     bool try_small = true;
+    const bool mesh_matrix = val64 == c->A_val.p;   // the one that is set up beside the momentum pass or alone
     int above = 0;   // levels built here
     for (int l = 0;; ++l) {
         AmgLevel<V>& L = h.lev[l];
-        if (try_small && small_setup_fits(L.A.n, L.A.nnz, s != c->stream)) {
+        if (try_small && small_setup_fits(L.A.n, L.A.nnz, mesh_matrix)) {
             StageScope sc(c, ST_SETUP_GALERKIN);
             read_back();
             small = small_setup(c, h, eps, omega, hf);

@@ -22,7 +22,12 @@
 // pass the line is lower, since a block here keeps a multiprocessor to
 // itself: with the finest level of a 47^3 box (103,823 rows) a time step was
 // 5.32 ms against 4.90, with the second level of an 80^3 box (46,686 rows,
-// 1.5M entries) 9.3 against 10.3.  For the same reason a block takes
+// 1.5M entries) 9.3 against 10.3.  The two ways differ by rounding, and a
+// hierarchy of the mesh's pressure matrix may be built beside the momentum pass
+// in one call, alone in the next, or kept from either, with the same result, so
+// that matrix takes the lower line always; the higher one is for the systems that
+// are never set up beside others (a caller's, the coupled system's pressure
+// stage).  For the first reason a block takes
 // kNnzPerBlock entries or more: 72 blocks instead of 152 at 32^3 made the
 // outer iteration 2.33 ms instead of 2.65.
 //
@@ -51,8 +56,8 @@ constexpr int kBigSlots = kWarps * kSlots;   // of the rows that the whole block
 constexpr int kTableBytes = kWarps * kSlots * kTableSlotBytes;
 constexpr int kListed = kSlots * kTableSlotBytes / 32 / 12;   // places a thread in prolongation rows
 constexpr int kBlockProducts = 768;   // products from which the whole block sums a row
-// the largest levels taken (see above), and those when the kernels of the
-// momentum pass run beside the setup
+// the largest levels taken (see above): of a system that is set up alone, and of
+// the mesh's pressure matrix
 constexpr int kSmallRows = 262144, kBesideRows = 65536;
 constexpr int64_t kSmallNnz = 2000000, kBesideNnz = 1700000;
 constexpr int kMostBlocks = 152, kNnzPerBlock = 3072;
@@ -940,8 +945,8 @@ __global__ void __launch_bounds__(kT, 1) k_small_inverse(SmallArgs<V> a) {
 
 }  // namespace
 
-bool small_setup_fits(int n, int64_t nnz, bool beside) {
-    return n <= (beside ? kBesideRows : kSmallRows) && nnz <= (beside ? kBesideNnz : kSmallNnz);
+bool small_setup_fits(int n, int64_t nnz, bool mesh_matrix) {
+    return n <= (mesh_matrix ? kBesideRows : kSmallRows) && nnz <= (mesh_matrix ? kBesideNnz : kSmallNnz);
 }
 
 template <class V>

@@ -405,7 +405,7 @@ void build_hierarchy(semo_ctx* c, Amg<V>& h, const int* ptr, const int* col, con
 // kernels take it).  Waits for the stream; sflag is then read: the error flags
 // of the levels above, whose copy the caller queued
 enum class SmallResult { done, needs_inverse, no_room };
-bool small_setup_fits(int n, int64_t nnz, bool beside);   // beside: kernels of another stream run meanwhile
+bool small_setup_fits(int n, int64_t nnz, bool mesh_matrix);   // mesh_matrix: may run beside the momentum pass
 template <class V>
 SmallResult small_setup(semo_ctx* c, Amg<V>& h, float eps, double omega, const int* sflag);
 // exclusive scan of d[0..n) in place on the context's stream; returns the total
