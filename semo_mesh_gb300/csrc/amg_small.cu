@@ -41,6 +41,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <utility>
 
 #include "amg_rows.cuh"
 #include "semo_internal.h"
@@ -62,6 +63,10 @@ constexpr int kSmallRows = 262144, kBesideRows = 65536;
 constexpr int64_t kSmallNnz = 2000000, kBesideNnz = 1700000;
 constexpr int kMostBlocks = 152, kNnzPerBlock = 3072;
 constexpr int kMaxBlocks = 256, kMaxLevels = 64, kMaxRounds = 200, kRoundSlots = 1024;
+// Scratch that may stay with a hierarchy: what a finished arena holds beyond it is
+// given back by a copy of the levels (an arena has 56 MB at 64,000 rows of 7
+// entries; the calls on such systems take as long as before)
+constexpr long long kSpareBytes = 16ll << 20;
 constexpr int kGjMax = 64;         // rows of the largest coarsest level inverted by k_small_inverse
 constexpr unsigned kSpinLimit = 1u << 23;
 // Levels this small are built by one block: its barrier costs some 30 ns
@@ -77,7 +82,7 @@ struct SmallRec {
 enum SmallStatus { SMALL_OK = 0, SMALL_NO_ROOM = 1, SMALL_NO_MIS = 2, SMALL_LONG_ROW = 3 };
 struct SmallCtl {
     int status, nlev, zero_diag, non_finite, singular, abort;
-    long long cinv;
+    long long cinv, kept;   // kept: bytes of the arena that the hierarchy needs
     SmallRec lev[kMaxLevels];
     // below: not read by the host
     unsigned arrived;
@@ -838,14 +843,15 @@ __global__ void __launch_bounds__(kT, 1) k_small_setup(SmallArgs<V> a) {
         nnz = nnzC;
     }
     // the coarsest level's inverse (k_small_inverse)
-    const long long o_inv = keep(8ll * n * n);
     if (n <= kGjMax) {
+        const long long o_inv = keep(8ll * n * n);
         if (lo > a.cap) {
             if (first) atomicExch(&ctl->status, SMALL_NO_ROOM);
         } else if (first) {
             ctl->cinv = o_inv;
         }
     }
+    if (first) ctl->kept = lo;
 #undef SMALL_ROOM
 #undef SMALL_SYNC
 }
@@ -1009,6 +1015,12 @@ SmallResult small_setup(semo_ctx* c, Amg<V>& h, float eps, double omega, const i
         return SmallResult::no_room;
     }
     if (r.singular) throw Error(SEMO_ERR_BREAKDOWN, "coarsest AMG matrix is singular");
+    if (a.cap - r.kept > kSpareBytes) {   // the levels stay, the scratch does not
+        DBuf<unsigned char> kept;
+        kept.alloc((size_t)r.kept, s);
+        SEMO_CUDA(cudaMemcpyAsync(kept.p, h.arena.p, (size_t)r.kept, cudaMemcpyDeviceToDevice, s));
+        h.arena = std::move(kept);
+    }
     unsigned char* const A = h.arena.p;
     auto ints = [&](DBuf<int>& b, long long off, int64_t count) { b.view(reinterpret_cast<int*>(A + off), (size_t)count); };
     auto vals = [&](DBuf<V>& b, long long off, int64_t count) { b.view(reinterpret_cast<V*>(A + off), (size_t)count); };
