@@ -40,6 +40,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <cstring>
 #include <utility>
 
@@ -951,6 +952,8 @@ __global__ void __launch_bounds__(kT, 1) k_small_inverse(SmallArgs<V> a) {
 
 }  // namespace
 
+size_t small_record_bytes() { return offsetof(SmallCtl, arrived); }
+
 bool small_setup_fits(int n, int64_t nnz, bool mesh_matrix) {
     return n <= (mesh_matrix ? kBesideRows : kSmallRows) && nnz <= (mesh_matrix ? kBesideNnz : kSmallNnz);
 }
@@ -999,9 +1002,8 @@ SmallResult small_setup(semo_ctx* c, Amg<V>& h, float eps, double omega, const i
     const int gj = kGjMax * kGjMax * (int)sizeof(double);
     k_small_inverse<V><<<1, kT, gj, s>>>(a);
     SEMO_CHECK_LAUNCH();
-    if (!c->hpin_small) SEMO_CUDA(cudaMallocHost(&c->hpin_small, sizeof(SmallCtl)));
     SmallCtl& r = *reinterpret_cast<SmallCtl*>(c->hpin_small);
-    SEMO_CUDA(cudaMemcpyAsync(&r, ctl.p, offsetof(SmallCtl, arrived), cudaMemcpyDeviceToHost, s));
+    SEMO_CUDA(cudaMemcpyAsync(&r, ctl.p, small_record_bytes(), cudaMemcpyDeviceToHost, s));
     SEMO_CUDA(cudaStreamSynchronize(s));   // whatever the caller queued before has landed too
     if (r.abort) throw Error(SEMO_ERR_CUDA, "AMG setup: a grid barrier was not reached");
     if (sflag[2]) r.zero_diag = 1;   // the levels above

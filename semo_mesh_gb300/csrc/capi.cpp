@@ -127,6 +127,7 @@ semo_status semo_ctx_create(semo_ctx** out, const semo_params* prm) {
         SEMO_CUDA(cudaMallocHost((void**)&c->hpin_setup, semo::kHostScalars * sizeof(double)));
         SEMO_CUDA(cudaMallocHost((void**)&c->hpin_scan, semo::kHostInts * sizeof(int)));
         SEMO_CUDA(cudaMallocHost((void**)&c->hpin_int, semo::kHostInts * sizeof(int)));
+        SEMO_CUDA(cudaMallocHost(&c->hpin_small, semo::small_record_bytes()));
         c->flag.alloc(16, c->stream);
         c->flag.zero();
     });

@@ -405,6 +405,7 @@ void build_hierarchy(semo_ctx* c, Amg<V>& h, const int* ptr, const int* col, con
 // kernels take it).  Waits for the stream; sflag is then read: the error flags
 // of the levels above, whose copy the caller queued
 enum class SmallResult { done, needs_inverse, no_room };
+size_t small_record_bytes();   // pinned bytes it reads its records into (semo_ctx::hpin_small)
 bool small_setup_fits(int n, int64_t nnz, bool mesh_matrix);   // mesh_matrix: may run beside the momentum pass
 template <class V>
 SmallResult small_setup(semo_ctx* c, Amg<V>& h, float eps, double omega, const int* sflag);
