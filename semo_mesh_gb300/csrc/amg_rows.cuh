@@ -25,7 +25,7 @@ __device__ __forceinline__ unsigned long long mis_key(int st, int i) {
 // on the integer pipes: the 24-bit significands multiply exactly into 48
 // bits, so this equals __double2ll_rn(((double)a * b) * 2^sc) (the FP64
 // product of two floats is exact too) without touching the FP64 unit.
-// Requires |a b| 2^sc < 2^62.
+// Requires |a b| 2^sc < 2^63.
 __device__ __forceinline__ long long fixed_product(float a, float b, int sc) {
     const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
     int ea = (int)((ua >> 23) & 0xff), eb = (int)((ub >> 23) & 0xff);
@@ -39,7 +39,7 @@ __device__ __forceinline__ long long fixed_product(float a, float b, int sc) {
     if (m == 0ull) {
         q = 0ull;
     } else if (e >= 0) {
-        q = (e < 64) ? (m << e) : 0ull;   // e <= 61 whenever the scale bound holds
+        q = (e < 64) ? (m << e) : 0ull;   // e <= 62 whenever the scale bound holds
     } else if (e <= -64) {
         q = 0ull;   // below half a unit (m < 2^48)
     } else {
@@ -71,7 +71,7 @@ __host__ __device__ __forceinline__ long long fixed_product(double a, double b, 
     const uint64_t hi = (uint64_t)(m >> 64), lo = (uint64_t)m;
     const int sh = 2150 - ea - eb - sc;   // |a b| 2^sc = m 2^-sh
     uint64_t q, rem, half;
-    if (sh <= 0) {   // m < 2^62 then, by the scale's bound
+    if (sh <= 0) {   // m < 2^63 then, by the scale's bound
         q = sh > -64 ? lo << -sh : 0ull;
         rem = 0ull;
         half = 1ull;
@@ -130,12 +130,13 @@ __device__ __forceinline__ Mag mag_warp_sum(Mag s) {
     for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
     return Mag{m, e};
 }
-// fixed-point scale exponent for sums of at most s: s 2^sc < 2^62.  The FP32
-// sums above round a few times; 2^-10 covers them.
+// fixed-point scale exponent for sums of at most s: s 2^sc < 2^63 by 2^-10 of it,
+// which covers the roundings of the FP32 sums above (2^-24 an addition, 3,072 in a
+// row at most) and of the scaled products (half a unit each)
 __device__ __forceinline__ int mag_scale(Mag s) {
     const float m = s.m * 1.0009765625f;
     const int e = m > 0.0f ? s.e + (int)((__float_as_uint(m) >> 23) & 0xff) - 126 : -1022;   // s < 2^e
-    return max(-960, min(1000, 62 - e));
+    return max(-960, min(1000, 63 - e));
 }
 // q 2^-sc rounded to the nearest V
 __device__ __forceinline__ double fixed_value(long long q, int sc, double) {
@@ -189,8 +190,8 @@ __device__ __forceinline__ int table_size(int most, int limit) {
 // in row order, B entries in chunks of 32) and summed as 64-bit fixed-point
 // integers (integer addition is associative, so the sums do not depend on the
 // order the shared-memory atomics land in): with S = sum_k |a_ik| bmag_k >=
-// the row's sum of |products|, each product is scaled by 2^s, S 2^s < 2^62,
-// and rounded to an integer -- an error of at most 2^-62 S per product, below
+// the row's sum of |products|, each product is scaled by 2^s, S 2^s < 2^63,
+// and rounded to an integer -- an error of at most 2^-63 (S + 2^-10 S) per product, below
 // what FP64 accumulation of the same products incurs (2^-53 S per addition).
 // The row is written sorted by column to ocol/oval.  Returns its length, or
 // -1 (nothing written) when more than 3/4 of the ht slots are taken.
