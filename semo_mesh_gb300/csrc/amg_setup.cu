@@ -543,18 +543,15 @@ template <class V>
 __global__ void __launch_bounds__(128) k_spgemm_small(int n, const int* __restrict__ aptr,
                                                       const int* __restrict__ acol, const V* __restrict__ aval,
                                                       const int* __restrict__ bptr, const int* __restrict__ bcol,
-                                                      const V* __restrict__ bval, int pass, int* __restrict__ small,
+                                                      const V* __restrict__ bval, int* __restrict__ small,
                                                       const int* __restrict__ cptr, int* __restrict__ ccol,
                                                       V* __restrict__ cval) {
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= n) return;
-    if (pass == 1 && small[row] < 0) return;
     const int ab = aptr[row], ae = aptr[row + 1];
-    if (pass != 1) {
-        int prod = 0;
-        for (int ka = ab; ka < ae; ++ka) prod += bptr[acol[ka] + 1] - bptr[acol[ka]];
-        if (prod > kSmallMaxProducts) { small[row] = -1; return; }
-    }
+    int prod = 0;
+    for (int ka = ab; ka < ae; ++ka) prod += bptr[acol[ka] + 1] - bptr[acol[ka]];
+    if (prod > kSmallMaxProducts) { small[row] = -1; return; }
     int cols[kSmallCap];
     V vals[kSmallCap];
 #pragma unroll
@@ -566,7 +563,7 @@ __global__ void __launch_bounds__(128) k_spgemm_small(int n, const int* __restri
         const V av = aval[ka];
         for (int q = bptr[a]; q < bptr[a + 1]; ++q) {
             const int cq = bcol[q];
-            const V pv = (pass != 0) ? av * bval[q] : V(0);
+            const V pv = av * bval[q];
             bool found = false;
 #pragma unroll
             for (int t = 0; t < kSmallCap; ++t)
@@ -585,18 +582,12 @@ __global__ void __launch_bounds__(128) k_spgemm_small(int n, const int* __restri
             ++d;
         }
     }
-    if (pass == 0) {
-        small[row] = over ? -1 : d;
-    } else {
-        if (pass == 2) {
-            small[row] = over ? -1 : d;
-            if (over) return;
-        }
-        const int base = cptr[row];
+    small[row] = over ? -1 : d;
+    if (over) return;
+    const int base = cptr[row];
 #pragma unroll
-        for (int t = 0; t < kSmallCap; ++t)
-            if (t < d) { ccol[base + t] = cols[t]; cval[base + t] = vals[t]; }
-    }
+    for (int t = 0; t < kSmallCap; ++t)
+        if (t < d) { ccol[base + t] = cols[t]; cval[base + t] = vals[t]; }
 }
 
 // Row-wise SpGEMM C = A * B, one warp per row (hash_row in amg_rows.cuh): rows
@@ -776,8 +767,8 @@ void spgemm(cudaStream_t s, semo_ctx* c, const DCsr<V>& A, const DCsr<V>& B, DCs
     DBuf<V> tval;
     tcol.alloc(std::max<int64_t>(total, 1), s);
     tval.alloc(std::max<int64_t>(total, 1), s);
-    k_spgemm_small<V><<<blocks(n, 128), 128, 0, s>>>(n, A.ptr, A.col, A.val, B.ptr, B.col, B.val, 2, cnt.p, up.p,
-                                                     tcol.p, tval.p);
+    k_spgemm_small<V><<<blocks(n, 128), 128, 0, s>>>(n, A.ptr, A.col, A.val, B.ptr, B.col, B.val, cnt.p, up.p, tcol.p,
+                                                     tval.p);
     SEMO_CHECK_LAUNCH();
     if (maxprod > kSmallMaxProducts) {
         // tables sized per row from its products (<= 3/4 load); most rows fit

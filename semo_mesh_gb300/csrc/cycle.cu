@@ -15,7 +15,9 @@
 //    for the neighbours), post-smoothing is two, with no separate x += d;
 //  * the CG update uses q = A z + beta q (so p and q update in place) and
 //    the dot products are folded into the kernels that produce their
-//    operands; one CG iteration is ~30 launches, captured as a CUDA graph.
+//    operands; one CG iteration is 22 launches at 48^3 to 128^3 cells (16 at
+//    32^3), captured as a CUDA graph; small systems are solved in one kernel
+//    (cycle_cluster.cuh).
 // FP32 V-cycle arithmetic stays on the FP32 pipes (FP64 is 1/58 of FP32
 // on GB300); dot products and the outer residual are FP64.
 #include <cuda_runtime.h>
@@ -320,7 +322,7 @@ struct FirstGather {   // d0 formed on the fly
 };
 
 // ------------------------------------------- programmatic dependent launch
-// The ~30 kernels of a CG iteration each depend on the one before and are
+// The 16 to 22 kernels of a CG iteration each depend on the one before and are
 // short, so the gap between one kernel's last block and the next one's first
 // is a real share of an iteration.  They are launched with programmatic
 // stream serialisation: a kernel's launch is processed while its predecessor
@@ -1440,7 +1442,7 @@ void pcg(semo_ctx* c, Amg<V>& h, Cycle<V>& cy, const OuterOp& outer, bool same, 
     k_fin_sum<<<1, kRedThreads, 0, s>>>(R.part + kRedBlocks, nb, R.scal + 12);   // ||r0||^2
     SEMO_CHECK_LAUNCH();
     // The loop is one graph: k_cg_begin, then a conditional WHILE node whose
-    // body is one CG iteration (~30 kernels) plus k_cg_check, which decides on
+    // body is one CG iteration plus k_cg_check, which decides on
     // the device whether to go on.  It is captured and instantiated while the
     // kernels above run, and the host waits once, after the true residual.
     GraphGuard gg;

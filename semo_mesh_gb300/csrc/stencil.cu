@@ -96,9 +96,9 @@ __global__ void __launch_bounds__(128) k_stencil(int nc, int ni, int nb, const i
         const double a2 = fma(-phi[q], sz, g[q][2]);
         // limits: U, V, W, VF, P in that order
         const int f = F0 + q, at = f == 0 ? 8 : (f == 4 ? 6 : 2 * (f - 1));
-        grad[(size_t)(3 * f) * N + i] = fma(m2, a2, fma(m1, a1, m0 * a0));
-        grad[(size_t)(3 * f + 1) * N + i] = fma(m4, a2, fma(m3, a1, m1 * a0));
-        grad[(size_t)(3 * f + 2) * N + i] = fma(m5, a2, fma(m4, a1, m2 * a0));
+        grad[(size_t)(3 * f) * N + i] = fma(m2, a2, fma(m1, a1, fma(m0, a0, 0.0)));
+        grad[(size_t)(3 * f + 1) * N + i] = fma(m4, a2, fma(m3, a1, fma(m1, a0, 0.0)));
+        grad[(size_t)(3 * f + 2) * N + i] = fma(m5, a2, fma(m4, a1, fma(m2, a0, 0.0)));
         mm[(size_t)at * N + i] = ounkey(kmax[q]);
         mm[(size_t)(at + 1) * N + i] = ounkey(kmin[q]);
     }
